@@ -32,7 +32,7 @@ struct ddd_ctx {
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   std::mutex mu;
   std::string err;
-  DevBuf coord, bvec, segidx, ext, soa, soadf, skip, partial, out, rows, x0, sigma, counters, probe, errflag;
+  DevBuf coord, bvec, segidx, ext, soa, soadf, skip, partial, expand, out, rows, x0, sigma, counters, probe, errflag;
   DevBuf links, conn, segforce;  // mobility inputs
   DevBuf vel, label, skippairs;  // collision inputs
   ddd::CollisionPlan* coll = nullptr;
@@ -83,6 +83,7 @@ cudaError_t prep_df_if_needed(ddd_ctx* c, int64_t npad, cudaStream_t st) {
 // its slot (one tile launch, one reduction); above it the launchers run bands
 // of tile columns through a buffer of the limit's size.
 constexpr int64_t kDefaultPartialLimit = (int64_t)16 << 30;
+int64_t partial_limit(const ddd_ctx* c) { return c->partialLimit ? c->partialLimit : kDefaultPartialLimit; }
 
 // Slots to allocate for npad segments: all nt(nt+1)/2 when they fit in the
 // context's limit, else as many as the limit holds, at least one column (nt).
@@ -90,7 +91,7 @@ int64_t partial_slots(const ddd_ctx* c, int64_t npad) {
   const int64_t tile = ddd::strict::segseg_npad(1);
   const int64_t slotBytes = (int64_t)ddd::strict::segseg_partial_bytes_all(tile);
   const int64_t nt = npad / tile, all = nt * (nt + 1) / 2;
-  const int64_t cap = (c->partialLimit ? c->partialLimit : kDefaultPartialLimit) / slotBytes;
+  const int64_t cap = partial_limit(c) / slotBytes;
   return cap >= all ? all : (cap < nt ? nt : cap);
 }
 
@@ -104,6 +105,26 @@ cudaError_t run_segseg_all(ddd_ctx* c, const ddd::KConsts& K, const double* soa,
   if (use_df(c)) {
     cudaError_t e = prep_df_if_needed(c, npad, st);
     if (e != cudaSuccess) return e;
+  }
+  // Small networks: one warp per 32 pairs, the pair values stored and folded.
+  // The store obeys the partial-sum limit too; without it (limit, no memory) the
+  // tile kernel gives the same bits.
+  const int64_t nt = npad / ddd::strict::segseg_npad(1), nb = nt * (nt + 1) / 2;
+  if (nb <= ddd::kExpandMaxPairs && cap >= nb && (int64_t)ddd::expand_bytes(nb) <= partial_limit(c)) {
+    const cudaError_t e = c->expand.ensure(ddd::expand_bytes(nb));
+    if (e == cudaSuccess) {
+      void* x = c->expand.p;
+      if (use_df(c))
+        return ddd::launch_segseg_small_df(K, soa, c->soadf.as<float>(), skip, npad, x, partial, out, numSeg, cnt, st,
+                                           df_form(c));
+      if (use_fx(c)) return ddd::launch_segseg_small_fx(K, soa, skip, npad, x, partial, out, numSeg, cnt, st);
+      return use_fma(c) ? ddd::fast::launch_segseg_small_f64(K, soa, skip, npad, x, partial, out, numSeg, cnt, st)
+                        : ddd::strict::launch_segseg_small_f64(K, soa, skip, npad, x, partial, out, numSeg, cnt, st);
+    }
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+  }
+  if (use_df(c)) {
     return ddd::launch_segseg_all_df(K, soa, c->soadf.as<float>(), skip, npad, partial, out, numSeg, cnt, st,
                                      df_form(c), cap);
   }
@@ -112,37 +133,34 @@ cudaError_t run_segseg_all(ddd_ctx* c, const ddd::KConsts& K, const double* soa,
                     : ddd::strict::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap);
 }
 
-// Index rows per launch: all of them when their partial sums (one block of
-// 6 x TILE doubles per row tile and column tile) fit in the context's limit,
-// else whole row tiles up to the limit, at least one.  Rows are independent,
-// so chunking changes no bit of the result.
-int64_t rows_per_chunk(const ddd_ctx* c, int64_t npad, int64_t nRows) {
+// Index rows per launch: all of them when their partial sums (6 doubles per row
+// and column block) fit in the context's limit, else as many as do, at least one
+// tile's worth.  Rows are independent, so chunking changes no bit of the result.
+int64_t rows_per_chunk(const ddd_ctx* c, const ddd::RowPlan& plan, int64_t nRows) {
   const int64_t tile = ddd::strict::segseg_npad(1);
-  const int64_t perTile = (int64_t)ddd::strict::segseg_partial_bytes_rows(tile, npad);  // one row tile
-  const int64_t limit = c->partialLimit ? c->partialLimit : kDefaultPartialLimit;
-  const int64_t tiles = limit / perTile;
-  const int64_t chunk = (tiles < 1 ? 1 : tiles) * tile;
+  const int64_t fit = partial_limit(c) / (int64_t)ddd::row_partial_bytes(plan, 1);
+  const int64_t chunk = fit < tile ? tile : fit;
   return chunk < nRows ? chunk : nRows;
 }
 
 cudaError_t run_segseg_rows(ddd_ctx* c, const ddd::KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
-                            const int64_t* rows, int64_t nRows, double* partial, double* out,
+                            const int64_t* rows, int64_t nRows, const ddd::RowPlan& plan, double* partial, double* out,
                             unsigned long long* cnt, cudaStream_t st) {
   if (use_df(c)) {
     cudaError_t e = prep_df_if_needed(c, npad, st);
     if (e != cudaSuccess) return e;
   }
-  const int64_t chunk = rows_per_chunk(c, npad, nRows);
+  const int64_t chunk = rows_per_chunk(c, plan, nRows);
   for (int64_t r0 = 0; r0 < nRows; r0 += chunk) {
     const int64_t n = nRows - r0 < chunk ? nRows - r0 : chunk;
+    const int64_t* r = rows + r0;
+    double* o = out + 6 * r0;
     const cudaError_t e =
-        use_df(c) ? ddd::launch_segseg_rows_df(K, soa, c->soadf.as<float>(), skip, npad, rows + r0, n, partial,
-                                               out + 6 * r0, cnt, st, df_form(c))
-        : use_fx(c)  ? ddd::launch_segseg_rows_fx(K, soa, skip, npad, rows + r0, n, partial, out + 6 * r0, cnt, st)
-        : use_fma(c) ? ddd::fast::launch_segseg_rows_f64(K, soa, skip, npad, rows + r0, n, partial, out + 6 * r0, cnt,
-                                                         st)
-                     : ddd::strict::launch_segseg_rows_f64(K, soa, skip, npad, rows + r0, n, partial, out + 6 * r0,
-                                                           cnt, st);
+        use_df(c) ? ddd::launch_segseg_rows_df(K, soa, c->soadf.as<float>(), skip, npad, r, n, plan, partial, o, cnt,
+                                               st, df_form(c))
+        : use_fx(c)  ? ddd::launch_segseg_rows_fx(K, soa, skip, npad, r, n, plan, partial, o, cnt, st)
+        : use_fma(c) ? ddd::fast::launch_segseg_rows_f64(K, soa, skip, npad, r, n, plan, partial, o, cnt, st)
+                     : ddd::strict::launch_segseg_rows_f64(K, soa, skip, npad, r, n, plan, partial, o, cnt, st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -276,12 +294,12 @@ int segseg_compute(ddd_ctx* ctx, const ddd_consts* k, const double* coord, int64
                        ctx->stream),
        "copy idx");
     h2d += nIdx * (int64_t)sizeof(int64_t);
-    const int64_t chunkRows = rows_per_chunk(ctx, npad, nIdx);
-    CK(ctx->partial.ensure(ddd::strict::segseg_partial_bytes_rows(chunkRows, npad)), "alloc partial sums");
+    const ddd::RowPlan plan = ddd::row_plan(npad, nIdx);
+    CK(ctx->partial.ensure(ddd::row_partial_bytes(plan, rows_per_chunk(ctx, plan, nIdx))), "alloc partial sums");
     CK(cudaEventRecord(ctx->ev[1], ctx->stream), "event");
     CK(run_segseg_rows(ctx, K, ctx->soa.as<double>(), ctx->skip.as<uint8_t>(), npad, ctx->rows.as<int64_t>(),
-                                   nIdx, ctx->partial.as<double>(), ctx->out.as<double>(),
-                                   ctx->counters.as<unsigned long long>(), ctx->stream),
+                       nIdx, plan, ctx->partial.as<double>(), ctx->out.as<double>(),
+                       ctx->counters.as<unsigned long long>(), ctx->stream),
        "segseg_rows_f64");
   }
   CK(cudaEventRecord(ctx->ev[2], ctx->stream), "event");
@@ -341,7 +359,7 @@ void ddd_destroy(ddd_ctx* c) {
   if (c->coll) ddd::collision_plan_destroy(c->coll);
   delete c->ut;
   c->upoints.release();
-  for (DevBuf* b : {&c->coord, &c->bvec, &c->segidx, &c->ext, &c->soa, &c->soadf, &c->skip, &c->partial, &c->out, &c->rows,
+  for (DevBuf* b : {&c->coord, &c->bvec, &c->segidx, &c->ext, &c->soa, &c->soadf, &c->skip, &c->partial, &c->expand, &c->out, &c->rows,
                     &c->x0, &c->sigma, &c->counters, &c->probe, &c->errflag})
     b->release();
   for (auto& ev : c->ev)

@@ -41,6 +41,29 @@ cudaError_t set_smem_once(Kernel* kernel, int bytes, std::atomic<uint64_t>& done
   return e;
 }
 
+// Index rows (segseg_small.cuh): a row's columns in nBlk blocks of 128 m, one
+// CTA each.  m grows from 1 to 8 with the work so that a call has ~1,216 CTAs
+// (four rounds of the 304 that are resident) before a CTA takes more steps; it
+// depends on the call's whole row count, so that chunks of rows change no sum.
+constexpr int kRowMaxSteps = 8;
+struct RowPlan {
+  int64_t nBlk;
+  int m;
+};
+inline RowPlan row_plan(int64_t npad, int64_t nRows) {
+  const int64_t q = nRows * (npad / 128) / 1216;
+  const int m = q < 1 ? 1 : q > kRowMaxSteps ? kRowMaxSteps : (int)q;
+  return RowPlan{(npad + 128 * m - 1) / (128 * m), m};
+}
+inline size_t row_partial_bytes(const RowPlan& p, int64_t nRows) { return (size_t)(nRows * p.nBlk) * 6 * sizeof(double); }
+
+// Expanded all-pairs of small networks (segseg_small.cuh): every pair's twelve
+// components, class and list entry stored, 128 x 128 positions per tile pair.
+// Up to 153 tile pairs (2,176 segments, 252 MB): beyond that the tile kernel has
+// two CTAs for most SMs and the store grows with the square of the size.
+constexpr int64_t kExpandMaxPairs = 153;
+inline size_t expand_bytes(int64_t nb) { return (size_t)nb * 128 * 128 * (12 * sizeof(double) + 4 + 1) + 256; }
+
 // All-pairs partial sums: one slot (12 x TILE doubles) per tile pair I <= J,
 // slot J(J+1)/2 + I.  The all-pairs launchers take the partial buffer's size
 // in slots; when it is below nt(nt+1)/2 they run bands of J columns (each band
@@ -53,7 +76,6 @@ cudaError_t set_smem_once(Kernel* kernel, int bytes, std::atomic<uint64_t>& done
   int64_t segseg_npad(int64_t numSeg); \
   size_t segseg_soa_bytes(int64_t npad); \
   size_t segseg_partial_bytes_all(int64_t npad); \
-  size_t segseg_partial_bytes_rows(int64_t nRows, int64_t npad); \
   cudaError_t launch_prep_segments(const double* coord, const double* bVec, const int64_t* segIdx, int64_t ld, \
                                    const uint8_t* extSeg, int64_t numSeg, int64_t npad, double* soa, uint8_t* skip, \
                                    cudaStream_t st); \
@@ -63,15 +85,17 @@ cudaError_t set_smem_once(Kernel* kernel, int bytes, std::atomic<uint64_t>& done
   cudaError_t launch_segseg_all_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad, \
                                     double* partial, double* out, int64_t numSeg, unsigned long long* counters, \
                                     cudaStream_t st, int64_t capSlots); \
+  cudaError_t launch_segseg_small_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad, \
+                                      void* scratch, double* partial, double* out, int64_t numSeg, \
+                                      unsigned long long* counters, cudaStream_t st); \
   cudaError_t launch_segseg_rows_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad, \
-                                     const int64_t* rows, int64_t nRows, double* partial, double* out, \
-                                     unsigned long long* counters, cudaStream_t st); \
+                                     const int64_t* rows, int64_t nRows, const RowPlan& plan, double* partial, \
+                                     double* out, unsigned long long* counters, cudaStream_t st); \
   cudaError_t launch_sigma_f64(const KConsts& K, const double* soa, int64_t npad, int64_t nSeg, const double* x0, \
                                int64_t M, double* sigma, cudaStream_t st); \
   cudaError_t launch_reduce_all(const double* partial, int64_t npad, int64_t numSeg, double* out, cudaStream_t st); \
   cudaError_t launch_reduce_band(const double* partial, int64_t J0, int64_t J1, int64_t numSeg, double* out, \
                                  cudaStream_t st); \
-  cudaError_t launch_reduce_rows(const double* partial, int64_t npad, int64_t nRows, double* out, cudaStream_t st); \
   cudaError_t preload_all_f64();
 
 namespace strict {
@@ -89,9 +113,13 @@ cudaError_t launch_prep_df(const double* soa, int64_t npad, float* soadf, cudaSt
 cudaError_t launch_segseg_all_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
                                  int64_t npad, double* partial, double* out, int64_t numSeg,
                                  unsigned long long* counters, cudaStream_t st, int form, int64_t capSlots);
+cudaError_t launch_segseg_small_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
+                                   int64_t npad, void* scratch, double* partial, double* out, int64_t numSeg,
+                                   unsigned long long* counters, cudaStream_t st, int form);
 cudaError_t launch_segseg_rows_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
-                                  int64_t npad, const int64_t* rows, int64_t nRows, double* partial, double* out,
-                                  unsigned long long* counters, cudaStream_t st, int form);
+                                  int64_t npad, const int64_t* rows, int64_t nRows, const RowPlan& plan,
+                                  double* partial, double* out, unsigned long long* counters, cudaStream_t st,
+                                  int form);
 // σ̃ in the mixed form: geometry and endpoint differences in df64, assembly in FP32.
 cudaError_t launch_sigma_mixed(const KConsts& K, const float* soadf, int64_t npad, int64_t nSeg, const double* x0,
                                int64_t M, double* sigma, cudaStream_t st);
@@ -105,9 +133,12 @@ cudaError_t launch_sigma_fx(const KConsts& K, const double* soa, int64_t npad, i
 cudaError_t launch_segseg_all_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                                  double* partial, double* out, int64_t numSeg, unsigned long long* counters,
                                  cudaStream_t st, int64_t capSlots);
+cudaError_t launch_segseg_small_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
+                                   void* scratch, double* partial, double* out, int64_t numSeg,
+                                   unsigned long long* counters, cudaStream_t st);
 cudaError_t launch_segseg_rows_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
-                                  const int64_t* rows, int64_t nRows, double* partial, double* out,
-                                  unsigned long long* counters, cudaStream_t st);
+                                  const int64_t* rows, int64_t nRows, const RowPlan& plan, double* partial,
+                                  double* out, unsigned long long* counters, cudaStream_t st);
 
 // tc_gemm.cu: tcgen05 GEMM, D = A * B^T (both K-major), A and B both BF16 or both F16.
 size_t tc_gemm_smem_bytes(int N);

@@ -91,7 +91,7 @@ persistent_tiles(TileArgs A, typename P::Consts KP, const int4* __restrict__ ite
     const int32_t w = s_item;
     if (w >= nItems) break;
     const int4 it = items[w];
-    tile_body<T, 0, P>(A, KP, sm, it.y, it.z, it.w != 0, nullptr, 0, partial + (int64_t)it.x * 12 * T, counters);
+    tile_body<T, 0, P>(A, KP, sm, it.y, it.z, it.w != 0, partial + (int64_t)it.x * 12 * T, counters);
   }
 }
 

@@ -17,6 +17,7 @@
 #include "ddd_internal.h"
 #include "pair_df.cuh"
 #include "pair_f64.cuh"
+#include "segseg_small.cuh"
 #include "tile_pol_df.cuh"
 #include "tile_body.cuh"
 
@@ -46,27 +47,22 @@ __device__ __forceinline__ void tile_index_df(int64_t b, int64_t& I, int64_t& J)
   I = b - Jc * (Jc + 1) / 2;
 }
 
-template <int MODE, int FORM>
+template <int FORM>
 __global__ void __launch_bounds__(TILE, 2)
-segseg_tile_df(TileArgs A, typename PolDF<FORM>::Consts KP, const int64_t* __restrict__ rows, int64_t nRows,
-               int64_t nJt, int64_t base, double* __restrict__ partial, unsigned long long* __restrict__ counters) {
+segseg_tile_df(TileArgs A, typename PolDF<FORM>::Consts KP, int64_t base, double* __restrict__ partial,
+               unsigned long long* __restrict__ counters) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& sm = *reinterpret_cast<TileSmemT<TILE, PolDF<FORM>>*>(smem_raw);
   int64_t I, J;
-  if (MODE == 0) {
-    tile_index_df(base + blockIdx.x, I, J);  // slots base.. (a band of J columns)
-  } else {
-    I = blockIdx.x / nJt;
-    J = blockIdx.x % nJt;
-  }
-  tile_body<TILE, MODE, PolDF<FORM>>(A, KP, sm, I * TILE, J * TILE, MODE == 0 && I == J, rows, nRows,
-                                     partial + (int64_t)blockIdx.x * (MODE == 0 ? 12 : 6) * TILE, counters);
+  tile_index_df(base + blockIdx.x, I, J);  // slots base.. (a band of J columns)
+  tile_body<TILE, 0, PolDF<FORM>>(A, KP, sm, I * TILE, J * TILE, I == J,
+                                  partial + (int64_t)blockIdx.x * 12 * TILE, counters);
 }
 
-template <int MODE, int FORM>
+template <int FORM>
 cudaError_t set_attr_df() {
   static std::atomic<uint64_t> done{0};
-  return set_smem_once(segseg_tile_df<MODE, FORM>, (int)sizeof(TileSmemT<TILE, PolDF<FORM>>), done);
+  return set_smem_once(segseg_tile_df<FORM>, (int)sizeof(TileSmemT<TILE, PolDF<FORM>>), done);
 }
 
 // σ̃ in the mixed form (sigma_point_mixed, pair_df.cuh): one thread per point,
@@ -137,7 +133,7 @@ cudaError_t launch_prep_df(const double* soa, int64_t npad, float* soadf, cudaSt
 cudaError_t launch_segseg_all_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
                                  int64_t npad, double* partial, double* out, int64_t numSeg,
                                  unsigned long long* counters, cudaStream_t st, int form, int64_t capSlots) {
-  cudaError_t e = form ? set_attr_df<0, 1>() : set_attr_df<0, 0>();
+  cudaError_t e = form ? set_attr_df<1>() : set_attr_df<0>();
   if (e != cudaSuccess) return e;
   const int64_t nt = npad / TILE;
   const int64_t nb = nt * (nt + 1) / 2;
@@ -148,11 +144,11 @@ cudaError_t launch_segseg_all_df(const KConsts& K, const double* soa, const floa
     const int64_t J1 = capSlots >= nb ? nt : strict::segseg_band_end(J0, nt, capSlots);
     const int64_t b0 = J0 * (J0 + 1) / 2, nbb = J1 * (J1 + 1) / 2 - b0;
     if (form)
-      segseg_tile_df<0, 1><<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolDF<1>>), st>>>(
-          A, PolDF<1>::Consts{kconsts_df(K), kconsts_f(K)}, nullptr, 0, 0, b0, partial, counters);
+      segseg_tile_df<1><<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolDF<1>>), st>>>(
+          A, PolDF<1>::Consts{kconsts_df(K), kconsts_f(K)}, b0, partial, counters);
     else
-      segseg_tile_df<0, 0><<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolDF<0>>), st>>>(
-          A, PolDF<0>::Consts{kconsts_df(K), kconsts_f(K)}, nullptr, 0, 0, b0, partial, counters);
+      segseg_tile_df<0><<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolDF<0>>), st>>>(
+          A, PolDF<0>::Consts{kconsts_df(K), kconsts_f(K)}, b0, partial, counters);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     e = capSlots >= nb ? strict::launch_reduce_all(partial, npad, numSeg, out, st)
@@ -163,24 +159,28 @@ cudaError_t launch_segseg_all_df(const KConsts& K, const double* soa, const floa
   return cudaSuccess;
 }
 
-cudaError_t launch_segseg_rows_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
-                                  int64_t npad, const int64_t* rows, int64_t nRows, double* partial, double* out,
-                                  unsigned long long* counters, cudaStream_t st, int form) {
-  cudaError_t e = form ? set_attr_df<1, 1>() : set_attr_df<1, 0>();
-  if (e != cudaSuccess) return e;
-  const int64_t nJt = npad / TILE;
-  const int64_t nrt = (nRows + TILE - 1) / TILE;
-  const unsigned grid = (unsigned)(nrt * nJt);
+cudaError_t launch_segseg_small_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
+                                   int64_t npad, void* scratch, double* partial, double* out, int64_t numSeg,
+                                   unsigned long long* counters, cudaStream_t st, int form) {
+  const int64_t nt = npad / TILE, nb = nt * (nt + 1) / 2;
   const TileArgs A{K, soa, skip, npad, soadf, nullptr};
-  if (form)
-    segseg_tile_df<1, 1><<<grid, TILE, sizeof(TileSmemT<TILE, PolDF<1>>), st>>>(
-        A, PolDF<1>::Consts{kconsts_df(K), kconsts_f(K)}, rows, nRows, nJt, 0, partial, counters);
-  else
-    segseg_tile_df<1, 0><<<grid, TILE, sizeof(TileSmemT<TILE, PolDF<0>>), st>>>(
-        A, PolDF<0>::Consts{kconsts_df(K), kconsts_f(K)}, rows, nRows, nJt, 0, partial, counters);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  return strict::launch_reduce_rows(partial, npad, nRows, out, st);
+  const KConstsDF kd = kconsts_df(K);
+  const KConstsF kf = kconsts_f(K);
+  cudaError_t e =
+      form ? launch_expanded<PolDF<1>>(A, PolDF<1>::Consts{kd, kf}, nb, scratch, partial, counters, st)
+           : launch_expanded<PolDF<0>>(A, PolDF<0>::Consts{kd, kf}, nb, scratch, partial, counters, st);
+  return e != cudaSuccess ? e : strict::launch_reduce_all(partial, npad, numSeg, out, st);
+}
+
+cudaError_t launch_segseg_rows_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
+                                  int64_t npad, const int64_t* rows, int64_t nRows, const RowPlan& plan,
+                                  double* partial, double* out, unsigned long long* counters, cudaStream_t st,
+                                  int form) {
+  const TileArgs A{K, soa, skip, npad, soadf, nullptr};
+  const KConstsDF kd = kconsts_df(K);
+  const KConstsF kf = kconsts_f(K);
+  return form ? launch_rows<PolDF<1>>(A, PolDF<1>::Consts{kd, kf}, rows, nRows, plan, partial, out, counters, st)
+              : launch_rows<PolDF<0>>(A, PolDF<0>::Consts{kd, kf}, rows, nRows, plan, partial, out, counters, st);
 }
 
 }  // namespace ddd

@@ -17,13 +17,13 @@
 //   serialise warps.  The CTA writes its two partial force blocks (forces on the
 //   I tile, forces on the J tile) to scratch; segseg_reduce sums them per segment
 //   in a fixed order.  Everything is deterministic: same inputs, same bits.
-// Index list (calcSegSegForce(..., idx), DislocationForces.jl:831-877):
-//   same kernel with ROWS mode: row slots come from idx, every j != i is paired,
-//   only Fnode1/Fnode2 are computed, partials per (row tile, J tile).
+// Small networks and the index list (calcSegSegForce(..., idx),
+// DislocationForces.jl:831-877): segseg_small.cuh.
 #include <cuda_runtime.h>
 
 #include "ddd_internal.h"
 #include "pair_f64.cuh"
+#include "segseg_small.cuh"
 #include "tile_body.cuh"
 
 // This file is compiled twice: DDD_VARIANT=strict with --fmad=false (every
@@ -115,25 +115,16 @@ __device__ __forceinline__ void tile_index(int64_t b, int64_t& I, int64_t& J) {
   I = b - Jc * (Jc + 1) / 2;
 }
 
-// MODE 0: all pairs (symmetric, i < j), one CTA per tile pair I <= J; the
-//         launch covers slots base.. (a band of J columns), its partial blocks
-//         indexed from base.
-// MODE 1: index rows (all j != i, F12 only), one CTA per (row tile, column tile).
-template <int MODE>
+// All pairs (i < j), one CTA per tile pair I <= J; the launch covers slots
+// base.. (a band of J columns), its partial blocks indexed from base.
 __global__ void __launch_bounds__(TILE, 2)
-segseg_tile_f64(TileArgs A, const int64_t* __restrict__ rows, int64_t nRows, int64_t nJt, int64_t base,
-                double* __restrict__ partial, unsigned long long* __restrict__ counters) {
+segseg_tile_f64(TileArgs A, int64_t base, double* __restrict__ partial, unsigned long long* __restrict__ counters) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& sm = *reinterpret_cast<TileSmemT<TILE, PolF64>*>(smem_raw);
   int64_t I, J;
-  if (MODE == 0) {
-    tile_index(base + blockIdx.x, I, J);
-  } else {
-    I = blockIdx.x / nJt;
-    J = blockIdx.x % nJt;
-  }
-  tile_body<TILE, MODE, PolF64>(A, PolF64::Consts{}, sm, I * TILE, J * TILE, MODE == 0 && I == J, rows, nRows,
-                                partial + (int64_t)blockIdx.x * (MODE == 0 ? 12 : 6) * TILE, counters);
+  tile_index(base + blockIdx.x, I, J);
+  tile_body<TILE, 0, PolF64>(A, PolF64::Consts{}, sm, I * TILE, J * TILE, I == J,
+                             partial + (int64_t)blockIdx.x * 12 * TILE, counters);
 }
 
 // Sum the partial blocks of each segment in a fixed order and write the
@@ -198,23 +189,6 @@ __global__ void segseg_reduce_band(const double* __restrict__ partial, int64_t J
   for (int c = 0; c < 6; ++c) out[6 * s + c] = acc[c];
 }
 
-// Index rows: row r (slot in the idx list) collects its nJt column blocks.
-__global__ void segseg_reduce_rows(const double* __restrict__ partial, int64_t nJt, int64_t nRows,
-                                   double* __restrict__ out) {
-  int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= nRows) return;
-  const int64_t A = r / TILE;
-  const int t = (int)(r % TILE);
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int64_t Jt = 0; Jt < nJt; ++Jt) {
-    const double* p = partial + (A * nJt + Jt) * 6 * TILE;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) acc[c] += p[c * TILE + t];
-  }
-#pragma unroll
-  for (int c = 0; c < 6; ++c) out[6 * r + c] = acc[c];
-}
-
 // ---------------------------------------------------------------------------
 // Host launchers.
 int64_t segseg_npad(int64_t numSeg) { return ((numSeg + TILE - 1) / TILE) * TILE; }
@@ -223,11 +197,6 @@ size_t segseg_partial_bytes_all(int64_t npad) {
   int64_t nt = npad / TILE;
   return (size_t)(nt * (nt + 1) / 2) * 12 * TILE * sizeof(double);
 }
-size_t segseg_partial_bytes_rows(int64_t nRows, int64_t npad) {
-  int64_t nrt = (nRows + TILE - 1) / TILE, nJt = npad / TILE;
-  return (size_t)(nrt * nJt) * 6 * TILE * sizeof(double);
-}
-
 cudaError_t launch_prep_segments(const double* coord, const double* bVec, const int64_t* segIdx, int64_t ld,
                                  const uint8_t* extSeg, int64_t numSeg, int64_t npad, double* soa, uint8_t* skip,
                                  cudaStream_t st) {
@@ -242,17 +211,16 @@ cudaError_t launch_prep_segments_packed(const double* in, int64_t ldIn, const ui
   return cudaGetLastError();
 }
 
-template <int MODE>
 static cudaError_t set_attr() {
   static std::atomic<uint64_t> done{0};
-  return set_smem_once(segseg_tile_f64<MODE>, (int)sizeof(TileSmemT<TILE, PolF64>), done);
+  return set_smem_once(segseg_tile_f64, (int)sizeof(TileSmemT<TILE, PolF64>), done);
 }
 
 // Loads the all-pairs kernels on the current device (under lazy module loading
 // the driver loads a kernel, and reserves its memory, at first use) and sets
 // the tile kernel's shared-memory attribute, without launching anything.
 cudaError_t preload_all_f64() {
-  cudaError_t e = set_attr<0>();
+  cudaError_t e = set_attr();
   cudaFuncAttributes fa;
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, prep_segments_packed);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, segseg_reduce_all);
@@ -279,22 +247,16 @@ cudaError_t launch_reduce_band(const double* partial, int64_t J0, int64_t J1, in
   return cudaGetLastError();
 }
 
-cudaError_t launch_reduce_rows(const double* partial, int64_t npad, int64_t nRows, double* out, cudaStream_t st) {
-  segseg_reduce_rows<<<(unsigned)((nRows + 127) / 128), 128, 0, st>>>(partial, npad / TILE, nRows, out);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_segseg_all_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                                   double* partial, double* out, int64_t numSeg, unsigned long long* counters,
                                   cudaStream_t st, int64_t capSlots) {
-  cudaError_t e = set_attr<0>();
+  cudaError_t e = set_attr();
   if (e != cudaSuccess) return e;
   const int64_t nt = npad / TILE;
   const int64_t nb = nt * (nt + 1) / 2;
   const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
   if (capSlots >= nb) {
-    segseg_tile_f64<0><<<(unsigned)nb, TILE, sizeof(TileSmemT<TILE, PolF64>), st>>>(A, nullptr, 0, 0, 0, partial,
-                                                                                    counters);
+    segseg_tile_f64<<<(unsigned)nb, TILE, sizeof(TileSmemT<TILE, PolF64>), st>>>(A, 0, partial, counters);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     segseg_reduce_all<<<(unsigned)((numSeg + 127) / 128), 128, 0, st>>>(partial, nt, numSeg, out);
@@ -304,8 +266,7 @@ cudaError_t launch_segseg_all_f64(const KConsts& K, const double* soa, const uin
   for (int64_t J0 = 0; J0 < nt;) {
     const int64_t J1 = segseg_band_end(J0, nt, capSlots);
     const int64_t b0 = J0 * (J0 + 1) / 2, nbb = J1 * (J1 + 1) / 2 - b0;
-    segseg_tile_f64<0><<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolF64>), st>>>(A, nullptr, 0, 0, b0, partial,
-                                                                                     counters);
+    segseg_tile_f64<<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolF64>), st>>>(A, b0, partial, counters);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     e = launch_reduce_band(partial, J0, J1, numSeg, out, st);
@@ -315,20 +276,20 @@ cudaError_t launch_segseg_all_f64(const KConsts& K, const double* soa, const uin
   return cudaSuccess;
 }
 
-cudaError_t launch_segseg_rows_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
-                                   const int64_t* rows, int64_t nRows, double* partial, double* out,
-                                   unsigned long long* counters, cudaStream_t st) {
-  cudaError_t e = set_attr<1>();
-  if (e != cudaSuccess) return e;
-  const int64_t nJt = npad / TILE;
-  const int64_t nrt = (nRows + TILE - 1) / TILE;
+cudaError_t launch_segseg_small_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
+                                    void* scratch, double* partial, double* out, int64_t numSeg,
+                                    unsigned long long* counters, cudaStream_t st) {
+  const int64_t nt = npad / TILE;
   const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
-  segseg_tile_f64<1><<<(unsigned)(nrt * nJt), TILE, sizeof(TileSmemT<TILE, PolF64>), st>>>(A, rows, nRows, nJt, 0,
-                                                                                           partial, counters);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  segseg_reduce_rows<<<(unsigned)((nRows + 127) / 128), 128, 0, st>>>(partial, nJt, nRows, out);
-  return cudaGetLastError();
+  cudaError_t e = launch_expanded<PolF64>(A, PolF64::Consts{}, nt * (nt + 1) / 2, scratch, partial, counters, st);
+  return e != cudaSuccess ? e : launch_reduce_all(partial, npad, numSeg, out, st);
+}
+
+cudaError_t launch_segseg_rows_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
+                                   const int64_t* rows, int64_t nRows, const RowPlan& plan, double* partial,
+                                   double* out, unsigned long long* counters, cudaStream_t st) {
+  const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
+  return launch_rows<PolF64>(A, PolF64::Consts{}, rows, nRows, plan, partial, out, counters, st);
 }
 
 }  // namespace DDD_VARIANT

@@ -14,6 +14,7 @@
 
 #include "ddd_internal.h"
 #include "pair_f64.cuh"
+#include "segseg_small.cuh"
 #include "tile_pol_fx.cuh"
 
 namespace ddd {
@@ -30,29 +31,20 @@ __device__ __forceinline__ void tile_index_fx(int64_t b, int64_t& I, int64_t& J)
   I = b - Jc * (Jc + 1) / 2;
 }
 
-// MODE 0: all pairs, one CTA per tile pair I <= J of the band starting at slot
-// `base`; MODE 1: index rows, one CTA per (row tile, column tile).
-template <int MODE>
+// All pairs, one CTA per tile pair I <= J of the band starting at slot `base`.
 __global__ void __launch_bounds__(TILE, 2)
-segseg_tile_fx(TileArgs A, const int64_t* __restrict__ rows, int64_t nRows, int64_t nJt, int64_t base,
-               double* __restrict__ partial, unsigned long long* __restrict__ counters) {
+segseg_tile_fx(TileArgs A, int64_t base, double* __restrict__ partial, unsigned long long* __restrict__ counters) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& sm = *reinterpret_cast<TileSmemT<TILE, PolF64Fast>*>(smem_raw);
   int64_t I, J;
-  if (MODE == 0) {
-    tile_index_fx(base + blockIdx.x, I, J);
-  } else {
-    I = blockIdx.x / nJt;
-    J = blockIdx.x % nJt;
-  }
-  tile_body<TILE, MODE, PolF64Fast>(A, PolF64Fast::Consts{}, sm, I * TILE, J * TILE, MODE == 0 && I == J, rows,
-                                    nRows, partial + (int64_t)blockIdx.x * (MODE == 0 ? 12 : 6) * TILE, counters);
+  tile_index_fx(base + blockIdx.x, I, J);
+  tile_body<TILE, 0, PolF64Fast>(A, PolF64Fast::Consts{}, sm, I * TILE, J * TILE, I == J,
+                                 partial + (int64_t)blockIdx.x * 12 * TILE, counters);
 }
 
-template <int MODE>
 cudaError_t set_attr_fx() {
   static std::atomic<uint64_t> done{0};
-  return set_smem_once(segseg_tile_fx<MODE>, (int)sizeof(TileSmemT<TILE, PolF64Fast>), done);
+  return set_smem_once(segseg_tile_fx, (int)sizeof(TileSmemT<TILE, PolF64Fast>), done);
 }
 
 }  // namespace
@@ -60,7 +52,7 @@ cudaError_t set_attr_fx() {
 cudaError_t launch_segseg_all_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                                  double* partial, double* out, int64_t numSeg, unsigned long long* counters,
                                  cudaStream_t st, int64_t capSlots) {
-  cudaError_t e = set_attr_fx<0>();
+  cudaError_t e = set_attr_fx();
   if (e != cudaSuccess) return e;
   const int64_t nt = npad / TILE;
   const int64_t nb = nt * (nt + 1) / 2;
@@ -70,8 +62,7 @@ cudaError_t launch_segseg_all_fx(const KConsts& K, const double* soa, const uint
   for (int64_t J0 = 0; J0 < nt;) {
     const int64_t J1 = capSlots >= nb ? nt : strict::segseg_band_end(J0, nt, capSlots);
     const int64_t b0 = J0 * (J0 + 1) / 2, nbb = J1 * (J1 + 1) / 2 - b0;
-    segseg_tile_fx<0><<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolF64Fast>), st>>>(A, nullptr, 0, 0, b0,
-                                                                                         partial, counters);
+    segseg_tile_fx<<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolF64Fast>), st>>>(A, b0, partial, counters);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     e = capSlots >= nb ? strict::launch_reduce_all(partial, npad, numSeg, out, st)
@@ -82,19 +73,21 @@ cudaError_t launch_segseg_all_fx(const KConsts& K, const double* soa, const uint
   return cudaSuccess;
 }
 
-cudaError_t launch_segseg_rows_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
-                                  const int64_t* rows, int64_t nRows, double* partial, double* out,
-                                  unsigned long long* counters, cudaStream_t st) {
-  cudaError_t e = set_attr_fx<1>();
-  if (e != cudaSuccess) return e;
-  const int64_t nJt = npad / TILE;
-  const int64_t nrt = (nRows + TILE - 1) / TILE;
+cudaError_t launch_segseg_small_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
+                                   void* scratch, double* partial, double* out, int64_t numSeg,
+                                   unsigned long long* counters, cudaStream_t st) {
+  const int64_t nt = npad / TILE;
   const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
-  segseg_tile_fx<1><<<(unsigned)(nrt * nJt), TILE, sizeof(TileSmemT<TILE, PolF64Fast>), st>>>(A, rows, nRows, nJt, 0,
-                                                                                              partial, counters);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  return strict::launch_reduce_rows(partial, npad, nRows, out, st);
+  cudaError_t e =
+      launch_expanded<PolF64Fast>(A, PolF64Fast::Consts{}, nt * (nt + 1) / 2, scratch, partial, counters, st);
+  return e != cudaSuccess ? e : strict::launch_reduce_all(partial, npad, numSeg, out, st);
+}
+
+cudaError_t launch_segseg_rows_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
+                                  const int64_t* rows, int64_t nRows, const RowPlan& plan, double* partial,
+                                  double* out, unsigned long long* counters, cudaStream_t st) {
+  const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
+  return launch_rows<PolF64Fast>(A, PolF64Fast::Consts{}, rows, nRows, plan, partial, out, counters, st);
 }
 
 }  // namespace ddd

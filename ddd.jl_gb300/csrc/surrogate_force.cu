@@ -233,7 +233,7 @@ exact_tiles(TileArgs A, typename P::Consts KP, const int4* __restrict__ items, c
     const int32_t w = s_item;
     if (w >= nItems) break;
     const int4 it = items[w];
-    tile_body<T, MODE, P>(A, KP, sm, it.y, it.z, it.w != 0, nullptr, 0, partial + (int64_t)it.x * 12 * T, counters);
+    tile_body<T, MODE, P>(A, KP, sm, it.y, it.z, it.w != 0, partial + (int64_t)it.x * 12 * T, counters);
   }
 }
 

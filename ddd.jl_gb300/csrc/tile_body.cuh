@@ -1,9 +1,8 @@
 // One tile pair of the seg-seg force: the body shared by every seg-seg kernel
-// (all-pairs, index rows, batched persistent), templated on
+// (all-pairs, batched persistent, the surrogate's exact passes), templated on
 //   T     tile size (segments per side = threads per CTA; 64 or 128),
-//   MODE  0 = unordered pairs i < j (both sides' forces), 1 = index rows (all
-//         j != i, forces on the row segment only), 2 = the pairs i < j outside
-//         the surrogate's trust region (near pairs; forces added to `p`),
+//   MODE  0 = unordered pairs i < j (both sides' forces), 2 = the pairs i < j
+//         outside the surrogate's trust region (near pairs; forces added to `p`),
 //   P     arithmetic policy (FP64, df64, mixed FP32; pair_f64.cuh / pair_df.cuh).
 //
 // Thread t owns row segment i (registers); the column tile sits in shared
@@ -12,9 +11,11 @@
 // per-warp shared arrays.  Near-parallel pairs (1 - c^2 <= sqrt(eps)) are only
 // flagged during the sweep, then compacted in a fixed order (by row, then by
 // step) and evaluated densely, T at a time, with the FP64 calcParSegSegForce.
-// The block's partial forces — 6 per row segment, and in MODE 0 6 per column
-// segment — are written to `p` as [side][component][T] doubles.  No
-// floating-point atomics: the result is deterministic.
+// The block's partial forces — 6 per row segment, 6 per column segment — are
+// written to `p` as [side][component][T] doubles.  A column segment's
+// near-parallel forces are summed warp of rows by warp of rows, then over the
+// warps (segseg_small.cuh adds in the same order).  No floating-point atomics:
+// the result is deterministic.
 //
 // In MODE 2 every selected pair goes through the compacted dense pass.  The
 // sweep takes the reference's FP64 branch decision for each selected pair and
@@ -67,25 +68,15 @@ struct TileSmemT {
 
 template <int T, int MODE, class P>
 __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::Consts& KP, TileSmemT<T, P>& sm,
-                                          int64_t iBase, int64_t j0, bool diag, const int64_t* __restrict__ rows,
-                                          int64_t nRows, double* __restrict__ p,
+                                          int64_t iBase, int64_t j0, bool diag, double* __restrict__ p,
                                           unsigned long long* __restrict__ counters) {
   constexpr int NW = T / 32;
   constexpr int CH = T;
   const int t = threadIdx.x;
   const int warp = t >> 5;
 
-  int64_t gi;
-  bool iActive;
-  if (MODE != 1) {
-    gi = iBase + t;
-    iActive = A.skip[gi] == 0;
-  } else {
-    const int64_t r = iBase + t;
-    iActive = r < nRows;
-    gi = iActive ? rows[r] : 0;
-    iActive = iActive && A.skip[gi] == 0;
-  }
+  const int64_t gi = iBase + t;
+  const bool iActive = A.skip[gi] == 0;
   constexpr bool CLS = MODE == 2;  // classified mode: dense pass only
   typename P::Seg si;
   if (!CLS) si = P::load_global(A, gi);
@@ -115,9 +106,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
 
   for (int k = 0; k < T; ++k) {
     const int jl = (t + k) & (T - 1);
-    bool act = iActive && sm.skip[jl] == 0;
-    if (MODE != 1) act = act && (!diag || jl > t);
-    if (MODE == 1) act = act && (j0 + jl != gi);
+    const bool act = iActive && sm.skip[jl] == 0 && (!diag || jl > t);
     if (CLS) {
       if (act) {
         const int64_t n = A.npad, gj = j0 + jl;
@@ -139,12 +128,8 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
       typename P::Scalar c;
       if (P::is_general(A, si, sj, gi, j0 + jl, c)) {
         typename P::Vec F1, F2, F3, F4;
-        if (MODE == 0) {
-          P::template general<true>(KP, A, si, sj, c, F1, F2, F3, F4);
-          P::template add_col<T>(sm.pol, warp, jl, F3, F4);
-        } else {
-          P::template general<false>(KP, A, si, sj, c, F1, F2, F3, F4);
-        }
+        P::template general<true>(KP, A, si, sj, c, F1, F2, F3, F4);
+        P::template add_col<T>(sm.pol, warp, jl, F3, F4);
         P::acc_add(fi1, F1);
         P::acc_add(fi2, F2);
         ++nGeneral;
@@ -216,6 +201,8 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
   __syncthreads();
   const int nPar = sm.total;
   D3 fp1 = {0, 0, 0}, fp2 = {0, 0, 0}, fjp3 = {0, 0, 0}, fjp4 = {0, 0, 0};
+  D3 fjt3 = {0, 0, 0}, fjt4 = {0, 0, 0};  // MODE 0: column sums of the warps before jw
+  int jw = 0;
   unsigned long long nCore = 0;
   // Chunks of CH never straddle the two runs, so a warp runs one branch.
   for (int base = 0; base < nPar;) {
@@ -229,15 +216,11 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
         P::dense_general(KP, A, iBase + il, j0 + jl, F1, F2, F3, F4);
         ++nGeneral;
       } else {
-        SegF64 a = tb_load_seg64(A.soa, A.npad, MODE != 1 ? iBase + il : rows[iBase + il]);
+        SegF64 a = tb_load_seg64(A.soa, A.npad, iBase + il);
         SegF64 b = tb_load_seg64(A.soa, A.npad, j0 + jl);
         double c = dot(a.t, b.t);
-        if (MODE != 1) {
-          ++nDenseParallel;
-          nCore += parallel_pair<true>(A.K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, c, F1, F2, F3, F4);
-        } else {
-          nCore += parallel_pair<false>(A.K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, c, F1, F2, F3, F4);
-        }
+        ++nDenseParallel;
+        nCore += parallel_pair<true>(A.K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, c, F1, F2, F3, F4);
       }
       sm.cf[t][0] = F1.x; sm.cf[t][1] = F1.y; sm.cf[t][2] = F1.z;
       sm.cf[t][3] = F2.x; sm.cf[t][4] = F2.y; sm.cf[t][5] = F2.z;
@@ -263,13 +246,18 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
         fp2 = fp2 + D3{f[3], f[4], f[5]};
       }
     }
-    if (MODE != 1) {
-      for (int q = 0; q < lim; ++q) {
-        if ((sm.plist[base + q] & 0xff) == t) {
-          const double* f = sm.cf[q];
-          fjp3 = fjp3 + D3{f[6], f[7], f[8]};
-          fjp4 = fjp4 + D3{f[9], f[10], f[11]};
+    for (int q = 0; q < lim; ++q) {
+      const int pe = sm.plist[base + q];
+      if ((pe & 0xff) == t) {
+        if (!CLS && (pe >> 13) != jw) {  // the rows of the next warp
+          fjt3 = fjt3 + fjp3;
+          fjt4 = fjt4 + fjp4;
+          fjp3 = fjp4 = {0, 0, 0};
+          jw = pe >> 13;
         }
+        const double* f = sm.cf[q];
+        fjp3 = fjp3 + D3{f[6], f[7], f[8]};
+        fjp4 = fjp4 + D3{f[9], f[10], f[11]};
       }
     }
     __syncthreads();
@@ -304,11 +292,11 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
   p[3 * T + t] = r2.x + fp2.x;
   p[4 * T + t] = r2.y + fp2.y;
   p[5 * T + t] = r2.z + fp2.z;
-  if (MODE == 0) {
-    const double add[6] = {fjp3.x, fjp3.y, fjp3.z, fjp4.x, fjp4.y, fjp4.z};
+  fjt3 = fjt3 + fjp3;
+  fjt4 = fjt4 + fjp4;
+  const double add[6] = {fjt3.x, fjt3.y, fjt3.z, fjt4.x, fjt4.y, fjt4.z};
 #pragma unroll
-    for (int c = 0; c < 6; ++c) p[(6 + c) * T + t] = P::template col_sum<T>(sm.pol, c, t) + add[c];
-  }
+  for (int c = 0; c < 6; ++c) p[(6 + c) * T + t] = P::template col_sum<T>(sm.pol, c, t) + add[c];
 
   if (counters) {
     unsigned long long g = nGeneral, cc = nCore;
@@ -390,6 +378,12 @@ struct PolF64 {
     fj[4 * T + j] += F4.y;
     fj[5 * T + j] += F4.z;
   }
+  // One component as segseg_small.cuh stores and adds it.
+  using Comp = double;
+  static __device__ __forceinline__ double pack(double v) { return v; }
+  static __device__ __forceinline__ double unpack(double v) { return v; }
+  static __device__ __forceinline__ double comp_zero() { return 0.0; }
+  static __device__ __forceinline__ double comp_to_double(double v) { return v; }
   static __device__ __forceinline__ D3 acc_zero() { return {0, 0, 0}; }
   static __device__ __forceinline__ void acc_add(D3& a, const D3& v) { a = a + v; }
   static __device__ __forceinline__ D3 acc_to_d3(const D3& a) { return a; }

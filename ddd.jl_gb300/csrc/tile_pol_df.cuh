@@ -129,6 +129,16 @@ struct PolDF {
     add_df(s.fj[warp][4][j], F4.y);
     add_df(s.fj[warp][5][j], F4.z);
   }
+  // One component as segseg_small.cuh stores (hi, lo in 8 bytes) and adds it.
+  using Comp = df64;
+  static __device__ __forceinline__ double pack(df64 v) {
+    return __hiloint2double(__float_as_int(v.hi), __float_as_int(v.lo));
+  }
+  static __device__ __forceinline__ df64 unpack(double v) {
+    return {__int_as_float(__double2hiint(v)), __int_as_float(__double2loint(v))};
+  }
+  static __device__ __forceinline__ df64 comp_zero() { return df(0.f); }
+  static __device__ __forceinline__ double comp_to_double(df64 v) { return df_to_double(v); }
   static __device__ __forceinline__ DV3 acc_zero() { return {df(0.f), df(0.f), df(0.f)}; }
   static __device__ __forceinline__ void acc_add(DV3& a, const DV3& v) { a = a + v; }
   static __device__ __forceinline__ D3 acc_to_d3(const DV3& a) {

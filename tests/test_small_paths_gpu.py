@@ -1,0 +1,56 @@
+"""The kernels whose unit of work is a step of pairs: small all-pairs networks (every pair's forces
+stored, then folded) and the index list.
+
+The fold adds in the tile kernel's order, so with a partial-sum limit that
+leaves room for the tile kernel's slots but not for the pair store (the tile
+kernel then runs) the forces are equal bit for bit, in every arithmetic."""
+import numpy as np
+import pytest
+
+from conftest import k5_of
+from test_segseg_gpu import _params, _synthetic, check_forces
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode", ["fp64", "fp64_fma", "fp64_fast", "df64", "f32c"])
+@pytest.mark.parametrize("n", [1, 2, 24, 33, 128, 129, 1001, 2176])
+def test_expanded_equals_tile_kernel(pkg, synth, mode, n):
+    net = _synthetic(pkg, synth, (n + 7) // 8, 90 + n, parallel_fraction=0.2, cube=3000.0)
+    net.numSeg = n
+    net.extSeg[5::17] = 1
+    dln, mat = _params(pkg)
+    ctx = pkg.get_context()
+    nt = -(-n // 128)
+    ctx.mode = mode
+    try:
+        F = pkg.calcSegSegForce(dln, mat, net)
+        rep = dict(ctx.last_report)
+        ctx.partial_limit = nt * (nt + 1) // 2 * 12288
+        T = pkg.calcSegSegForce(dln, mat, net)
+        rep_t = dict(ctx.last_report)
+    finally:
+        ctx.mode, ctx.partial_limit = "fp64", 0
+    if mode == "fp64_fma":  # the compiler contracts each kernel on its own
+        assert np.linalg.norm(F - T) <= 1e-10 * np.linalg.norm(T)
+    else:
+        assert np.array_equal(F, T)
+    for key in ("pairs_general", "pairs_parallel", "core_sides"):
+        assert rep[key] == rep_t[key]
+
+
+@pytest.mark.parametrize("n,rows", [(2, 1), (33, 40), (2017, 1), (2017, 600)])
+def test_index_rows(pkg, synth, oracle, n, rows):
+    """One step and seven steps per CTA (600 rows of 2,017 segments), columns
+    that end inside a block, repeated and external rows."""
+    net = _synthetic(pkg, synth, (n + 7) // 8, 7 + n, parallel_fraction=0.2, cube=3000.0)
+    net.numSeg = n
+    if n > 2:
+        net.extSeg[[4, 30]] = 1
+    dln, mat = _params(pkg)
+    k5 = k5_of(dln, mat)
+    idx = np.random.default_rng(n + rows).integers(1, n + 1, rows)
+    if n > 2 and rows > 2:
+        idx[:3] = [5, n, n]
+    Fi = pkg.calcSegSegForce(dln, mat, net, idx)
+    check_forces(Fi, oracle, k5, net, rows=idx - 1, ref=oracle.segseg_idx(k5, net, idx))
