@@ -20,6 +20,7 @@
 #pragma once
 #include <cstdint>
 
+#include "f64reg.cuh"
 #include "intmath_f64.cuh"
 
 namespace ddd {
@@ -36,16 +37,18 @@ constexpr double kHCotanThetac = 4075.672300430329;
 struct D3 {
   double x, y, z;
 };
-__device__ __forceinline__ D3 operator+(D3 a, D3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ D3 operator-(D3 a, D3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+// Sums and products through rd (f64reg.cuh): the plain operations' bits.
+__device__ __forceinline__ D3 d3(rd x, rd y, rd z) { return {x, y, z}; }
+__device__ __forceinline__ D3 operator+(D3 a, D3 b) { return d3(rd(a.x) + b.x, rd(a.y) + b.y, rd(a.z) + b.z); }
+__device__ __forceinline__ D3 operator-(D3 a, D3 b) { return d3(rd(a.x) - b.x, rd(a.y) - b.y, rd(a.z) - b.z); }
 __device__ __forceinline__ D3 operator-(D3 a) { return {-a.x, -a.y, -a.z}; }
-__device__ __forceinline__ D3 operator*(double s, D3 a) { return {s * a.x, s * a.y, s * a.z}; }
-__device__ __forceinline__ D3 operator*(D3 a, double s) { return {a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ double dot(D3 a, D3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ D3 operator*(rd s, D3 a) { return d3(s * a.x, s * a.y, s * a.z); }
+__device__ __forceinline__ D3 operator*(D3 a, rd s) { return d3(a.x * s, a.y * s, a.z * s); }
+__device__ __forceinline__ rd dot(D3 a, D3 b) { return rd(a.x) * b.x + rd(a.y) * b.y + rd(a.z) * b.z; }
 __device__ __forceinline__ D3 cross(D3 a, D3 b) {
-  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+  return d3(rd(a.y) * b.z - rd(a.z) * b.y, rd(a.z) * b.x - rd(a.x) * b.z, rd(a.x) * b.y - rd(a.y) * b.x);
 }
-__device__ __forceinline__ double norm(D3 a) { return sqrt(a.x * a.x + a.y * a.y + a.z * a.z); }
+__device__ __forceinline__ rd norm(D3 a) { return sqrt(rd(a.x) * a.x + rd(a.y) * a.y + rd(a.z) * a.z); }
 
 // One segment as the pair kernels see it.
 struct SegF64 {
@@ -60,57 +63,57 @@ __device__ __forceinline__ void seg_direction(D3 n1, D3 n2, D3& t, double& tN) {
 }
 
 // v with its sign flipped when sm is the sign-bit mask (integer pipe, exact).
-__device__ __forceinline__ double sgn(double v, unsigned long long sm) {
+__device__ __forceinline__ rd sgn(rd v, unsigned long long sm) {
   return __longlong_as_double(__double_as_longlong(v) ^ (long long)sm);
 }
 
 // SegSegInteg at one corner, added (sm = 0) or subtracted (sm = sign bit) into integ[19].
 // aSq_dSq = aSq + d^2 (1 - c^2) and den = 1 / sqrt((1 - c^2) aSq_dSq) do not depend
 // on the corner; the caller computes them once per pair with the same operations.
-__device__ __forceinline__ void seg_seg_integ_acc(double aSq_dSq, double den, double c, double cSq, double omcSqI,
-                                                  double x, double y, unsigned long long sm, double* integ) {
-  double xSq = x * x;
-  double ySq = y * y;
-  double Ra = sqrt(aSq_dSq + xSq + ySq + 2.0 * x * y * c);
-  double RaInv = 1.0 / Ra;
+__device__ __forceinline__ void seg_seg_integ_acc(rd aSq_dSq, rd den, rd c, rd cSq, rd omcSqI,
+                                                  rd x, rd y, unsigned long long sm, rd* integ) {
+  rd xSq = x * x;
+  rd ySq = y * y;
+  rd Ra = sqrt(aSq_dSq + xSq + ySq + twice(x) * y * c);
+  rd RaInv = 1.0 / Ra;
 
-  double Ra_Rd_t1 = Ra + y + x * c;
-  double Ra_Rd_t2 = Ra + x + y * c;
+  rd Ra_Rd_t1 = Ra + y + x * c;
+  rd Ra_Rd_t2 = Ra + x + y * c;
 
-  double log_Ra_Rd_t1 = im::log(Ra_Rd_t1);
-  double xlog_Ra_Rd_t1 = x * log_Ra_Rd_t1;
-  double log_Ra_Rd_t2 = im::log(Ra_Rd_t2);
-  double ylog_Ra_Rd_t2 = y * log_Ra_Rd_t2;
+  rd log_Ra_Rd_t1 = im::log(Ra_Rd_t1);
+  rd xlog_Ra_Rd_t1 = x * log_Ra_Rd_t1;
+  rd log_Ra_Rd_t2 = im::log(Ra_Rd_t2);
+  rd ylog_Ra_Rd_t2 = y * log_Ra_Rd_t2;
 
-  double RaSq_R_t1_I = RaInv / Ra_Rd_t1;
-  double xRaSq_R_t1_I = x * RaSq_R_t1_I;
-  double xSqRaSq_R_t1_I = x * xRaSq_R_t1_I;
+  rd RaSq_R_t1_I = RaInv / Ra_Rd_t1;
+  rd xRaSq_R_t1_I = x * RaSq_R_t1_I;
+  rd xSqRaSq_R_t1_I = x * xRaSq_R_t1_I;
 
-  double RaSq_R_t2_I = RaInv / Ra_Rd_t2;
-  double yRaSq_R_t2_I = y * RaSq_R_t2_I;
-  double ySqRaSq_R_t2_I = y * yRaSq_R_t2_I;
+  rd RaSq_R_t2_I = RaInv / Ra_Rd_t2;
+  rd yRaSq_R_t2_I = y * RaSq_R_t2_I;
+  rd ySqRaSq_R_t2_I = y * yRaSq_R_t2_I;
 
-  double integ1 = -2.0 * den * im::atan((1.0 + c) * (Ra + x + y) * den);
+  rd integ1 = -twice(den) * rd(im::atan((rd_one() + c) * (Ra + x + y) * den));
 
-  double c_1 = aSq_dSq * integ1;
-  double c_5_6 = (c * Ra - c_1) * omcSqI;
+  rd c_1 = aSq_dSq * integ1;
+  rd c_5_6 = (c * Ra - c_1) * omcSqI;
 
-  double integ2 = (c * log_Ra_Rd_t2 - log_Ra_Rd_t1) * omcSqI;
-  double integ3 = (c * log_Ra_Rd_t1 - log_Ra_Rd_t2) * omcSqI;
-  double integ4 = (c * c_1 - Ra) * omcSqI;
-  double integ5 = ylog_Ra_Rd_t2 + c_5_6;
-  double integ6 = xlog_Ra_Rd_t1 + c_5_6;
+  rd integ2 = (c * log_Ra_Rd_t2 - log_Ra_Rd_t1) * omcSqI;
+  rd integ3 = (c * log_Ra_Rd_t1 - log_Ra_Rd_t2) * omcSqI;
+  rd integ4 = (c * c_1 - Ra) * omcSqI;
+  rd integ5 = ylog_Ra_Rd_t2 + c_5_6;
+  rd integ6 = xlog_Ra_Rd_t1 + c_5_6;
 
-  double c_11_12 = integ1 - c * RaInv;
-  double c_15_18 = c * xRaSq_R_t1_I - RaInv;
-  double x_13_14 = x * c_15_18;
-  double c_19 = c * yRaSq_R_t2_I - RaInv;
-  double y_13_14 = y * c_19;
-  double c_16 = log_Ra_Rd_t2 - (x - c * y) * RaInv - cSq * ySqRaSq_R_t2_I;
-  double z_15_18 = y * c_16;
-  double c_17_19 = log_Ra_Rd_t1 - (y - c * x) * RaInv - cSq * xSqRaSq_R_t1_I;
+  rd c_11_12 = integ1 - c * RaInv;
+  rd c_15_18 = c * xRaSq_R_t1_I - RaInv;
+  rd x_13_14 = x * c_15_18;
+  rd c_19 = c * yRaSq_R_t2_I - RaInv;
+  rd y_13_14 = y * c_19;
+  rd c_16 = log_Ra_Rd_t2 - (x - c * y) * RaInv - cSq * ySqRaSq_R_t2_I;
+  rd z_15_18 = y * c_16;
+  rd c_17_19 = log_Ra_Rd_t1 - (y - c * x) * RaInv - cSq * xSqRaSq_R_t1_I;
 
-  double c15_18_19 = 2.0 * integ4;
+  rd c15_18_19 = twice(integ4);
 
   integ[0] += sgn(integ1, sm);
   integ[1] += sgn(integ2, sm);
@@ -127,13 +130,13 @@ __device__ __forceinline__ void seg_seg_integ_acc(double aSq_dSq, double den, do
   integ[12] += sgn(((integ3 - x_13_14 + c * (y_13_14 - integ2)) * omcSqI), sm);
   integ[13] += sgn(((integ2 - y_13_14 + c * (x_13_14 - integ3)) * omcSqI), sm);
   integ[14] += sgn(((integ5 - z_15_18 + c * (xSq * c_15_18 - c15_18_19)) * omcSqI), sm);
-  integ[15] += sgn(((xSqRaSq_R_t1_I + c * c_16 + 2.0 * integ2) * omcSqI), sm);
-  integ[16] += sgn(((ySqRaSq_R_t2_I + c * c_17_19 + 2.0 * integ3) * omcSqI), sm);
+  integ[15] += sgn(((xSqRaSq_R_t1_I + c * c_16 + twice(integ2)) * omcSqI), sm);
+  integ[16] += sgn(((ySqRaSq_R_t2_I + c * c_17_19 + twice(integ3)) * omcSqI), sm);
   integ[17] += sgn(((c15_18_19 - xSq * c_15_18 + c * (z_15_18 - integ5)) * omcSqI), sm);
   integ[18] += sgn(((c15_18_19 - ySq * c_19 + c * (x * c_17_19 - integ6)) * omcSqI), sm);
 }
 
-__device__ __forceinline__ D3 fsum11(const D3* V, const double* F) {
+__device__ __forceinline__ D3 fsum11(const D3* V, const rd* F) {
   D3 s = V[0] * F[0] + V[1] * F[1];
 #pragma unroll
   for (int k = 2; k < 11; ++k) s = s + V[k] * F[k];
@@ -143,27 +146,27 @@ __device__ __forceinline__ D3 fsum11(const D3* V, const double* F) {
 // General branch (1 - c^2 > sqrt(eps)) of calcSegSegForce.  NEED12 / NEED34 drop
 // the work of the forces on segment 1 / segment 2 when the caller discards them.
 template <bool NEED12, bool NEED34>
-__device__ __forceinline__ void general_pair(const KConsts& K, D3 b1, D3 n11, D3 n12, D3 t1, double t1N, D3 b2, D3 n21,
-                                             D3 n22, D3 t2, double t2N, double c, D3& F1, D3& F2, D3& F3, D3& F4) {
-  const double mu4pi = K.mu4pi, mu4pinu = K.mu4pinu, mu8piaSq = K.mu8piaSq, mu4pinuaSq = K.mu4pinuaSq;
-  double cSq = c * c;
-  double omcSq = 1.0 - cSq;
-  double omcSqI = 1.0 / omcSq;
+__device__ __forceinline__ void general_pair(const KConsts& K, D3 b1, D3 n11, D3 n12, D3 t1, rd t1N, D3 b2, D3 n21,
+                                             D3 n22, D3 t2, rd t2N, rd c, D3& F1, D3& F2, D3& F3, D3& F4) {
+  const rd mu4pi = K.mu4pi, mu4pinu = K.mu4pinu, mu8piaSq = K.mu8piaSq, mu4pinuaSq = K.mu4pinuaSq;
+  rd cSq = c * c;
+  rd omcSq = rd_one() - cSq;
+  rd omcSqI = 1.0 / omcSq;
 
   D3 t2ct1 = cross(t2, t1);
   D3 t1ct2 = -t2ct1;
   D3 b2ct2 = cross(b2, t2);
   D3 b1ct1 = cross(b1, t1);
 
-  double t2db2 = dot(t2, b2);
-  double t2db1 = dot(t2, b1);
-  double t1db2 = dot(t1, b2);
-  double t1db1 = dot(t1, b1);
+  rd t2db2 = dot(t2, b2);
+  rd t2db1 = dot(t2, b1);
+  rd t1db2 = dot(t1, b2);
+  rd t1db1 = dot(t1, b1);
 
-  double t2ct1db2 = dot(t2ct1, b2);
-  double t1ct2db1 = dot(t1ct2, b1);
-  double b1ct1db2 = dot(b1ct1, b2);
-  double b2ct2db1 = dot(b2ct2, b1);
+  rd t2ct1db2 = dot(t2ct1, b2);
+  rd t1ct2db1 = dot(t1ct2, b1);
+  rd b1ct1db2 = dot(b1ct1, b2);
+  rd b2ct2db1 = dot(b2ct2, b1);
 
   D3 t2ct1ct2 = t1 - c * t2;
   D3 t1ct2ct1 = t2 - c * t1;
@@ -172,48 +175,48 @@ __device__ __forceinline__ void general_pair(const KConsts& K, D3 b1, D3 n11, D3
   D3 b1ct1ct2 = t2db1 * t1 - c * b1;
   D3 b2ct2ct1 = t1db2 * t2 - c * b2;
 
-  double t2ct1cb1dt1 = t2db1 - t1db1 * c;
-  double t1ct2cb2dt2 = t1db2 - t2db2 * c;
-  double t2ct1cb1db2 = t2db1 * t1db2 - t1db1 * t2db2;
+  rd t2ct1cb1dt1 = t2db1 - t1db1 * c;
+  rd t1ct2cb2dt2 = t1db2 - t2db2 * c;
+  rd t2ct1cb1db2 = t2db1 * t1db2 - t1db1 * t2db2;
 
   D3 R1 = n21 - n11;
   D3 R2 = n22 - n12;
-  double d = dot(R2, t2ct1) * omcSqI;
+  rd d = dot(R2, t2ct1) * omcSqI;
 
-  double mu4pid = mu4pi * d;
-  double mu4pinud = mu4pinu * d;
-  double mu4pinudSq = mu4pinud * d;
-  double mu4pinudCu = mu4pinudSq * d;
-  double mu4pinuaSqd = mu4pinuaSq * d;
-  double mu8piaSqd = mu8piaSq * d;
+  rd mu4pid = mu4pi * d;
+  rd mu4pinud = mu4pinu * d;
+  rd mu4pinudSq = mu4pinud * d;
+  rd mu4pinudCu = mu4pinudSq * d;
+  rd mu4pinuaSqd = mu4pinuaSq * d;
+  rd mu8piaSqd = mu8piaSq * d;
 
-  double lim11 = dot(R1, t1);
-  double lim12 = dot(R1, t2);
-  double lim21 = dot(R2, t1);
-  double lim22 = dot(R2, t2);
+  rd lim11 = dot(R1, t1);
+  rd lim12 = dot(R1, t2);
+  rd lim21 = dot(R2, t1);
+  rd lim22 = dot(R2, t2);
 
-  double x1 = (lim12 - c * lim11) * omcSqI;
-  double x2 = (lim22 - c * lim21) * omcSqI;
-  double y1 = (lim11 - c * lim12) * omcSqI;
-  double y2 = (lim21 - c * lim22) * omcSqI;
+  rd x1 = (lim12 - c * lim11) * omcSqI;
+  rd x2 = (lim22 - c * lim21) * omcSqI;
+  rd y1 = (lim11 - c * lim12) * omcSqI;
+  rd y2 = (lim21 - c * lim22) * omcSqI;
 
-  double integ[19];
+  rd integ[19];
 #pragma unroll
   for (int k = 0; k < 19; ++k) integ[k] = 0.0;
-  const double aSq_dSq = K.aSq + d * d * omcSq;
-  const double den = 1.0 / sqrt(omcSq * aSq_dSq);
+  const rd aSq_dSq = K.aSq + d * d * omcSq;
+  const rd den = 1.0 / sqrt(omcSq * aSq_dSq);
   // ((I(x1,y1) - I(x1,y2)) - I(x2,y1)) + I(x2,y2), DislocationForces.jl:948-951.
 #pragma unroll 1
   for (int q = 0; q < 4; ++q) {
-    double x = (q & 2) ? x2 : x1;
-    double y = (q & 1) ? y2 : y1;
+    rd x = (q & 2) ? x2 : x1;
+    rd y = (q & 1) ? y2 : y1;
     unsigned long long sm = (q == 1 || q == 2) ? 0x8000000000000000ull : 0ull;
     seg_seg_integ_acc(aSq_dSq, den, c, cSq, omcSqI, x, y, sm, integ);
   }
 
   D3 V[11];
-  double Fi[11];
-  double tmp1, tmp2;
+  rd Fi[11];
+  rd tmp1, tmp2;
   if (NEED12) {
     tmp1 = t1db2 * t2db1 + t2ct1cb1db2;
     D3 V1 = tmp1 * t2ct1;
@@ -337,22 +340,22 @@ __device__ __forceinline__ void general_pair(const KConsts& K, D3 b1, D3 n11, D3
 }
 
 // ParSegSegInteg at one corner, added or subtracted (sm) into integ[12].
-__device__ __forceinline__ void par_seg_seg_integ_acc(double aSq_dSq, double aSq_dSqI, double x, double y,
-                                                      unsigned long long sm, double* integ) {
-  double xpy = x + y;
-  double xmy = x - y;
-  double Ra = sqrt(aSq_dSq + xpy * xpy);
-  double RaInv = 1.0 / Ra;
-  double Log_Ra_ypz = im::log(Ra + xpy);
-  double tmp = xmy * Ra * aSq_dSqI;
-  double i10 = -aSq_dSqI * xpy * RaInv;
+__device__ __forceinline__ void par_seg_seg_integ_acc(rd aSq_dSq, rd aSq_dSqI, rd x, rd y,
+                                                      unsigned long long sm, rd* integ) {
+  rd xpy = x + y;
+  rd xmy = x - y;
+  rd Ra = sqrt(aSq_dSq + xpy * xpy);
+  rd RaInv = 1.0 / Ra;
+  rd Log_Ra_ypz = im::log(Ra + xpy);
+  rd tmp = xmy * Ra * aSq_dSqI;
+  rd i10 = -aSq_dSqI * xpy * RaInv;
   integ[0] += sgn((Ra * aSq_dSqI), sm);
   integ[1] += sgn((-0.5 * (Log_Ra_ypz - tmp)), sm);
   integ[2] += sgn((-0.5 * (Log_Ra_ypz + tmp)), sm);
   integ[3] += sgn((-Log_Ra_ypz), sm);
   integ[4] += sgn((y * Log_Ra_ypz - Ra), sm);
   integ[5] += sgn((x * Log_Ra_ypz - Ra), sm);
-  integ[6] += sgn((aSq_dSqI * (2.0 * aSq_dSqI * Ra - RaInv)), sm);
+  integ[6] += sgn((aSq_dSqI * (twice(aSq_dSqI) * Ra - RaInv)), sm);
   integ[7] += sgn((aSq_dSqI * (tmp - x * RaInv)), sm);
   integ[8] += sgn((-aSq_dSqI * (tmp + y * RaInv)), sm);
   integ[9] += sgn(i10, sm);
@@ -368,25 +371,25 @@ __device__ __forceinline__ void par_seg_seg_integ_acc(double aSq_dSq, double aSq
 // whose projection roles and integration-variable roles are mirrored.
 // Returns 1 when the core corrections were applied, else 0.
 template <int SIDE>
-__device__ __forceinline__ int par_side(const KConsts& K, D3 na1, D3 na2, D3 ta, double taN, D3 ba, D3 nb1, D3 nb2,
-                                        D3 tb, double tbN, D3 bb, D3& Fa1, D3& Fa2) {
-  const double mu4pi = K.mu4pi, mu4pinu = K.mu4pinu, mu8piaSq = K.mu8piaSq, mu4pinuaSq = K.mu4pinuaSq;
+__device__ __forceinline__ int par_side(const KConsts& K, D3 na1, D3 na2, D3 ta, rd taN, D3 ba, D3 nb1, D3 nb2,
+                                        D3 tb, rd tbN, D3 bb, D3& Fa1, D3& Fa2) {
+  const rd mu4pi = K.mu4pi, mu4pinu = K.mu4pinu, mu8piaSq = K.mu8piaSq, mu4pinuaSq = K.mu4pinuaSq;
   // Project segment b onto segment a's line: nbm1/nbm2 are b's nodes moved onto
   // a's line and pulled apart by the critical angle.
-  double tmp = dot(nb2 - nb1, ta);
+  rd tmp = dot(nb2 - nb1, ta);
   D3 nbm2 = nb1 + tmp * ta;
   D3 diff = nb2 - nbm2;
-  double magDiff = norm(diff);
+  rd magDiff = norm(diff);
   D3 tv1 = 0.5 * diff;
   D3 tv2 = kHCotanThetac * magDiff * ta;
   D3 nbm1 = nb1 + tv1 + tv2;
   nbm2 = nbm2 + tv1 - tv2;
 
   D3 R, nd;
-  double x1, x2, y1, y2;
+  rd x1, x2, y1, y2;
   if (SIDE == 1) {
     R = nbm1 - na1;
-    double Rdt = dot(R, ta);
+    rd Rdt = dot(R, ta);
     nd = R - Rdt * ta;
     x1 = dot(nbm1, ta);
     x2 = dot(nbm2, ta);
@@ -394,34 +397,34 @@ __device__ __forceinline__ int par_side(const KConsts& K, D3 na1, D3 na2, D3 ta,
     y2 = -dot(na2, ta);
   } else {
     R = na1 - nbm1;
-    double Rdt = dot(R, ta);
+    rd Rdt = dot(R, ta);
     nd = R - Rdt * ta;
     x1 = dot(na1, ta);
     x2 = dot(na2, ta);
     y1 = -dot(nbm1, ta);
     y2 = -dot(nbm2, ta);
   }
-  double dSq = dot(nd, nd);
-  double aSq_dSq = K.aSq + dSq;
-  double aSq_dSqI = 1.0 / aSq_dSq;
+  rd dSq = dot(nd, nd);
+  rd aSq_dSq = K.aSq + dSq;
+  rd aSq_dSqI = 1.0 / aSq_dSq;
 
-  double tadbb = dot(ta, bb);
-  double tadba = dot(ta, ba);
-  double nddba = dot(nd, ba);
+  rd tadbb = dot(ta, bb);
+  rd tadba = dot(ta, ba);
+  rd nddba = dot(nd, ba);
   D3 bbcta = cross(bb, ta);
   D3 bacta = cross(ba, ta);
   D3 ndcta = cross(nd, ta);
-  double bbctadba = dot(bbcta, ba);
-  double bbctadnd = dot(bbcta, nd);
+  rd bbctadba = dot(bbcta, ba);
+  rd bbctadnd = dot(bbcta, nd);
   D3 bbctacta = tadbb * ta - bb;
 
-  double integ[12];
+  rd integ[12];
 #pragma unroll
   for (int k = 0; k < 12; ++k) integ[k] = 0.0;
 #pragma unroll 1
   for (int q = 0; q < 4; ++q) {
-    double x = (q & 2) ? x2 : x1;
-    double y = (q & 1) ? y2 : y1;
+    rd x = (q & 2) ? x2 : x1;
+    rd y = (q & 1) ? y2 : y1;
     unsigned long long sm = (q == 1 || q == 2) ? 0x8000000000000000ull : 0ull;
     par_seg_seg_integ_acc(aSq_dSq, aSq_dSqI, x, y, sm, integ);
   }
@@ -435,10 +438,10 @@ __device__ __forceinline__ int par_side(const KConsts& K, D3 na1, D3 na2, D3 ta,
   tmp = mu4pinu * bbctadnd * nddba;
   D3 V3 = -mu8piaSq * w1 - mu4pinuaSq * w2 - tmp * ndcta;
   tmp = mu8piaSq * tadba;
-  double tmp2 = mu4pinu * bbctadnd * tadba;
+  rd tmp2 = mu4pinu * bbctadnd * tadba;
   D3 V4 = -tmp * bbctacta - tmp2 * ndcta;
 
-  double Fint1, Fint2, Fint3, Fint4;
+  rd Fint1, Fint2, Fint3, Fint4;
   if (SIDE == 1) {
     Fint1 = integ[2] - y1 * integ[0];
     Fint2 = integ[5] - y1 * integ[3];
@@ -465,12 +468,13 @@ __device__ __forceinline__ int par_side(const KConsts& K, D3 na1, D3 na2, D3 ta,
 
   // Core corrections (DislocationForces.jl:1280-1317, :1396-1433): the two
   // connector segments nb1 -> nbm1 and nbm2 -> nb2 acting on segment a.
-  double magDiffSq = (SIDE == 1) ? dot(diff, diff) : magDiff * magDiff;
-  double m1 = dot(nbm1, nbm1);
-  double m2 = dot(nbm2, nbm2);
+  rd magDiffSq = (SIDE == 1) ? dot(diff, diff) : magDiff * magDiff;
+  rd m1 = dot(nbm1, nbm1);
+  rd m2 = dot(nbm2, nbm2);
   if (magDiffSq > kSqrtEps * (m1 + m2)) {
     D3 F1, F2, F3, F4, tc;
-    double tcN, c;
+    double tcN;
+    rd c;
     seg_direction(nb1, nbm1, tc, tcN);
     c = dot(tc, ta);
     general_pair<false, true>(K, bb, nb1, nbm1, tc, tcN, ba, na1, na2, ta, taN, c, F1, F2, F3, F4);
@@ -492,8 +496,8 @@ __device__ __forceinline__ int par_side(const KConsts& K, D3 na1, D3 na2, D3 ta,
 // the second side (the index-list form discards it).  Returns the number of
 // sides (0-2) that needed the two core-correction evaluations.
 template <bool NEED34>
-__device__ __forceinline__ int parallel_pair(const KConsts& K, D3 b1, D3 n11, D3 n12, D3 t1, double t1N, D3 b2,
-                                              D3 n21, D3 n22, D3 t2, double t2N, double c, D3& F1, D3& F2, D3& F3,
+__device__ __forceinline__ int parallel_pair(const KConsts& K, D3 b1, D3 n11, D3 n12, D3 t1, rd t1N, D3 b2,
+                                              D3 n21, D3 n22, D3 t2, rd t2N, rd c, D3& F1, D3& F2, D3& F3,
                                               D3& F4) {
   bool flip = c < 0.0;
   if (flip) {
@@ -516,65 +520,65 @@ __device__ __forceinline__ int parallel_pair(const KConsts& K, D3 b1, D3 n11, D3
 // σ̃ of one segment at one point, added into sig[6] (xx, yy, zz, xy, xz, yz).
 // txb = t x b depends on the segment only: the caller computes it once per
 // segment with the same operations (the same bits as computing it here).
-__device__ __forceinline__ void sigma_point(const KConsts& K, D3 b, D3 n1, D3 n2, D3 t, D3 txb, D3 x, double* sig) {
-  const double mu4pi = K.mu4pi, mu4pinu = K.mu4pinu, nuMu4pinu = K.nuMu4pinu, a2 = K.aSq;
-  const double a2mu8pi = a2 * K.mu8pi;
+__device__ __forceinline__ void sigma_point(const KConsts& K, D3 b, D3 n1, D3 n2, D3 t, D3 txb, D3 x, rd* sig) {
+  const rd mu4pi = K.mu4pi, mu4pinu = K.mu4pinu, nuMu4pinu = K.nuMu4pinu, a2 = K.aSq;
+  const rd a2mu8pi = a2 * K.mu8pi;
   D3 R = x - n1;
-  double Rdt = dot(R, t);
+  rd Rdt = dot(R, t);
   D3 nd = R - Rdt * t;
-  double d2 = dot(nd, nd);
-  double s1 = -Rdt;
-  double s2 = -dot(x - n2, t);
-  double a2_d2 = a2 + d2;
-  double a2d2inv = 1.0 / a2_d2;
+  rd d2 = dot(nd, nd);
+  rd s1 = -Rdt;
+  rd s2 = -dot(x - n2, t);
+  rd a2_d2 = a2 + d2;
+  rd a2d2inv = 1.0 / a2_d2;
 
-  double Ra = sqrt(a2_d2 + s1 * s1);
-  double Rainv = 1.0 / Ra;
-  double Ra3inv = Rainv * Rainv * Rainv;
-  double sRa3inv = s1 * Ra3inv;
-  double s_03a = s1 * Rainv * a2d2inv;
-  double s_13a = -Rainv;
-  double s_05a = (2.0 * s_03a + sRa3inv) * a2d2inv;
-  double s_15a = -Ra3inv;
-  double s_25a = s_03a - sRa3inv;
+  rd Ra = sqrt(a2_d2 + s1 * s1);
+  rd Rainv = 1.0 / Ra;
+  rd Ra3inv = Rainv * Rainv * Rainv;
+  rd sRa3inv = s1 * Ra3inv;
+  rd s_03a = s1 * Rainv * a2d2inv;
+  rd s_13a = -Rainv;
+  rd s_05a = (twice(s_03a) + sRa3inv) * a2d2inv;
+  rd s_15a = -Ra3inv;
+  rd s_25a = s_03a - sRa3inv;
 
   Ra = sqrt(a2_d2 + s2 * s2);
   Rainv = 1.0 / Ra;
   Ra3inv = Rainv * Rainv * Rainv;
   sRa3inv = s2 * Ra3inv;
-  double s_03b = s2 * Rainv * a2d2inv;
-  double s_13b = -Rainv;
-  double s_05b = (2.0 * s_03b + sRa3inv) * a2d2inv;
-  double s_15b = -Ra3inv;
-  double s_25b = s_03b - sRa3inv;
+  rd s_03b = s2 * Rainv * a2d2inv;
+  rd s_13b = -Rainv;
+  rd s_05b = (twice(s_03b) + sRa3inv) * a2d2inv;
+  rd s_15b = -Ra3inv;
+  rd s_25b = s_03b - sRa3inv;
 
-  double s_03 = s_03b - s_03a;
-  double s_13 = s_13b - s_13a;
-  double s_05 = s_05b - s_05a;
-  double s_15 = s_15b - s_15a;
-  double s_25 = s_25b - s_25a;
+  rd s_03 = s_03b - s_03a;
+  rd s_13 = s_13b - s_13a;
+  rd s_05 = s_05b - s_05a;
+  rd s_15 = s_15b - s_15a;
+  rd s_25 = s_25b - s_25a;
 
   D3 dxb = cross(nd, b);
-  double dxbdt = dot(dxb, t);
-  double common = mu4pinu * dxbdt;
+  rd dxbdt = dot(dxb, t);
+  rd common = mu4pinu * dxbdt;
 
   // Component tables: (xx, yy, zz, xy, xz, yz) index pairs.
-  const double tt[3] = {t.x, t.y, t.z};
-  const double dd[3] = {nd.x, nd.y, nd.z};
-  const double tb_[3] = {txb.x, txb.y, txb.z};
-  const double db_[3] = {dxb.x, dxb.y, dxb.z};
+  const rd tt[3] = {t.x, t.y, t.z};
+  const rd dd[3] = {nd.x, nd.y, nd.z};
+  const rd tb_[3] = {txb.x, txb.y, txb.z};
+  const rd db_[3] = {dxb.x, dxb.y, dxb.z};
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
     const int p = (c < 3) ? c : (c == 3 ? 0 : (c == 4 ? 0 : 1));
     const int q = (c < 3) ? c : (c == 3 ? 1 : 2);
-    double dmd, tmt, tmd, tmtxb, dmtxb, tmdxb;
+    rd dmd, tmt, tmd, tmtxb, dmtxb, tmdxb;
     if (c < 3) {
       dmd = dd[p] * dd[p];
       tmt = tt[p] * tt[p];
-      tmd = 2.0 * tt[p] * dd[p];
-      tmtxb = 2.0 * tt[p] * tb_[p];
-      dmtxb = 2.0 * dd[p] * tb_[p];
-      tmdxb = 2.0 * tt[p] * db_[p];
+      tmd = twice(tt[p]) * dd[p];
+      tmtxb = twice(tt[p]) * tb_[p];
+      dmtxb = twice(dd[p]) * tb_[p];
+      tmdxb = twice(tt[p]) * db_[p];
     } else {
       dmd = dd[p] * dd[q];
       tmt = tt[p] * tt[q];
@@ -583,11 +587,11 @@ __device__ __forceinline__ void sigma_point(const KConsts& K, D3 b, D3 n1, D3 n2
       dmtxb = dd[p] * tb_[q] + dd[q] * tb_[p];
       tmdxb = tt[p] * db_[q] + tt[q] * db_[p];
     }
-    double I03 = (c < 3) ? (common + mu4pinu * dmtxb - mu4pi * tmdxb) : (mu4pinu * dmtxb - mu4pi * tmdxb);
-    double I13 = -nuMu4pinu * tmtxb;
-    double I05 = (c < 3) ? (common * (a2 + dmd) - a2mu8pi * tmdxb) : (common * dmd - a2mu8pi * tmdxb);
-    double I15 = a2mu8pi * tmtxb - common * tmd;
-    double I25 = common * tmt;
+    rd I03 = (c < 3) ? (common + mu4pinu * dmtxb - mu4pi * tmdxb) : (mu4pinu * dmtxb - mu4pi * tmdxb);
+    rd I13 = -nuMu4pinu * tmtxb;
+    rd I05 = (c < 3) ? (common * (a2 + dmd) - a2mu8pi * tmdxb) : (common * dmd - a2mu8pi * tmdxb);
+    rd I15 = a2mu8pi * tmtxb - common * tmd;
+    rd I25 = common * tmt;
     sig[c] += I03 * s_03 + I13 * s_13 + I05 * s_05 + I15 * s_15 + I25 * s_25;
   }
 }

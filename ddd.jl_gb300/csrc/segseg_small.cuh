@@ -87,15 +87,7 @@ x_pairs(TileArgs A, typename P::Consts KP, const uint8_t* __restrict__ flags, co
       const int t = pos & (XT - 1), k = (pos >> 7) & (XT - 1), jl = (t + k) & (XT - 1);
       int64_t I, J;
       x_tile_index(pos >> 14, I, J);
-      const SegF64 a = tb_load_seg64(A.soa, A.npad, I * XT + t), s = tb_load_seg64(A.soa, A.npad, J * XT + jl);
-      D3 F1, F2, F3, F4;
-      nCore += parallel_pair<true>(A.K, a.b, a.n1, a.n2, a.t, a.tN, s.b, s.n1, s.n2, s.t, s.tN, dot(a.t, s.t), F1, F2,
-                                   F3, F4);
-      double* v = vals + (int64_t)(pos >> 7) * 12 * XT + t;
-      v[0 * XT] = F1.x; v[1 * XT] = F1.y; v[2 * XT] = F1.z;
-      v[3 * XT] = F2.x; v[4 * XT] = F2.y; v[5 * XT] = F2.z;
-      v[6 * XT] = F3.x; v[7 * XT] = F3.y; v[8 * XT] = F3.z;
-      v[9 * XT] = F4.x; v[10 * XT] = F4.y; v[11 * XT] = F4.z;
+      nCore += tb_parallel_pair(A, I * XT + t, J * XT + jl, vals + (int64_t)(pos >> 7) * 12 * XT + t, XT);
     }
     if (counters && nCore) atomicAdd(&counters[2], nCore);
     return;

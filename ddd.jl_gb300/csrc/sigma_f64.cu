@@ -35,7 +35,7 @@ sigma_tilde_f64(KConsts K, const double* __restrict__ soa, int64_t npad, int64_t
   const int64_t j = blockIdx.x * (int64_t)SIG_TILE + t;
   D3 x = {0, 0, 0};
   if (j < M) x = {x0[3 * j], x0[3 * j + 1], x0[3 * j + 2]};
-  double sig[6] = {0, 0, 0, 0, 0, 0};
+  rd sig[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   for (int64_t s0 = 0; s0 < nSeg; s0 += SIG_TILE) {
     __syncthreads();
 #pragma unroll

@@ -26,7 +26,7 @@ sigma_tilde_fx(sx::KS K, const double* __restrict__ soa, int64_t npad, int64_t n
   const int64_t j = blockIdx.x * (int64_t)SIG_TILE + t;
   sx::X3 x = {0, 0, 0};
   if (j < M) x = {x0[3 * j], x0[3 * j + 1], x0[3 * j + 2]};
-  double sig[6] = {0, 0, 0, 0, 0, 0};
+  rd sig[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   for (int64_t s0 = 0; s0 < nSeg; s0 += SIG_TILE) {
     __syncthreads();
     {

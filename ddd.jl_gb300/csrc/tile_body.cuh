@@ -54,6 +54,21 @@ __device__ __forceinline__ SegF64 tb_load_seg64(const double* __restrict__ soa, 
   return s;
 }
 
+// The near-parallel pair (row gi, column gj): its forces as 12 doubles at
+// f[c * stride].  Returns the sides that needed core corrections.  A function of
+// its own so that the general branch's registers are not allocated around it.
+static __device__ __forceinline__ int tb_parallel_pair(const TileArgs& A, int64_t gi, int64_t gj, double* f, int stride) {
+  const SegF64 a = tb_load_seg64(A.soa, A.npad, gi), b = tb_load_seg64(A.soa, A.npad, gj);
+  D3 F1, F2, F3, F4;
+  const int cores = parallel_pair<true>(A.K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, dot(a.t, b.t), F1,
+                                        F2, F3, F4);
+  f[0 * stride] = F1.x; f[1 * stride] = F1.y; f[2 * stride] = F1.z;
+  f[3 * stride] = F2.x; f[4 * stride] = F2.y; f[5 * stride] = F2.z;
+  f[6 * stride] = F3.x; f[7 * stride] = F3.y; f[8 * stride] = F3.z;
+  f[9 * stride] = F4.x; f[10 * stride] = F4.y; f[11 * stride] = F4.z;
+  return cores;
+}
+
 // Shared memory of one tile: the policy's column tile and column accumulators,
 // plus the near-parallel compaction state.
 template <int T, class P>
@@ -211,21 +226,18 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
     const int e = base + t;
     if (e < end) {
       const int il = sm.plist[e] >> 8, jl = sm.plist[e] & 0xff;
-      D3 F1, F2, F3 = {0, 0, 0}, F4 = {0, 0, 0};
       if (genRun) {
+        D3 F1, F2, F3, F4;
         P::dense_general(KP, A, iBase + il, j0 + jl, F1, F2, F3, F4);
         ++nGeneral;
+        sm.cf[t][0] = F1.x; sm.cf[t][1] = F1.y; sm.cf[t][2] = F1.z;
+        sm.cf[t][3] = F2.x; sm.cf[t][4] = F2.y; sm.cf[t][5] = F2.z;
+        sm.cf[t][6] = F3.x; sm.cf[t][7] = F3.y; sm.cf[t][8] = F3.z;
+        sm.cf[t][9] = F4.x; sm.cf[t][10] = F4.y; sm.cf[t][11] = F4.z;
       } else {
-        SegF64 a = tb_load_seg64(A.soa, A.npad, iBase + il);
-        SegF64 b = tb_load_seg64(A.soa, A.npad, j0 + jl);
-        double c = dot(a.t, b.t);
         ++nDenseParallel;
-        nCore += parallel_pair<true>(A.K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, c, F1, F2, F3, F4);
+        nCore += tb_parallel_pair(A, iBase + il, j0 + jl, sm.cf[t], 1);
       }
-      sm.cf[t][0] = F1.x; sm.cf[t][1] = F1.y; sm.cf[t][2] = F1.z;
-      sm.cf[t][3] = F2.x; sm.cf[t][4] = F2.y; sm.cf[t][5] = F2.z;
-      sm.cf[t][6] = F3.x; sm.cf[t][7] = F3.y; sm.cf[t][8] = F3.z;
-      sm.cf[t][9] = F4.x; sm.cf[t][10] = F4.y; sm.cf[t][11] = F4.z;
     }
     __syncthreads();
     const int lim = min(CH, end - base);
@@ -371,12 +383,12 @@ struct PolF64 {
   template <int T>
   static __device__ __forceinline__ void add_col(Tile<T>& s, int warp, int j, const D3& F3, const D3& F4) {
     double* fj = &s.fj[warp][0][0];
-    fj[0 * T + j] += F3.x;
-    fj[1 * T + j] += F3.y;
-    fj[2 * T + j] += F3.z;
-    fj[3 * T + j] += F4.x;
-    fj[4 * T + j] += F4.y;
-    fj[5 * T + j] += F4.z;
+    fj[0 * T + j] = rd(fj[0 * T + j]) + F3.x;
+    fj[1 * T + j] = rd(fj[1 * T + j]) + F3.y;
+    fj[2 * T + j] = rd(fj[2 * T + j]) + F3.z;
+    fj[3 * T + j] = rd(fj[3 * T + j]) + F4.x;
+    fj[4 * T + j] = rd(fj[4 * T + j]) + F4.y;
+    fj[5 * T + j] = rd(fj[5 * T + j]) + F4.z;
   }
   // One component as segseg_small.cuh stores and adds it.
   using Comp = double;
