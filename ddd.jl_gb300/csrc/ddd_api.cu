@@ -166,16 +166,37 @@ cudaError_t run_segseg_rows(ddd_ctx* c, const ddd::KConsts& K, const double* soa
   return cudaSuccess;
 }
 
+// Scratch of a σ̃ call in ctx->expand, which no other call in flight uses: null
+// when none is wanted, or when there is no memory for it (the caller then takes
+// the form without).
+cudaError_t sigma_scratch(ddd_ctx* c, size_t bytes, double** out) {
+  *out = nullptr;
+  if (!bytes) return cudaSuccess;
+  const cudaError_t e = c->expand.ensure(bytes);
+  if (e == cudaSuccess) *out = c->expand.as<double>();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  return cudaSuccess;
+}
+
 cudaError_t run_sigma(ddd_ctx* c, const ddd::KConsts& K, const double* soa, int64_t npad, int64_t nSeg,
                       const double* x0, int64_t M, double* sigma, cudaStream_t st) {
-  if (use_df(c)) {  // both precision modes: the mixed σ̃ form
-    cudaError_t e = prep_df_if_needed(c, npad, st);
+  double* scratch = nullptr;
+  if (use_df(c) || use_fx(c)) {
+    // Resident CTAs: 152 SMs x 8 CTAs of 128 (mixed) or 24 warps (fast).
+    ddd::SigmaPlan plan = use_df(c) ? ddd::sigma_plan(nSeg, M, 128, 1216) : ddd::sigma_plan(nSeg, M, 32, 3648);
+    const size_t bytes = ddd::sigma_part_bytes(plan, M);
+    cudaError_t e = sigma_scratch(c, bytes, &scratch);
     if (e != cudaSuccess) return e;
-    return ddd::launch_sigma_mixed(K, c->soadf.as<float>(), npad, nSeg, x0, M, sigma, st);
+    if (!scratch) plan = ddd::SigmaPlan{1, 1, npad};
+    if (use_fx(c)) return ddd::launch_sigma_fx(K, soa, npad, nSeg, x0, M, sigma, plan, scratch, st);
+    if ((e = prep_df_if_needed(c, npad, st)) != cudaSuccess) return e;  // both precision modes: the mixed σ̃ form
+    return ddd::launch_sigma_mixed(K, c->soadf.as<float>(), npad, nSeg, x0, M, sigma, plan, scratch, st);
   }
-  if (use_fx(c)) return ddd::launch_sigma_fx(K, soa, npad, nSeg, x0, M, sigma, st);
-  return use_fma(c) ? ddd::fast::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, st)
-                    : ddd::strict::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, st);
+  const cudaError_t e = sigma_scratch(c, M < ddd::kSigmaSplitPoints ? ddd::sigma_split_bytes(npad) : 0, &scratch);
+  if (e != cudaSuccess) return e;
+  return use_fma(c) ? ddd::fast::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, scratch, st)
+                    : ddd::strict::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, scratch, st);
 }
 
 

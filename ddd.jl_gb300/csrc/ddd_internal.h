@@ -64,6 +64,42 @@ inline size_t row_partial_bytes(const RowPlan& p, int64_t nRows) { return (size_
 constexpr int64_t kExpandMaxPairs = 153;
 inline size_t expand_bytes(int64_t nb) { return (size_t)nb * 128 * 128 * (12 * sizeof(double) + 4 + 1) + 256; }
 
+// σ̃ with few points.  The literal FP64 kernels (strict, FMA) take sigma_split
+// (sigma_f64.cu) below kSigmaSplitPoints, where a thread per point leaves fewer
+// than ~5 warps per SM; its scratch is two stores of kSigmaChunk evaluations and
+// t x b.
+constexpr int64_t kSigmaSplitPoints = 24576;
+constexpr int64_t kSigmaChunk = 1 << 19;
+inline size_t sigma_split_bytes(int64_t npad) { return (size_t)(12 * kSigmaChunk + 3 * npad) * sizeof(double); }
+
+// The fast and the mixed form cut the segments into slices of whole tiles
+// (blockIdx.y) until the call has ~4 times the CTAs that are resident, and a warp
+// (CTA) with fewer points than lanes lets `lanes` of them share a point.
+// 5,000 points x 8,192 segments: fast 34.8 -> 9.0 ms, mixed 8.2 -> 1.2 ms; the
+// mixed form at 32,768 points (256 CTAs of 128 on 152 SMs before) 22.3 -> 15.6 ms
+// with 16,384 segments.
+struct SigmaPlan {
+  int slices = 1, lanes = 1;
+  int64_t segs = 0;  // segments per slice
+};
+inline SigmaPlan sigma_plan(int64_t nSeg, int64_t M, int tile, int64_t ctas) {
+  SigmaPlan p;
+  while (p.lanes < 32 && M * 2 * p.lanes <= tile) p.lanes *= 2;
+  const int pts = tile / p.lanes;
+  const int64_t blocks = (M + pts - 1) / pts, tiles = (nSeg + tile - 1) / tile;
+  int64_t want = (4 * ctas + blocks - 1) / blocks;
+  if (blocks >= 4 * ctas) want = 1;
+  if (want > tiles) want = tiles;
+  if (want < 1) want = 1;
+  const int64_t per = (tiles + want - 1) / want;
+  p.segs = per * tile;
+  p.slices = (int)((tiles + per - 1) / per);
+  return p;
+}
+inline size_t sigma_part_bytes(const SigmaPlan& p, int64_t M) {
+  return p.slices * p.lanes > 1 ? (size_t)p.slices * p.lanes * 6 * M * sizeof(double) : 0;
+}
+
 // All-pairs partial sums: one slot (12 x TILE doubles) per tile pair I <= J,
 // slot J(J+1)/2 + I.  The all-pairs launchers take the partial buffer's size
 // in slots; when it is below nt(nt+1)/2 they run bands of J columns (each band
@@ -92,7 +128,7 @@ inline size_t expand_bytes(int64_t nb) { return (size_t)nb * 128 * 128 * (12 * s
                                      const int64_t* rows, int64_t nRows, const RowPlan& plan, double* partial, \
                                      double* out, unsigned long long* counters, cudaStream_t st); \
   cudaError_t launch_sigma_f64(const KConsts& K, const double* soa, int64_t npad, int64_t nSeg, const double* x0, \
-                               int64_t M, double* sigma, cudaStream_t st); \
+                               int64_t M, double* sigma, double* scratch, cudaStream_t st); \
   cudaError_t launch_reduce_all(const double* partial, int64_t npad, int64_t numSeg, double* out, cudaStream_t st); \
   cudaError_t launch_reduce_band(const double* partial, int64_t J0, int64_t J1, int64_t numSeg, double* out, \
                                  cudaStream_t st); \
@@ -122,14 +158,16 @@ cudaError_t launch_segseg_rows_df(const KConsts& K, const double* soa, const flo
                                   int form);
 // σ̃ in the mixed form: geometry and endpoint differences in df64, assembly in FP32.
 cudaError_t launch_sigma_mixed(const KConsts& K, const float* soadf, int64_t npad, int64_t nSeg, const double* x0,
-                               int64_t M, double* sigma, cudaStream_t st);
+                               int64_t M, double* sigma, const SigmaPlan& plan, double* part, cudaStream_t st);
 
 // segseg_f64fast.cu: the FP64 tile kernels with the fast general branch
 // (pair_f64fast.cuh: fewer divisions, table-driven log/atan, explicit FMAs);
 // near-parallel branch, segment preparation and reductions strict.
 // The fast FP64 form of σ̃ (sigma_fx.cu).
 cudaError_t launch_sigma_fx(const KConsts& K, const double* soa, int64_t npad, int64_t nSeg, const double* x0,
-                            int64_t M, double* sigma, cudaStream_t st);
+                            int64_t M, double* sigma, const SigmaPlan& plan, double* part, cudaStream_t st);
+// Sum of `slices` partial results of 6 M doubles, in order (sigma_fx.cu).
+cudaError_t launch_sigma_slices(const double* part, int64_t M, int slices, double* sigma, cudaStream_t st);
 cudaError_t launch_segseg_all_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                                  double* partial, double* out, int64_t numSeg, unsigned long long* counters,
                                  cudaStream_t st, int64_t capSlots);

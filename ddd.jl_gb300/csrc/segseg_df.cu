@@ -68,19 +68,22 @@ cudaError_t set_attr_df() {
 // σ̃ in the mixed form (sigma_point_mixed, pair_df.cuh): one thread per point,
 // segments streamed through shared memory as df64 pairs (n1, n2, t) and FP32
 // (b), six df64 accumulators per point in the segment order of the FP64 kernel.
+// Slices as in sigma_fx.cu.
 constexpr int SIG_TILE = 128;
 __global__ void __launch_bounds__(SIG_TILE)
-sigma_tilde_mixed(KConstsSig K, const float* __restrict__ soadf, int64_t npad, int64_t nSeg,
-                  const double* __restrict__ x0, int64_t M, double* __restrict__ sigma) {
+sigma_tilde_mixed(KConstsSig K, const float* __restrict__ soadf, int64_t npad, int64_t nSegAll,
+                  const double* __restrict__ x0, int64_t M, SigmaPlan plan, double* __restrict__ sigma) {
   __shared__ float seg[21][SIG_TILE];  // n1 hi/lo (6), n2 hi/lo (6), b hi (3), t hi/lo (6)
   const int t = threadIdx.x;
-  const int64_t j = blockIdx.x * (int64_t)SIG_TILE + t;
+  const int pts = SIG_TILE / plan.lanes, sub = t / pts;
+  const int64_t j = blockIdx.x * (int64_t)pts + t % pts;
+  const int64_t sBeg = blockIdx.y * plan.segs, nSeg = min(nSegAll, sBeg + plan.segs);
   DV3 x = {df(0.f), df(0.f), df(0.f)};
   if (j < M) x = {df_from_double(x0[3 * j]), df_from_double(x0[3 * j + 1]), df_from_double(x0[3 * j + 2])};
   df64 sig[6];
 #pragma unroll
   for (int c = 0; c < 6; ++c) sig[c] = df(0.f);
-  for (int64_t s0 = 0; s0 < nSeg; s0 += SIG_TILE) {
+  for (int64_t s0 = sBeg; s0 < nSeg; s0 += SIG_TILE) {
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 12; ++k) seg[k][t] = soadf[k * npad + s0 + t];  // rows 0-11: n1, n2 (hi, lo)
@@ -91,7 +94,7 @@ sigma_tilde_mixed(KConstsSig K, const float* __restrict__ soadf, int64_t npad, i
     __syncthreads();
     const int n = (int)min((int64_t)SIG_TILE, nSeg - s0);
     if (j < M) {
-      for (int q = 0; q < n; ++q) {
+      for (int q = sub; q < n; q += plan.lanes) {
         const DV3 n1 = {df64{seg[0][q], seg[1][q]}, df64{seg[2][q], seg[3][q]}, df64{seg[4][q], seg[5][q]}};
         const DV3 n2 = {df64{seg[6][q], seg[7][q]}, df64{seg[8][q], seg[9][q]}, df64{seg[10][q], seg[11][q]}};
         const F3 b = {seg[12][q], seg[13][q], seg[14][q]};
@@ -101,8 +104,9 @@ sigma_tilde_mixed(KConstsSig K, const float* __restrict__ soadf, int64_t npad, i
     }
   }
   if (j < M) {
+    double* o = sigma + 6 * (M * (blockIdx.y * (int64_t)plan.lanes + sub) + j);
 #pragma unroll
-    for (int c = 0; c < 6; ++c) sigma[6 * j + c] = df_to_double(sig[c]);
+    for (int c = 0; c < 6; ++c) o[c] = df_to_double(sig[c]);
   }
 }
 
@@ -111,7 +115,7 @@ sigma_tilde_mixed(KConstsSig K, const float* __restrict__ soadf, int64_t npad, i
 size_t segseg_df_soa_bytes(int64_t npad) { return (size_t)npad * 26 * sizeof(float); }
 
 cudaError_t launch_sigma_mixed(const KConsts& K, const float* soadf, int64_t npad, int64_t nSeg, const double* x0,
-                               int64_t M, double* sigma, cudaStream_t st) {
+                               int64_t M, double* sigma, const SigmaPlan& plan, double* part, cudaStream_t st) {
   if (M == 0) return cudaSuccess;
   KConstsSig KS;
   KS.aSq = kconsts_df(K).aSq;
@@ -120,9 +124,11 @@ cudaError_t launch_sigma_mixed(const KConsts& K, const float* soadf, int64_t npa
   KS.nuMu4pinu = (float)K.nuMu4pinu;
   KS.aSq32 = (float)K.aSq;
   KS.aSqMu8pi = (float)(K.aSq * K.mu8pi);
-  sigma_tilde_mixed<<<(unsigned)((M + SIG_TILE - 1) / SIG_TILE), SIG_TILE, 0, st>>>(KS, soadf, npad, nSeg, x0, M,
-                                                                                     sigma);
-  return cudaGetLastError();
+  const int pts = SIG_TILE / plan.lanes;
+  const dim3 grid((unsigned)((M + pts - 1) / pts), (unsigned)plan.slices);
+  sigma_tilde_mixed<<<grid, SIG_TILE, 0, st>>>(KS, soadf, npad, nSeg, x0, M, plan, part ? part : sigma);
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess || !part ? e : launch_sigma_slices(part, M, plan.slices * plan.lanes, sigma, st);
 }
 
 cudaError_t launch_prep_df(const double* soa, int64_t npad, float* soadf, cudaStream_t st) {

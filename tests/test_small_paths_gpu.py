@@ -54,3 +54,28 @@ def test_index_rows(pkg, synth, oracle, n, rows):
         idx[:3] = [5, n, n]
     Fi = pkg.calcSegSegForce(dln, mat, net, idx)
     check_forces(Fi, oracle, k5, net, rows=idx - 1, ref=oracle.segseg_idx(k5, net, idx))
+
+
+@pytest.mark.parametrize("mode,rel", [("fp64", 0.0), ("fp64_fast", 1e-12), ("f32c", 1e-11)])
+@pytest.mark.parametrize("nseg", [1, 31, 1000])
+def test_sigma_few_points(pkg, synth, mode, rel, nseg):
+    """σ̃ with too few points for a thread each (1 point shared by a whole warp or
+    CTA, 33, 100, and 24,575, the most that the FP64 store takes) against the same
+    points inside a call that has enough.  FP64 keeps the segment order, so the
+    bits; the other forms regroup a sum of 1,000 terms (1,000 x 2^-53 and
+    1,000 x 2^-47, of sums that cancel by less than a factor of ten)."""
+    net = _synthetic(pkg, synth, 125, 3, cube=2000.0)
+    net.numSeg = nseg
+    dln, mat = _params(pkg)
+    k = pkg.consts_of(dln, mat)
+    M = 122880 if mode != "fp64" else 24576
+    x0 = np.asfortranarray(np.random.default_rng(nseg).uniform(0.0, 2000.0, (3, M)))
+    ctx = pkg.get_context()
+    ctx.mode = mode
+    try:
+        whole = ctx.sigma_tilde(k, x0, net)
+        for m in (1, 33, 100, 24575):
+            part = ctx.sigma_tilde(k, np.asfortranarray(x0[:, :m]), net)
+            assert np.all(np.abs(part - whole[:, :m]) <= rel * np.abs(whole).max())
+    finally:
+        ctx.mode = "fp64"
