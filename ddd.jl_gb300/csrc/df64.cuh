@@ -219,4 +219,190 @@ DF_HD df64 df_atan(df64 x) {
   return neg ? -r : r;
 }
 
+// ---------------------------------------------------------------------------
+// Two df64 values at once, on GB300's packed FP32 instructions (add / mul / fma
+// .f32x2: two lanes of a 64-bit register pair, each lane rounded as the scalar
+// instruction does, so a lane holds the scalar form's bits).
+//
+// Why: a packed instruction takes the FMA pipe as long as two scalar ones but one
+// issue slot and one 4-cycle latency (measured).  The pair kernels hold 8 warps
+// per SM (255 registers), and their df64 code is chains of dependent additions:
+// the FMA pipe was 46 % busy.
+#if defined(__CUDACC__)
+struct f2 {
+  unsigned long long v;
+};
+DF_HD f2 f2_make(float x, float y) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+  return r;
+}
+DF_HD float f2_x(f2 a) { return __int_as_float((int)(unsigned)a.v); }
+DF_HD float f2_y(f2 a) { return __int_as_float((int)(a.v >> 32)); }
+DF_HD f2 operator+(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+DF_HD f2 operator-(f2 a, f2 b) {
+  f2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+DF_HD f2 operator*(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+DF_HD f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+DF_HD f2 operator-(f2 a) { return {a.v ^ 0x8000000080000000ull}; }
+#else
+struct f2 {
+  float x, y;
+};
+DF_HD f2 f2_make(float x, float y) { return {x, y}; }
+DF_HD float f2_x(f2 a) { return a.x; }
+DF_HD float f2_y(f2 a) { return a.y; }
+DF_HD f2 operator+(f2 a, f2 b) { return {a.x + b.x, a.y + b.y}; }
+DF_HD f2 operator-(f2 a, f2 b) { return {a.x - b.x, a.y - b.y}; }
+DF_HD f2 operator*(f2 a, f2 b) { return {a.x * b.x, a.y * b.y}; }
+DF_HD f2 f2_fma(f2 a, f2 b, f2 c) { return {df_fma(a.x, b.x, c.x), df_fma(a.y, b.y, c.y)}; }
+DF_HD f2 operator-(f2 a) { return {-a.x, -a.y}; }
+#endif
+DF_HD f2 f2_dup(float a) { return f2_make(a, a); }
+
+struct df2 {
+  f2 hi, lo;
+};
+DF_HD df2 df2_make(df64 x, df64 y) { return {f2_make(x.hi, y.hi), f2_make(x.lo, y.lo)}; }
+DF_HD df2 df2_dup(df64 a) { return {f2_dup(a.hi), f2_dup(a.lo)}; }
+DF_HD df64 df2_x(df2 a) { return {f2_x(a.hi), f2_x(a.lo)}; }
+DF_HD df64 df2_y(df2 a) { return {f2_y(a.hi), f2_y(a.lo)}; }
+DF_HD f2 f2_swap(f2 a) { return f2_make(f2_y(a), f2_x(a)); }
+DF_HD df2 df2_swap(df2 a) { return {f2_swap(a.hi), f2_swap(a.lo)}; }
+
+DF_HD df2 two_sum(f2 a, f2 b) {
+  f2 s = a + b;
+  f2 bb = s - a;
+  return {s, (a - (s - bb)) + (b - bb)};
+}
+DF_HD df2 two_diff(f2 a, f2 b) {  // two_sum(a, -b)
+  f2 s = a - b;
+  f2 bb = s - a;
+  return {s, (a - (s - bb)) - (b + bb)};
+}
+DF_HD df2 fast_two_sum(f2 a, f2 b) {
+  f2 s = a + b;
+  return {s, b - (s - a)};
+}
+DF_HD df2 operator-(df2 a) { return {-a.hi, -a.lo}; }
+DF_HD df2 operator+(df2 a, df2 b) {
+  df2 s = two_sum(a.hi, b.hi);
+  return fast_two_sum(s.hi, s.lo + (a.lo + b.lo));
+}
+DF_HD df2 operator-(df2 a, df2 b) {
+  df2 s = two_diff(a.hi, b.hi);
+  return fast_two_sum(s.hi, s.lo + (a.lo - b.lo));
+}
+DF_HD df2 operator+(df2 a, f2 b) {
+  df2 s = two_sum(a.hi, b);
+  return fast_two_sum(s.hi, s.lo + a.lo);
+}
+DF_HD df2 operator-(df2 a, f2 b) {
+  df2 s = two_diff(a.hi, b);
+  return fast_two_sum(s.hi, s.lo + a.lo);
+}
+DF_HD df2 operator*(df2 a, df2 b) {
+  f2 p = a.hi * b.hi;
+  f2 e = f2_fma(a.hi, b.hi, -p);
+  e = f2_fma(a.hi, b.lo, e);
+  e = f2_fma(a.lo, b.hi, e);
+  return fast_two_sum(p, e);
+}
+DF_HD df2 operator*(df2 a, f2 b) {
+  f2 p = a.hi * b;
+  f2 e = f2_fma(a.hi, b, -p);
+  e = f2_fma(a.lo, b, e);
+  return fast_two_sum(p, e);
+}
+DF_HD df2 df_scale(df2 a, float p2) {
+  const f2 s = f2_dup(p2);
+  return {a.hi * s, a.lo * s};
+}
+DF_HD f2 df_qapprox(f2 a, f2 b) { return f2_make(df_qapprox(f2_x(a), f2_x(b)), df_qapprox(f2_y(a), f2_y(b))); }
+DF_HD df2 operator/(df2 a, df2 b) {
+  f2 q1 = df_qapprox(a.hi, b.hi);
+  df2 r = a - b * q1;
+  f2 q2 = df_qapprox(r.hi, b.hi);
+  r = r - b * q2;
+  f2 q3 = df_qapprox(r.hi, b.hi);
+  return fast_two_sum(q1, q2) + q3;
+}
+DF_HD df2 df_recip(df2 b) { return df2{f2_dup(1.0f), f2_dup(0.0f)} / b; }
+
+DF_HD df2 df_sqrt(df2 a) {
+  const float ax = f2_x(a.hi), ay = f2_y(a.hi);
+  if (!(ax > 0.0f && ay > 0.0f)) return df2_make(df_sqrt(df2_x(a)), df_sqrt(df2_y(a)));
+  const f2 s = f2_make(df_sqrtf(ax), df_sqrtf(ay));
+  const f2 p = s * s;
+  const df2 r = a - df2{p, f2_fma(s, s, -p)};
+  return fast_two_sum(s, df_qapprox(r.hi, f2_dup(2.0f) * s));
+}
+
+DF_HD df2 df_log(df2 a) {
+  const int32_t bx = df_bits(f2_x(a.hi)), by = df_bits(f2_y(a.hi));
+  const int32_t ex = ((bx >> 23) & 0xff) - 127, ey = ((by >> 23) & 0xff) - 127;
+  const int32_t jx = (bx >> 17) & 63, jy = (by >> 17) & 63;
+  const f2 scale = f2_make(df_from_bits((127 - ex) << 23), df_from_bits((127 - ey) << 23));
+  const df2 m = {a.hi * scale, a.lo * scale};
+  const f2 c = f2_dup(1.0f) + (f2_make((float)jx, (float)jy) + f2_dup(0.5f)) * f2_dup(0.015625f);
+  const df2 u = (m - c) / (m + c);
+  const df2 u2 = u * u;
+  const f2 t = u2.hi;
+  // Lane by lane: a packed product used once would be fused into its sum.
+  auto poly = [](float w) { return w * (0.2f + w * 0.14285714285714285f); };
+  const f2 tail = f2_make(poly(f2_x(t)), poly(f2_y(t)));
+  const df2 P = df2{f2_dup(kDfThird_HI), f2_dup(kDfThird_LO)} + tail;
+  const df2 r = df_scale(u + u * u2 * P, 2.0f);
+  const float2_ lx = kDfLogC[jx], ly = kDfLogC[jy];
+  const df2 le = df2{f2_dup(kDfLn2_HI), f2_dup(kDfLn2_LO)} * f2_make((float)ex, (float)ey);
+  return le + (df2{f2_make(lx.x, ly.x), f2_make(lx.y, ly.y)} + r);
+}
+
+DF_HD df2 df_atan(df2 x) {
+  const bool nx = f2_x(x.hi) < 0.0f, ny = f2_y(x.hi) < 0.0f;
+  const f2 sg = f2_make(nx ? -1.0f : 1.0f, ny ? -1.0f : 1.0f);
+  df2 z = {x.hi * sg, x.lo * sg};
+  const bool ix = f2_x(z.hi) > 1.0f, iy = f2_y(z.hi) > 1.0f;
+  if (ix || iy) {
+    const df2 w = df_recip(z);
+    z = {f2_make(ix ? f2_x(w.hi) : f2_x(z.hi), iy ? f2_y(w.hi) : f2_y(z.hi)),
+         f2_make(ix ? f2_x(w.lo) : f2_x(z.lo), iy ? f2_y(w.lo) : f2_y(z.lo))};
+  }
+  int jx = (int)(f2_x(z.hi) * 32.0f + 0.5f), jy = (int)(f2_y(z.hi) * 32.0f + 0.5f);
+  jx = jx < 0 ? 0 : (jx > 32 ? 32 : jx);
+  jy = jy < 0 ? 0 : (jy > 32 ? 32 : jy);
+  const f2 c = f2_make((float)jx, (float)jy) * f2_dup(0.03125f);
+  const df2 one = {f2_dup(1.0f), f2_dup(0.0f)};
+  const df2 u = (z - c) / (one + z * c);
+  const df2 u2 = u * u;
+  const f2 t = u2.hi;
+  auto poly = [](float w) {
+    return w * (0.2f + w * (-0.14285714285714285f + w * (0.1111111111111111f - w * 0.09090909090909091f)));
+  };
+  const f2 tail = f2_make(poly(f2_x(t)), poly(f2_y(t)));
+  const df2 Q = df2{f2_dup(-kDfThird_HI), f2_dup(-kDfThird_LO)} + tail;
+  const df2 au = u + u * u2 * Q;
+  const float2_ cx = kDfAtanC[jx], cy = kDfAtanC[jy];
+  df2 r = df2{f2_make(cx.x, cy.x), f2_make(cx.y, cy.y)} + au;
+  const df2 w = df2{f2_dup(kDfPiHalf_HI), f2_dup(kDfPiHalf_LO)} - r;
+  r = {f2_make(ix ? f2_x(w.hi) : f2_x(r.hi), iy ? f2_y(w.hi) : f2_y(r.hi)),
+       f2_make(ix ? f2_x(w.lo) : f2_x(r.lo), iy ? f2_y(w.lo) : f2_y(r.lo))};
+  return {r.hi * sg, r.lo * sg};
+}
+
 }  // namespace ddd

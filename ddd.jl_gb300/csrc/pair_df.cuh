@@ -22,76 +22,145 @@ struct KConstsDF {
   df64 aSq, mu4pi, mu4pinu, mu8piaSq, mu4pinuaSq;
 };
 
-// SegSegInteg at one corner in df64, added or subtracted (neg) into integ[19].
-// aSq_dSq = aSq + d^2 (1 - c^2), its inverse, and den = 1 / sqrt((1 - c^2) aSq_dSq)
-// are computed once per pair by the caller.
-DF_HD void seg_seg_integ_df(df64 aSq_dSq, df64 aSq_dSqI, df64 den, df64 c, df64 cSq, df64 omcSqI, df64 x, df64 y,
-                            bool neg, df64* integ) {
-  df64 xSq = x * x;
-  df64 ySq = y * y;
-  df64 Ra = df_sqrt(aSq_dSq + xSq + ySq + df_scale(x, 2.0f) * y * c);
-  df64 RaInv = df_recip(Ra);
+// The integration domain of a general pair and its 19 integrals,
+// ((I(x1,y1) - I(x1,y2)) - I(x2,y1)) + I(x2,y2) (SegSegInteg,
+// DislocationForces.jl:1480-1561), in two loops of packed df64:
+//   * Ra, 1/Ra and the arctangent integral, two corners per iteration (lanes
+//     (x, y1) and (x, y2));
+//   * the rest, one corner per iteration, with the mirrored quantities of the
+//     formulas in the lanes: R_t1 | R_t2, x | y, integ2 | integ3, integ6 | integ5,
+//     integ 7 | 8, 10 | 11, 12 | 13, 15 | 16 and 17 | 18 (0-based, as stored).
+// Each lane does the scalar formula's operations, so the bits are the scalar's.
+//
+// Why two loops: a warp runs ~8,000 instructions per pair.  An SM's sub-core
+// holds 2,048 of them (32 KB); past that all four share 1.5 fetched instructions
+// per cycle (both measured), and one straight body for two whole corners ran at
+// exactly that (ncu: 33 % of the warp cycles without an instruction).  These
+// bodies are ~400 and ~1,000 instructions, fetched once per pair and run two and
+// four times.
+struct PairDF {
+  df64 c, d, x1, x2, y1, y2, integ[19];
+};
+DF_HD void pair_integrals_df(df64 aSq, DV3 t1, DV3 n11, DV3 n12, DV3 t2, DV3 n21, DV3 n22, df64 c, PairDF& out) {
+  const df64 cSq = c * c;
+  const df64 omcSq = df(1.0f) - cSq;
+  const df64 omcSqI = df_recip(omcSq);
+  // Lanes: R1 = n21 - n11 and R2 = n22 - n12.
+  auto two = [](df64 a, df64 b) { return df2_make(a, b); };
+  const df2 Rx = two(n21.x, n22.x) - two(n11.x, n12.x), Ry = two(n21.y, n22.y) - two(n11.y, n12.y),
+            Rz = two(n21.z, n22.z) - two(n11.z, n12.z);
+  const df2 lim1 = Rx * df2_dup(t1.x) + Ry * df2_dup(t1.y) + Rz * df2_dup(t1.z);
+  const df2 lim2 = Rx * df2_dup(t2.x) + Ry * df2_dup(t2.y) + Rz * df2_dup(t2.z);
+  const df2 C = df2_dup(c), CSq = df2_dup(cSq), Q = df2_dup(omcSqI);
+  const df2 xs = (lim2 - C * lim1) * Q, ys = (lim1 - C * lim2) * Q;
+  const DV3 t2ct1 = cross(t2, t1);
+  struct {
+    df64 d, x1, x2, y1, y2;
+  } g;
+  g.d = (df2_y(Rx) * t2ct1.x + df2_y(Ry) * t2ct1.y + df2_y(Rz) * t2ct1.z) * omcSqI;
+  g.x1 = df2_x(xs);
+  g.x2 = df2_y(xs);
+  g.y1 = df2_x(ys);
+  g.y2 = df2_y(ys);
+  const df64 aSq_dSq = aSq + g.d * g.d * omcSq;
+  const df64 aSq_dSqI = df_recip(aSq_dSq);
+  const df64 den = df_recip(df_sqrt(omcSq * aSq_dSq));
 
-  df64 Ra_Rd_t1 = Ra + y + x * c;
-  df64 Ra_Rd_t2 = Ra + x + y * c;
+  df2 Ras[2], RaIs[2], ats[2];
+  {
+    const df2 A = df2_dup(aSq_dSq), D = df2_dup(den), M = df2_dup(df_scale(-den, 2.0f)), C1 = df2_dup(df(1.0f) + c);
+#ifdef __CUDACC__
+#pragma unroll 1
+#endif
+    for (int q = 0; q < 2; ++q) {
+      const df2 x = df2_dup(q ? g.x2 : g.x1);
+      const df2 R = df_sqrt(A + x * x + ys * ys + df_scale(x, 2.0f) * ys * C);
+      const df2 RI = df_recip(R), at = M * df_atan(C1 * (R + x + ys) * D);
+      if (q == 0) {
+        Ras[0] = R;
+        RaIs[0] = RI;
+        ats[0] = at;
+      } else {
+        Ras[1] = R;
+        RaIs[1] = RI;
+        ats[1] = at;
+      }
+    }
+  }
 
-  df64 log_Ra_Rd_t1 = df_log(Ra_Rd_t1);
-  df64 xlog_Ra_Rd_t1 = x * log_Ra_Rd_t1;
-  df64 log_Ra_Rd_t2 = df_log(Ra_Rd_t2);
-  df64 ylog_Ra_Rd_t2 = y * log_Ra_Rd_t2;
+  df64 s0 = df(0.0f), s3 = s0, s6 = s0, s9 = s0, s14 = s0;
+  const df2 zero = {f2_dup(0.0f), f2_dup(0.0f)};
+  df2 s12 = zero, s54 = zero, s78 = zero, sab = zero, scd = zero, sfg = zero, shi = zero;
+#ifdef __CUDACC__
+#pragma unroll 1
+#endif
+  for (int q = 0; q < 4; ++q) {
+    auto pick = [&](const df2* v) {
+      const df2 w = q & 2 ? v[1] : v[0];
+      return q & 1 ? df2_y(w) : df2_x(w);
+    };
+    const df64 Ra = pick(Ras), RaInv = pick(RaIs), integ1 = pick(ats);
+    const df2 X = df2_make(q & 2 ? g.x2 : g.x1, q & 1 ? g.y2 : g.y1), Y = df2_swap(X);
+    const df2 RI = df2_dup(RaInv);
+    const df2 Rt = df2_dup(Ra) + Y + X * C;  // Ra_Rd_t1 | t2
+    const df2 L = df_log(Rt);
+    const df2 XL = X * L;
+    const df2 S = RI / Rt;  // RaSq_R_t1_I | t2
+    const df2 XS = X * S, XXS = X * XS;
 
-  df64 RaSq_R_t1_I = RaInv / Ra_Rd_t1;
-  df64 xRaSq_R_t1_I = x * RaSq_R_t1_I;
-  df64 xSqRaSq_R_t1_I = x * xRaSq_R_t1_I;
+    const df64 c_1 = aSq_dSq * integ1;
+    const df2 c56i4 = (C * df2_make(Ra, c_1) - df2_make(c_1, Ra)) * Q;  // c_5_6 | integ4
+    const df64 integ4 = df2_y(c56i4);
+    const df2 i23 = (C * df2_swap(L) - L) * Q;         // integ2 | integ3
+    const df2 i65 = XL + df2_dup(df2_x(c56i4));        // integ6 | integ5
+    const df2 C11 = df2_dup(integ1 - c * RaInv);       // c_11_12
+    const df2 K = C * XS - RI;                         // c_15_18 | c_19
+    const df2 D = L - (Y - C * X) * RI - CSq * XXS;    // c_17_19 | c_16
+    const df2 XD = X * D;                              // x c_17_19 | z_15_18
+    const df2 T = df2_dup(df_scale(integ4, 2.0f));     // c15_18_19
+    const df2 XSs = df2_swap(XS);
 
-  df64 RaSq_R_t2_I = RaInv / Ra_Rd_t2;
-  df64 yRaSq_R_t2_I = y * RaSq_R_t2_I;
-  df64 ySqRaSq_R_t2_I = y * yRaSq_R_t2_I;
+    const df64 v6 = (integ1 - df2_x(XS) - df2_y(XS)) * aSq_dSqI;
+    const df2 v78 = (S - C * df2_swap(S)) * Q;
+    const df64 v9 = (RaInv - c * (df2_x(XS) + df2_y(XS) + integ1)) * omcSqI;
+    const df2 vab = (XS + CSq * XSs + C11) * Q;
+    const df2 W = df2_swap(i23) - X * K;  // integ3 - x_13_14 | integ2 - y_13_14
+    const df2 vcd = (W - C * df2_swap(W)) * Q;
+    const df2 G = T - X * X * K;          // c15_18_19 - xSq c_15_18 | ... - ySq c_19
+    const df2 H = XD - i65;               // x c_17_19 - integ6 | z_15_18 - integ5
+    const df2 vhi = (G + C * df2_swap(H)) * Q;
+    const df64 v14 = (df2_y(H) + c * df2_x(G)) * omcSqI;  // -integ 14
+    const df2 vfg = (XXS + C * df2_swap(D) + df_scale(i23, 2.0f)) * Q;
 
-  df64 integ1 = df_scale(-den, 2.0f) * df_atan((df(1.0f) + c) * (Ra + x + y) * den);
-
-  df64 c_1 = aSq_dSq * integ1;
-  df64 c_5_6 = (c * Ra - c_1) * omcSqI;
-
-  df64 integ2 = (c * log_Ra_Rd_t2 - log_Ra_Rd_t1) * omcSqI;
-  df64 integ3 = (c * log_Ra_Rd_t1 - log_Ra_Rd_t2) * omcSqI;
-  df64 integ4 = (c * c_1 - Ra) * omcSqI;
-  df64 integ5 = ylog_Ra_Rd_t2 + c_5_6;
-  df64 integ6 = xlog_Ra_Rd_t1 + c_5_6;
-
-  df64 c_11_12 = integ1 - c * RaInv;
-  df64 c_15_18 = c * xRaSq_R_t1_I - RaInv;
-  df64 x_13_14 = x * c_15_18;
-  df64 c_19 = c * yRaSq_R_t2_I - RaInv;
-  df64 y_13_14 = y * c_19;
-  df64 c_16 = log_Ra_Rd_t2 - (x - c * y) * RaInv - cSq * ySqRaSq_R_t2_I;
-  df64 z_15_18 = y * c_16;
-  df64 c_17_19 = log_Ra_Rd_t1 - (y - c * x) * RaInv - cSq * xSqRaSq_R_t1_I;
-
-  df64 c15_18_19 = df_scale(integ4, 2.0f);
-
-  df64 v[19];
-  v[0] = integ1;
-  v[1] = integ2;
-  v[2] = integ3;
-  v[3] = integ4;
-  v[4] = integ5;
-  v[5] = integ6;
-  v[6] = (integ1 - xRaSq_R_t1_I - yRaSq_R_t2_I) * aSq_dSqI;
-  v[7] = (RaSq_R_t1_I - c * RaSq_R_t2_I) * omcSqI;
-  v[8] = (RaSq_R_t2_I - c * RaSq_R_t1_I) * omcSqI;
-  v[9] = (RaInv - c * (xRaSq_R_t1_I + yRaSq_R_t2_I + integ1)) * omcSqI;
-  v[10] = (xRaSq_R_t1_I + cSq * yRaSq_R_t2_I + c_11_12) * omcSqI;
-  v[11] = (yRaSq_R_t2_I + cSq * xRaSq_R_t1_I + c_11_12) * omcSqI;
-  v[12] = (integ3 - x_13_14 + c * (y_13_14 - integ2)) * omcSqI;
-  v[13] = (integ2 - y_13_14 + c * (x_13_14 - integ3)) * omcSqI;
-  v[14] = (integ5 - z_15_18 + c * (xSq * c_15_18 - c15_18_19)) * omcSqI;
-  v[15] = (xSqRaSq_R_t1_I + c * c_16 + df_scale(integ2, 2.0f)) * omcSqI;
-  v[16] = (ySqRaSq_R_t2_I + c * c_17_19 + df_scale(integ3, 2.0f)) * omcSqI;
-  v[17] = (c15_18_19 - xSq * c_15_18 + c * (z_15_18 - integ5)) * omcSqI;
-  v[18] = (c15_18_19 - ySq * c_19 + c * (x * c_17_19 - integ6)) * omcSqI;
+    // The corners' signs (+, -, -, +) as a factor: one body for all.
+    const float sg = q == 1 || q == 2 ? -1.0f : 1.0f;
+    const f2 sg2 = f2_dup(sg);
+    auto add1 = [&](df64& a, df64 v) { a = a + df_scale(v, sg); };
+    auto add2 = [&](df2& a, df2 v) { a = a + df2{v.hi * sg2, v.lo * sg2}; };
+    add1(s0, integ1);
+    add1(s3, integ4);
+    add1(s6, v6);
+    add1(s9, v9);
+    add1(s14, -v14);
+    add2(s12, i23);
+    add2(s54, i65);
+    add2(s78, v78);
+    add2(sab, vab);
+    add2(scd, vcd);
+    add2(sfg, vfg);
+    add2(shi, vhi);
+  }
+  out.c = c;
+  out.d = g.d;
+  out.x1 = g.x1;
+  out.x2 = g.x2;
+  out.y1 = g.y1;
+  out.y2 = g.y2;
+  const df64 all[19] = {s0,         df2_x(s12), df2_y(s12), s3,         df2_y(s54), df2_x(s54), s6,
+                        df2_x(s78), df2_y(s78), s9,         df2_x(sab), df2_y(sab), df2_x(scd), df2_y(scd),
+                        s14,        df2_x(sfg), df2_y(sfg), df2_x(shi), df2_y(shi)};
 #pragma unroll
-  for (int k = 0; k < 19; ++k) integ[k] = integ[k] + (neg ? -v[k] : v[k]);
+  for (int k = 0; k < 19; ++k) out.integ[k] = all[k];
 }
 
 DF_HD DV3 fsum11_df(const DV3* V, const df64* F) {
@@ -101,15 +170,14 @@ DF_HD DV3 fsum11_df(const DV3* V, const df64* F) {
   return s;
 }
 
-// General branch of calcSegSegForce in df64 (forces on seg 1 if NEED12, seg 2 if NEED34).
+// The node forces of the general branch from its integrals, in df64 (forces on
+// seg 1 if NEED12, seg 2 if NEED34).
 template <bool NEED12, bool NEED34>
-DF_HD void general_pair_df(const KConstsDF& K, DV3 b1, DV3 n11, DV3 n12, DV3 t1, df64 t1N, DV3 b2, DV3 n21, DV3 n22,
-                           DV3 t2, df64 t2N, df64 c, DV3& F1, DV3& F2, DV3& F3, DV3& F4) {
+DF_HD void assemble_df(const KConstsDF& K, const PairDF& g, DV3 b1, DV3 t1, df64 t1N, DV3 b2, DV3 t2, df64 t2N, DV3& F1,
+                       DV3& F2, DV3& F3, DV3& F4) {
+  const df64 c = g.c, d = g.d, x1 = g.x1, x2 = g.x2, y1 = g.y1, y2 = g.y2;
+  const df64* integ = g.integ;
   const df64 mu4pi = K.mu4pi, mu4pinu = K.mu4pinu, mu8piaSq = K.mu8piaSq, mu4pinuaSq = K.mu4pinuaSq;
-  df64 cSq = c * c;
-  df64 omcSq = df(1.0f) - cSq;
-  df64 omcSqI = df_recip(omcSq);
-
   DV3 t2ct1 = cross(t2, t1);
   DV3 t1ct2 = -t2ct1;
   DV3 b2ct2 = cross(b2, t2);
@@ -136,41 +204,12 @@ DF_HD void general_pair_df(const KConstsDF& K, DV3 b1, DV3 n11, DV3 n12, DV3 t1,
   df64 t1ct2cb2dt2 = t1db2 - t2db2 * c;
   df64 t2ct1cb1db2 = t2db1 * t1db2 - t1db1 * t2db2;
 
-  DV3 R1 = n21 - n11;
-  DV3 R2 = n22 - n12;
-  df64 d = dot(R2, t2ct1) * omcSqI;
-
   df64 mu4pid = mu4pi * d;
   df64 mu4pinud = mu4pinu * d;
   df64 mu4pinudSq = mu4pinud * d;
   df64 mu4pinudCu = mu4pinudSq * d;
   df64 mu4pinuaSqd = mu4pinuaSq * d;
   df64 mu8piaSqd = mu8piaSq * d;
-
-  df64 lim11 = dot(R1, t1);
-  df64 lim12 = dot(R1, t2);
-  df64 lim21 = dot(R2, t1);
-  df64 lim22 = dot(R2, t2);
-
-  df64 x1 = (lim12 - c * lim11) * omcSqI;
-  df64 x2 = (lim22 - c * lim21) * omcSqI;
-  df64 y1 = (lim11 - c * lim12) * omcSqI;
-  df64 y2 = (lim21 - c * lim22) * omcSqI;
-
-  df64 integ[19];
-#pragma unroll
-  for (int k = 0; k < 19; ++k) integ[k] = df(0.0f);
-  const df64 aSq_dSq = K.aSq + d * d * omcSq;
-  const df64 aSq_dSqI = df_recip(aSq_dSq);
-  const df64 den = df_recip(df_sqrt(omcSq * aSq_dSq));
-#ifdef __CUDACC__
-#pragma unroll 1
-#endif
-  for (int q = 0; q < 4; ++q) {
-    df64 x = (q & 2) ? x2 : x1;
-    df64 y = (q & 1) ? y2 : y1;
-    seg_seg_integ_df(aSq_dSq, aSq_dSqI, den, c, cSq, omcSqI, x, y, q == 1 || q == 2, integ);
-  }
 
   DV3 V[11];
   df64 Fi[11];
@@ -324,44 +363,12 @@ struct KConstsF {
 // Burgers vectors and powers of d, no cancellation of that order) in FP32.
 // The 11-term node sums are taken in df64 from FP32 V and df64 Fint.
 template <bool NEED12, bool NEED34, bool SUM32 = false>
-DF_HD void general_pair_mixed(const KConstsDF& K, const KConstsF& KF, F3 b1, DV3 n11, DV3 n12, DV3 t1, float t1N,
-                              F3 b2, DV3 n21, DV3 n22, DV3 t2, float t2N, df64 c, DV3& F1, DV3& F2, DV3& F3_,
-                              DV3& F4) {
-  df64 cSq = c * c;
-  df64 omcSq = df(1.0f) - cSq;
-  df64 omcSqI = df_recip(omcSq);
-
-  DV3 t2ct1d = cross(t2, t1);
-  DV3 R1 = n21 - n11;
-  DV3 R2 = n22 - n12;
-  df64 d = dot(R2, t2ct1d) * omcSqI;
-  df64 lim11 = dot(R1, t1);
-  df64 lim12 = dot(R1, t2);
-  df64 lim21 = dot(R2, t1);
-  df64 lim22 = dot(R2, t2);
-  df64 x1 = (lim12 - c * lim11) * omcSqI;
-  df64 x2 = (lim22 - c * lim21) * omcSqI;
-  df64 y1 = (lim11 - c * lim12) * omcSqI;
-  df64 y2 = (lim21 - c * lim22) * omcSqI;
-
-  df64 integ[19];
-#pragma unroll
-  for (int k = 0; k < 19; ++k) integ[k] = df(0.0f);
-  const df64 aSq_dSq = K.aSq + d * d * omcSq;
-  const df64 aSq_dSqI = df_recip(aSq_dSq);
-  const df64 den = df_recip(df_sqrt(omcSq * aSq_dSq));
-#ifdef __CUDACC__
-#pragma unroll 1
-#endif
-  for (int q = 0; q < 4; ++q) {
-    df64 x = (q & 2) ? x2 : x1;
-    df64 y = (q & 1) ? y2 : y1;
-    seg_seg_integ_df(aSq_dSq, aSq_dSqI, den, c, cSq, omcSqI, x, y, q == 1 || q == 2, integ);
-  }
-
+DF_HD void assemble_mixed(const KConstsF& KF, const PairDF& g, F3 b1, F3 ft1, float t1N, F3 b2, F3 ft2, float t2N,
+                          DV3& F1, DV3& F2, DV3& F3_, DV3& F4) {
+  const df64 c = g.c, d = g.d, x1 = g.x1, x2 = g.x2, y1 = g.y1, y2 = g.y2;
+  const df64* integ = g.integ;
   // FP32 geometry of the V vectors.
   const float mu4pi = KF.mu4pi, mu4pinu = KF.mu4pinu, mu8piaSq = KF.mu8piaSq, mu4pinuaSq = KF.mu4pinuaSq;
-  const F3 ft1 = f3(t1), ft2 = f3(t2);
   const float cf = c.hi;
   const float dfl = d.hi;
   F3 t2ct1 = cross(ft2, ft1);
@@ -387,24 +394,32 @@ DF_HD void general_pair_mixed(const KConstsDF& K, const KConstsF& KF, F3 b1, DV3
   float mu8piaSqd = mu8piaSq * dfl;
 
   F3 V[11];
-  df64 Fi[11];
   float tmp1, tmp2;
-  auto nodesum = [&](float tN) {
+  // First moments of both nodes of a segment in the lanes: A + Y b with A = +-a
+  // and Y = (-y2, y1) or (x2, -x1), then the 11-term node sums.
+  df2 Fi[11];
+  auto node = [&](float tN, auto lane) {
     if (SUM32) {
       F3 s = {0.f, 0.f, 0.f};
 #pragma unroll
-      for (int k = 0; k < 11; ++k) s = s + V[k] * (Fi[k].hi + Fi[k].lo);
+      for (int k = 0; k < 11; ++k) {
+        const df64 f = lane(Fi[k]);
+        s = s + V[k] * (f.hi + f.lo);
+      }
       return DV3{df(s.x * tN), df(s.y * tN), df(s.z * tN)};
     }
     DV3 s = {df(0.f), df(0.f), df(0.f)};
 #pragma unroll
     for (int k = 0; k < 11; ++k) {
-      s.x = s.x + Fi[k] * V[k].x;
-      s.y = s.y + Fi[k] * V[k].y;
-      s.z = s.z + Fi[k] * V[k].z;
+      const df64 f = lane(Fi[k]);
+      s.x = s.x + f * V[k].x;
+      s.y = s.y + f * V[k].y;
+      s.z = s.z + f * V[k].z;
     }
     return DV3{s.x * tN, s.y * tN, s.z * tN};
   };
+  auto first = [](df2 v) { return df2_x(v); };
+  auto second = [](df2 v) { return df2_y(v); };
   if (NEED12) {
     tmp1 = t1db2 * t2db1 + t2ct1cb1db2;
     F3 V1 = tmp1 * t2ct1;
@@ -438,30 +453,20 @@ DF_HD void general_pair_mixed(const KConstsDF& K, const KConstsF& KF, F3 b1, DV3
     V[9] = -tv * t2db1;
     V[10] = -tv * t1db1;
 
-    Fi[0] = integ[2] - y2 * integ[0];
-    Fi[1] = integ[3] - y2 * integ[1];
-    Fi[2] = integ[5] - y2 * integ[2];
-    Fi[3] = integ[8] - y2 * integ[6];
-    Fi[4] = integ[9] - y2 * integ[7];
-    Fi[5] = integ[11] - y2 * integ[8];
-    Fi[6] = integ[13] - y2 * integ[9];
-    Fi[7] = integ[12] - y2 * integ[10];
-    Fi[8] = integ[16] - y2 * integ[11];
-    Fi[9] = integ[14] - y2 * integ[12];
-    Fi[10] = integ[18] - y2 * integ[13];
-    F1 = nodesum(t1N);
-    Fi[0] = y1 * integ[0] - integ[2];
-    Fi[1] = y1 * integ[1] - integ[3];
-    Fi[2] = y1 * integ[2] - integ[5];
-    Fi[3] = y1 * integ[6] - integ[8];
-    Fi[4] = y1 * integ[7] - integ[9];
-    Fi[5] = y1 * integ[8] - integ[11];
-    Fi[6] = y1 * integ[9] - integ[13];
-    Fi[7] = y1 * integ[10] - integ[12];
-    Fi[8] = y1 * integ[11] - integ[16];
-    Fi[9] = y1 * integ[12] - integ[14];
-    Fi[10] = y1 * integ[13] - integ[18];
-    F2 = nodesum(t1N);
+    const df2 Y = df2_make(-y2, y1);
+    Fi[0] = df2_make(integ[2], -integ[2]) + Y * df2_dup(integ[0]);
+    Fi[1] = df2_make(integ[3], -integ[3]) + Y * df2_dup(integ[1]);
+    Fi[2] = df2_make(integ[5], -integ[5]) + Y * df2_dup(integ[2]);
+    Fi[3] = df2_make(integ[8], -integ[8]) + Y * df2_dup(integ[6]);
+    Fi[4] = df2_make(integ[9], -integ[9]) + Y * df2_dup(integ[7]);
+    Fi[5] = df2_make(integ[11], -integ[11]) + Y * df2_dup(integ[8]);
+    Fi[6] = df2_make(integ[13], -integ[13]) + Y * df2_dup(integ[9]);
+    Fi[7] = df2_make(integ[12], -integ[12]) + Y * df2_dup(integ[10]);
+    Fi[8] = df2_make(integ[16], -integ[16]) + Y * df2_dup(integ[11]);
+    Fi[9] = df2_make(integ[14], -integ[14]) + Y * df2_dup(integ[12]);
+    Fi[10] = df2_make(integ[18], -integ[18]) + Y * df2_dup(integ[13]);
+    F1 = node(t1N, first);
+    F2 = node(t1N, second);
   }
   if (NEED34) {
     tmp1 = t2db1 * t1db2 + t2ct1cb1db2;
@@ -496,31 +501,38 @@ DF_HD void general_pair_mixed(const KConstsDF& K, const KConstsF& KF, F3 b1, DV3
     V[9] = tv * t2db2;
     V[10] = tv * t1db2;
 
-    Fi[0] = x2 * integ[0] - integ[1];
-    Fi[1] = x2 * integ[1] - integ[4];
-    Fi[2] = x2 * integ[2] - integ[3];
-    Fi[3] = x2 * integ[6] - integ[7];
-    Fi[4] = x2 * integ[7] - integ[10];
-    Fi[5] = x2 * integ[8] - integ[9];
-    Fi[6] = x2 * integ[9] - integ[12];
-    Fi[7] = x2 * integ[10] - integ[15];
-    Fi[8] = x2 * integ[11] - integ[13];
-    Fi[9] = x2 * integ[12] - integ[17];
-    Fi[10] = x2 * integ[13] - integ[14];
-    F3_ = nodesum(t2N);
-    Fi[0] = integ[1] - x1 * integ[0];
-    Fi[1] = integ[4] - x1 * integ[1];
-    Fi[2] = integ[3] - x1 * integ[2];
-    Fi[3] = integ[7] - x1 * integ[6];
-    Fi[4] = integ[10] - x1 * integ[7];
-    Fi[5] = integ[9] - x1 * integ[8];
-    Fi[6] = integ[12] - x1 * integ[9];
-    Fi[7] = integ[15] - x1 * integ[10];
-    Fi[8] = integ[13] - x1 * integ[11];
-    Fi[9] = integ[17] - x1 * integ[12];
-    Fi[10] = integ[14] - x1 * integ[13];
-    F4 = nodesum(t2N);
+    const df2 Y = df2_make(x2, -x1);
+    Fi[0] = df2_make(-integ[1], integ[1]) + Y * df2_dup(integ[0]);
+    Fi[1] = df2_make(-integ[4], integ[4]) + Y * df2_dup(integ[1]);
+    Fi[2] = df2_make(-integ[3], integ[3]) + Y * df2_dup(integ[2]);
+    Fi[3] = df2_make(-integ[7], integ[7]) + Y * df2_dup(integ[6]);
+    Fi[4] = df2_make(-integ[10], integ[10]) + Y * df2_dup(integ[7]);
+    Fi[5] = df2_make(-integ[9], integ[9]) + Y * df2_dup(integ[8]);
+    Fi[6] = df2_make(-integ[12], integ[12]) + Y * df2_dup(integ[9]);
+    Fi[7] = df2_make(-integ[15], integ[15]) + Y * df2_dup(integ[10]);
+    Fi[8] = df2_make(-integ[13], integ[13]) + Y * df2_dup(integ[11]);
+    Fi[9] = df2_make(-integ[17], integ[17]) + Y * df2_dup(integ[12]);
+    Fi[10] = df2_make(-integ[14], integ[14]) + Y * df2_dup(integ[13]);
+    F3_ = node(t2N, first);
+    F4 = node(t2N, second);
   }
+}
+
+// General branch of calcSegSegForce in df64 and in the mixed form.
+template <bool NEED12, bool NEED34>
+DF_HD void general_pair_df(const KConstsDF& K, DV3 b1, DV3 n11, DV3 n12, DV3 t1, df64 t1N, DV3 b2, DV3 n21, DV3 n22,
+                           DV3 t2, df64 t2N, df64 c, DV3& F1, DV3& F2, DV3& F3, DV3& F4) {
+  PairDF g;
+  pair_integrals_df(K.aSq, t1, n11, n12, t2, n21, n22, c, g);
+  assemble_df<NEED12, NEED34>(K, g, b1, t1, t1N, b2, t2, t2N, F1, F2, F3, F4);
+}
+template <bool NEED12, bool NEED34, bool SUM32 = false>
+DF_HD void general_pair_mixed(const KConstsDF& K, const KConstsF& KF, F3 b1, DV3 n11, DV3 n12, DV3 t1, float t1N,
+                              F3 b2, DV3 n21, DV3 n22, DV3 t2, float t2N, df64 c, DV3& F1, DV3& F2, DV3& F3_,
+                              DV3& F4) {
+  PairDF g;
+  pair_integrals_df(K.aSq, t1, n11, n12, t2, n21, n22, c, g);
+  assemble_mixed<NEED12, NEED34, SUM32>(KF, g, b1, f3(t1), t1N, b2, f3(t2), t2N, F1, F2, F3_, F4);
 }
 
 // Constants of the mixed σ̃ form.
