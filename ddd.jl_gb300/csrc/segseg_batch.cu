@@ -13,10 +13,8 @@
 // in a fixed order.  Results are deterministic and equal, bit for bit, to the
 // per-network launches with the same tile size and arithmetic.
 //
-// Arithmetic: DDD_MODE_FP64 (strict), DDD_MODE_FP64_FAST (tile_pol_fx.cuh),
-// DDD_MODE_DF64, DDD_MODE_F32C.  The file is compiled with --fmad=false (strict
-// FP64 rounding, the fast form's explicit fused operations only, exact df64
-// transforms).
+// Arithmetic: DDD_MODE_FP64 (strict), DDD_MODE_FP64_FAST, DDD_MODE_DF64,
+// DDD_MODE_F32C; the tile kernels are tile_launch.cu's.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,20 +26,16 @@
 
 #include "../../include/ddd_gb300.h"
 #include "ddd_internal.h"
-#include "pair_df.cuh"
 #include "pair_f64.cuh"
-#include "tile_body.cuh"
-#include "tile_pol_df.cuh"
-#include "tile_pol_fx.cuh"
+#include "tile_launch.h"
 
 namespace ddd {
 namespace batch {
 
-template <int FORM>
-using PolDFb = PolDF<FORM>;  // tile_pol_df.cuh
-
 // The precision forms read the df64 SoA as well.
 bool uses_df(int mode) { return mode == DDD_MODE_DF64 || mode == DDD_MODE_F32C; }
+// The policy within its group (tile_launch.h).
+int second_policy(int mode) { return mode == DDD_MODE_F32C || mode == DDD_MODE_FP64_FAST ? 1 : 0; }
 
 // Padded SoA from the caller's packed 9 × ld array; src[g] = source column or -1.
 __global__ void prep_batched(const double* __restrict__ in, int64_t ldIn, const uint8_t* __restrict__ ext,
@@ -74,25 +68,6 @@ __global__ void prep_batched(const double* __restrict__ in, int64_t ldIn, const 
 #pragma unroll
   for (int k = 0; k < 13; ++k) soa[k * ntot + g] = v[k];
   skip[g] = sk;
-}
-
-// Work item: (slot, first row segment, first column segment, diagonal flag).
-template <int T, class P>
-__global__ void __launch_bounds__(T, 256 / T)
-persistent_tiles(TileArgs A, typename P::Consts KP, const int4* __restrict__ items, int32_t nItems,
-                 int32_t* __restrict__ next, double* __restrict__ partial, unsigned long long* __restrict__ counters) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  auto& sm = *reinterpret_cast<TileSmemT<T, P>*>(smem_raw);
-  __shared__ int32_t s_item;
-  for (;;) {
-    __syncthreads();  // the previous item's shared memory is no longer read
-    if (threadIdx.x == 0) s_item = atomicAdd(next, 1);
-    __syncthreads();
-    const int32_t w = s_item;
-    if (w >= nItems) break;
-    const int4 it = items[w];
-    tile_body<T, 0, P>(A, KP, sm, it.y, it.z, it.w != 0, partial + (int64_t)it.x * 12 * T, counters);
-  }
 }
 
 // Per segment (unpadded, caller order): sum of its row and column slots in a
@@ -265,33 +240,6 @@ KConsts kconsts(const ddd_consts* k) {
   return K;
 }
 
-// Shared-memory attribute and grid size of the persistent kernel, set up outside
-// any stream capture.
-template <int T, class P>
-cudaError_t prepare_persistent(int device, Layout& L) {
-  static std::atomic<uint64_t> attr{0};
-  const int smem = (int)sizeof(TileSmemT<T, P>);
-  cudaError_t e = set_smem_once(persistent_tiles<T, P>, smem, attr);
-  if (e != cudaSuccess) return e;
-  int sms = 0, per = 0;
-  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, persistent_tiles<T, P>, T, smem);
-  if (e != cudaSuccess) return e;
-  if (per < 1) per = 1;
-  const int64_t want = (int64_t)sms * per;
-  L.grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, L.nItems));
-  return cudaSuccess;
-}
-
-template <int T, class P>
-cudaError_t launch_persistent(const TileArgs& A, const typename P::Consts& KP, const Layout& L, int32_t* next,
-                              unsigned long long* counters, cudaStream_t st) {
-  persistent_tiles<T, P><<<L.grid, T, sizeof(TileSmemT<T, P>), st>>>(A, KP, (const int4*)L.items.p, (int32_t)L.nItems,
-                                                                     next, (double*)L.partial.p, counters);
-  return cudaGetLastError();
-}
-
 // The whole batch on stream st with layout L: counter reset, prep, tiles, reduction.
 cudaError_t enqueue(ddd_batch* b, Layout& L, const ddd_consts* k, const double* segs, const uint8_t* ext,
                     double* force, unsigned long long* counters, cudaStream_t st) {
@@ -308,21 +256,12 @@ cudaError_t enqueue(ddd_batch* b, Layout& L, const ddd_consts* k, const double* 
   const KConsts K = kconsts(k);
   const TileArgs A{K, (const double*)L.soa.p, (const uint8_t*)L.skip.p, ntot, (const float*)L.soadf.p, nullptr};
   int32_t* next = (int32_t*)b->next.p;
-  if (b->mode == DDD_MODE_FP64) {
-    e = L.T == 64 ? launch_persistent<64, PolF64>(A, PolF64::Consts{}, L, next, counters, st)
-                  : launch_persistent<128, PolF64>(A, PolF64::Consts{}, L, next, counters, st);
-  } else if (b->mode == DDD_MODE_FP64_FAST) {
-    e = L.T == 64 ? launch_persistent<64, PolF64Fast>(A, PolF64Fast::Consts{}, L, next, counters, st)
-                  : launch_persistent<128, PolF64Fast>(A, PolF64Fast::Consts{}, L, next, counters, st);
-  } else if (b->mode == DDD_MODE_DF64) {
-    const PolDFb<0>::Consts KP{kconsts_df(K), kconsts_f(K)};
-    e = L.T == 64 ? launch_persistent<64, PolDFb<0>>(A, KP, L, next, counters, st)
-                  : launch_persistent<128, PolDFb<0>>(A, KP, L, next, counters, st);
-  } else {
-    const PolDFb<1>::Consts KP{kconsts_df(K), kconsts_f(K)};
-    e = L.T == 64 ? launch_persistent<64, PolDFb<1>>(A, KP, L, next, counters, st)
-                  : launch_persistent<128, PolDFb<1>>(A, KP, L, next, counters, st);
-  }
+  const int pol = second_policy(b->mode);
+  const int4* items = (const int4*)L.items.p;
+  double* part = (double*)L.partial.p;
+  e = uses_df(b->mode) ? df_tiles::batch_launch(pol, L.T, A, L.grid, items, (int32_t)L.nItems, next, part, counters, st)
+                       : f64_tiles::batch_launch(pol, L.T, A, L.grid, items, (int32_t)L.nItems, next, part, counters,
+                                                 st);
   if (e != cudaSuccess) return e;
   const int64_t nNet = (int64_t)b->numSeg.size();
   if (b->totalSeg > 0) {
@@ -340,14 +279,9 @@ cudaError_t enqueue(ddd_batch* b, Layout& L, const ddd_consts* k, const double* 
 Layout& layout_of(ddd_batch* b, const Config& c) { return b->lay[c.T == 64 ? 0 : 1][c.order]; }
 
 cudaError_t prepare(ddd_batch* b, Layout& L) {
-  if (b->mode == DDD_MODE_FP64) return L.T == 64 ? prepare_persistent<64, PolF64>(b->device, L)
-                                                 : prepare_persistent<128, PolF64>(b->device, L);
-  if (b->mode == DDD_MODE_FP64_FAST) return L.T == 64 ? prepare_persistent<64, PolF64Fast>(b->device, L)
-                                                      : prepare_persistent<128, PolF64Fast>(b->device, L);
-  if (b->mode == DDD_MODE_DF64) return L.T == 64 ? prepare_persistent<64, PolDFb<0>>(b->device, L)
-                                                 : prepare_persistent<128, PolDFb<0>>(b->device, L);
-  return L.T == 64 ? prepare_persistent<64, PolDFb<1>>(b->device, L)
-                   : prepare_persistent<128, PolDFb<1>>(b->device, L);
+  const int pol = second_policy(b->mode);
+  return uses_df(b->mode) ? df_tiles::batch_prepare(pol, L.T, b->device, L.nItems, &L.grid)
+                          : f64_tiles::batch_prepare(pol, L.T, b->device, L.nItems, &L.grid);
 }
 
 std::string tune_key(const ddd_batch* b) {

@@ -38,8 +38,7 @@
 #include "surrogate.cuh"
 #include "surrogate_state.h"
 #include "tile_body.cuh"
-#include "tile_pol_df.cuh"
-#include "tile_pol_fx.cuh"
+#include "tile_launch.h"
 
 namespace ddd {
 
@@ -215,28 +214,6 @@ __global__ void near_items(const int4* __restrict__ all, int32_t nAll, const flo
   if (d2 < cut * cut) out[atomicAdd(count, 1)] = it;
 }
 
-// Persistent loop of the exact tile body (arithmetic policy P) over a work
-// list; the item count is read from the device (nDev) when given.
-template <int MODE, class P>
-__global__ void __launch_bounds__(T, 2)
-exact_tiles(TileArgs A, typename P::Consts KP, const int4* __restrict__ items, const int32_t* __restrict__ nDev,
-            int32_t nHost, int32_t* __restrict__ next, double* __restrict__ partial,
-            unsigned long long* __restrict__ counters) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  auto& sm = *reinterpret_cast<TileSmemT<T, P>*>(smem_raw);
-  __shared__ int32_t s_item;
-  const int32_t nItems = nDev ? *nDev : nHost;
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_item = atomicAdd(next, 1);
-    __syncthreads();
-    const int32_t w = s_item;
-    if (w >= nItems) break;
-    const int4 it = items[w];
-    tile_body<T, MODE, P>(A, KP, sm, it.y, it.z, it.w != 0, partial + (int64_t)it.x * 12 * T, counters);
-  }
-}
-
 // Per audited tile pair: squared error of the network's slot against the exact
 // far-pair slot, and the squared norm of the exact one (fixed-order tree).
 __global__ void audit_compare(const double* __restrict__ partial, const double* __restrict__ abuf,
@@ -396,38 +373,15 @@ uint32_t slot_hash(uint32_t x) {
   return x;
 }
 
-template <int MODE, class P>
-cudaError_t set_exact_attr() {
-  static std::atomic<uint64_t> done{0};
-  return set_smem_once(sf::exact_tiles<MODE, P>, (int)sizeof(TileSmemT<sf::T, P>), done);
-}
-
-template <int MODE, class P>
-cudaError_t launch_exact_p(const TileArgs& A, const typename P::Consts& KP, const int4* items, const int32_t* nDev,
-                           int32_t nHost, int32_t* next, double* partial, unsigned long long* counters, int grid,
-                           cudaStream_t st) {
-  cudaError_t e = set_exact_attr<MODE, P>();
-  if (e != cudaSuccess) return e;
-  sf::exact_tiles<MODE, P><<<grid, sf::T, sizeof(TileSmemT<sf::T, P>), st>>>(A, KP, items, nDev, nHost, next,
-                                                                             partial, counters);
-  return cudaGetLastError();
-}
-
 // The exact tile pass in the arithmetic of `mode` (DDD_MODE_FP64 strict,
 // DDD_MODE_FP64_FAST, DDD_MODE_DF64 or DDD_MODE_F32C for the general branch).
 template <int MODE>
 cudaError_t launch_exact(int mode, const TileArgs& A, const int4* items, const int32_t* nDev, int32_t nHost,
                          int32_t* next, double* partial, unsigned long long* counters, int grid, cudaStream_t st) {
-  if (mode == DDD_MODE_FP64)
-    return launch_exact_p<MODE, PolF64>(A, PolF64::Consts{}, items, nDev, nHost, next, partial, counters, grid, st);
-  if (mode == DDD_MODE_FP64_FAST)
-    return launch_exact_p<MODE, PolF64Fast>(A, PolF64Fast::Consts{}, items, nDev, nHost, next, partial, counters, grid,
-                                            st);
-  const typename PolDF<0>::Consts KP{kconsts_df(A.K), kconsts_f(A.K)};
-  if (mode == DDD_MODE_DF64)
-    return launch_exact_p<MODE, PolDF<0>>(A, KP, items, nDev, nHost, next, partial, counters, grid, st);
-  return launch_exact_p<MODE, PolDF<1>>(A, typename PolDF<1>::Consts{KP.K, KP.KF}, items, nDev, nHost, next, partial,
-                                        counters, grid, st);
+  if (mode == DDD_MODE_FP64 || mode == DDD_MODE_FP64_FAST)
+    return f64_tiles::exact_launch(mode == DDD_MODE_FP64_FAST, MODE, A, items, nDev, nHost, next, partial, counters,
+                                   grid, st);
+  return df_tiles::exact_launch(mode != DDD_MODE_DF64, MODE, A, items, nDev, nHost, next, partial, counters, grid, st);
 }
 
 cudaError_t ensure_plan(ddd_surrogate* s, int64_t numSeg, double auditFraction) {
@@ -442,11 +396,8 @@ cudaError_t ensure_plan(ddd_surrogate* s, int64_t numSeg, double auditFraction) 
     P.nItems = P.nt * (P.nt + 1) / 2;
     P.auditFraction = -1.0;
     if ((e = cudaDeviceGetAttribute(&P.sms, cudaDevAttrMultiProcessorCount, s->device)) != cudaSuccess) return e;
-    if ((e = set_exact_attr<2, PolF64>()) != cudaSuccess) return e;
     int per = 0;  // the df64 policies use the same shared memory and register budget
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sf::exact_tiles<2, PolF64>, sf::T,
-                                                           sizeof(TileSmemT<sf::T, PolF64>))) != cudaSuccess)
-      return e;
+    if ((e = f64_tiles::exact_occupancy(&per)) != cudaSuccess) return e;
     P.gridExact = P.sms * std::max(1, per);
     P.gridQuad = P.sms * quad_far_blocks_per_sm(3);
     const size_t n = (size_t)numSeg, np = (size_t)P.npad;
