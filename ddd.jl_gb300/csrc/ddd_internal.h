@@ -289,14 +289,14 @@ struct UTildeScratch {
   std::vector<double> explicitTri;
   GrowBuf order_d, ex_d, tri_d, u_d, part_d;
   int64_t lastTriangles = 0, lastChunks = 0;
-  int sms = 0, occStrict = 0, occFast = 0;
+  int sms = 0, occStrict[2] = {0, 0}, occFast[2] = {0, 0};  // CTAs per SM at 32 and 128 points
 };
 cudaError_t u_tilde_compute(const UTildeArgs& a, double* u, cudaEvent_t e0, cudaEvent_t e1, cudaStream_t st,
                             UTildeScratch& S);
-int u_field_fast_blocks_per_sm();
+int u_field_fast_blocks_per_sm(int pts);
 // Partial sums part[k][p] over triangle chunk k (K chunks of `chunk`).
 cudaError_t launch_u_field_fast(const double* tri, int64_t nTri, int64_t chunk, int64_t K, const double* points,
-                                int64_t M, double omNuInv8pi, double om2NuOmNuInv8pi, const double C[3], double* part,
+                                int64_t M, double omNuInv8pi, double om2NuOmNuInv8pi, const double C[3], double* part, int pts,
                                 cudaStream_t st);
 
 // ddd_api.cu: context accessors for the other C-ABI files.

@@ -25,24 +25,26 @@
 #include <vector>
 
 #include "ddd_internal.h"
+#include "f64reg.cuh"
 #include "intmath_f64.cuh"
 
 namespace ddd {
 namespace {
 
-constexpr int PT = 128;   // points per CTA of the field kernel
 constexpr int TCH = 32;   // triangles per shared-memory chunk
 constexpr int TROW = kUTriRows;  // doubles per triangle (layout below)
 
 struct V {
   double x, y, z;
 };
-__host__ __device__ __forceinline__ V operator+(V a, V b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-__host__ __device__ __forceinline__ V operator-(V a, V b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-__host__ __device__ __forceinline__ V operator*(V a, double s) { return {a.x * s, a.y * s, a.z * s}; }
-__host__ __device__ __forceinline__ double dot(V a, V b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__host__ __device__ __forceinline__ V cross(V a, V b) {
-  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+// Sums and products through rd (f64reg.cuh): the plain operations' bits.
+__device__ __forceinline__ V v3(rd x, rd y, rd z) { return {x, y, z}; }
+__device__ __forceinline__ V operator+(V a, V b) { return v3(rd(a.x) + b.x, rd(a.y) + b.y, rd(a.z) + b.z); }
+__device__ __forceinline__ V operator-(V a, V b) { return v3(rd(a.x) - b.x, rd(a.y) - b.y, rd(a.z) - b.z); }
+__device__ __forceinline__ V operator*(V a, rd s) { return v3(a.x * s, a.y * s, a.z * s); }
+__device__ __forceinline__ rd dot(V a, V b) { return rd(a.x) * b.x + rd(a.y) * b.y + rd(a.z) * b.z; }
+__device__ __forceinline__ V cross(V a, V b) {
+  return v3(rd(a.y) * b.z - rd(a.z) * b.y, rd(a.z) * b.x - rd(a.x) * b.z, rd(a.x) * b.y - rd(a.y) * b.x);
 }
 __device__ __forceinline__ V ld3(const double* a, int64_t n) { return {a[3 * n], a[3 * n + 1], a[3 * n + 2]}; }
 
@@ -51,8 +53,8 @@ __device__ __forceinline__ V ld3(const double* a, int64_t n) { return {a[3 * n],
 __device__ __forceinline__ double safe_norm(V& x) {
   const double n = sqrt(dot(x, x));
   if (n > DBL_EPSILON) {
-    const double inv = 1.0 / n;
-    x = {inv * x.x, inv * x.y, inv * x.z};
+    const rd inv = 1.0 / n;
+    x = v3(inv * x.x, inv * x.y, inv * x.z);
     return n;
   }
   x = {0.0, 0.0, 0.0};
@@ -181,31 +183,31 @@ __device__ __forceinline__ V tri_u(const double* s, double omNuInv8pi, double om
   // RC . RA here equals the previous triangle's RB . RC term by term.
   const double ta = acos(RAdRB), tb = acos(RBdRC), tc = (chained && closure && ch.closure) ? ch.tb : acos(RCdRA);
   ch = {RB, RBn, tb, closure, true};
-  const double th = (ta + tb + tc) / 2.0;
-  const double factor =
-      jl_max0(tan(th / 2.0) * tan((th - ta) / 2.0) * tan((th - tb) / 2.0) * tan((th - tc) / 2.0));
-  double omega = 4.0 * im::atan(sqrt(factor));
+  const rd th = (rd(ta) + tb + tc) * 0.5;  // halving is exact
+  const rd factor = jl_max0(rd(tan(th * 0.5)) * rd(tan((th - ta) * 0.5)) * rd(tan((th - tb) * 0.5)) *
+                            rd(tan((th - tc) * 0.5)));
+  rd omega = 4.0 * im::atan(sqrt(double(factor)));
   omega = -jl_sign(dot(RA, cross(CA, AB))) * omega;
-  const double fourPi = 4.0 * 3.141592653589793;
-  V u = {-b.x * omega / fourPi, -b.y * omega / fourPi, -b.z * omega / fourPi};
+  const rd fourPi = 4.0 * 3.141592653589793;
+  V u = v3(-b.x * omega / fourPi, -b.y * omega / fourPi, -b.z * omega / fourPi);
   if (s[21] == 0.0) return u;
   const V bAB = {s[23], s[24], s[25]}, bBC = {s[26], s[27], s[28]}, bCA = {s[29], s[30], s[31]};
-  const V fAB = bAB * im::log((RBn / RAn) * (1.0 + dot(RB, AB)) / (1.0 + dot(RA, AB)));
-  const V fBC = bBC * im::log((RCn / RBn) * (1.0 + dot(RC, BC)) / (1.0 + dot(RB, BC)));
-  const V fCA = bCA * im::log((RAn / RCn) * (1.0 + dot(RA, CA)) / (1.0 + dot(RC, CA)));
-  const double sAB = dot(b, cross(RA, RB)), sBC = dot(b, cross(RB, RC)), sCA = dot(b, cross(RC, RA));
+  const V fAB = bAB * rd(im::log((rd(RBn) / RAn) * (rd_one() + dot(RB, AB)) / (rd_one() + dot(RA, AB))));
+  const V fBC = bBC * rd(im::log((rd(RCn) / RBn) * (rd_one() + dot(RC, BC)) / (rd_one() + dot(RB, BC))));
+  const V fCA = bCA * rd(im::log((rd(RAn) / RCn) * (rd_one() + dot(RA, CA)) / (rd_one() + dot(RC, CA))));
+  const rd sAB = dot(b, cross(RA, RB)), sBC = dot(b, cross(RB, RC)), sCA = dot(b, cross(RC, RA));
   const V vAB = RA + RB, vBC = RB + RC, vCA = RC + RA;
-  const double dAB = 1.0 + RAdRB, dBC = 1.0 + RBdRC, dCA = 1.0 + RCdRA;
-  const V gAB = {sAB * vAB.x / dAB, sAB * vAB.y / dAB, sAB * vAB.z / dAB};
-  const V gBC = {sBC * vBC.x / dBC, sBC * vBC.y / dBC, sBC * vBC.z / dBC};
-  const V gCA = {sCA * vCA.x / dCA, sCA * vCA.y / dCA, sCA * vCA.z / dCA};
+  const rd dAB = rd_one() + RAdRB, dBC = rd_one() + RBdRC, dCA = rd_one() + RCdRA;
+  const V gAB = v3(sAB * vAB.x / dAB, sAB * vAB.y / dAB, sAB * vAB.z / dAB);
+  const V gBC = v3(sBC * vBC.x / dBC, sBC * vBC.y / dBC, sBC * vBC.z / dBC);
+  const V gCA = v3(sCA * vCA.x / dCA, sCA * vCA.y / dCA, sCA * vCA.z / dCA);
   const V fs = fAB + fBC + fCA, gs = gAB + gBC + gCA;
-  return u - V{om2NuOmNuInv8pi * fs.x, om2NuOmNuInv8pi * fs.y, om2NuOmNuInv8pi * fs.z} +
-         V{omNuInv8pi * gs.x, omNuInv8pi * gs.y, omNuInv8pi * gs.z};
+  return u - fs * om2NuOmNuInv8pi + gs * omNuInv8pi;
 }
 
 // Block (x, y): points x * PT.., triangles [y * chunk, (y + 1) * chunk), in
 // order; partial sums to part[y][p] (the reduce kernel adds them in y order).
+template <int PT>
 __global__ void __launch_bounds__(PT) u_field(const double* __restrict__ tri, int64_t nTri, int64_t chunk,
                                               const double* __restrict__ points, int64_t M, double omNuInv8pi,
                                               double om2NuOmNuInv8pi, V Cl, double* __restrict__ part) {
@@ -368,26 +370,34 @@ cudaError_t u_tilde_compute(const UTildeArgs& a, double* u, cudaEvent_t e0, cuda
   if ((e = S.order_d.ensure((size_t)std::max<int64_t>(nTri, 1) * 8)) != cudaSuccess) return e;
   if ((e = S.ex_d.ensure(std::max<size_t>(ex.size(), 1) * 8)) != cudaSuccess) return e;
   if ((e = S.tri_d.ensure((size_t)std::max<int64_t>(nTri, 1) * TROW * 8)) != cudaSuccess) return e;
-  // Triangle chunks of at least 256 triangles; one chunk keeps each point's
-  // sum strictly sequential.
   if (!S.sms) {
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&S.sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   }
-  int& occ = a.fast ? S.occFast : S.occStrict;
+  // Points per CTA: 128 from 1,024 points (the four warps of a CTA stay together
+  // and share their instruction fetch: 1,122 points x 16,384 triangles 20.0 ms
+  // against 20.4 with one-warp CTAs), below that 32, for the lanes that the last
+  // CTA leaves idle.
+  const bool wide = a.numPoints >= 1024;
+  const int pts = wide ? 128 : 32;
+  int& occ = a.fast ? S.occFast[wide] : S.occStrict[wide];
   if (!occ) {
     if (a.fast)
-      occ = u_field_fast_blocks_per_sm();
-    else if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, u_field, PT, 0)) != cudaSuccess)
+      occ = u_field_fast_blocks_per_sm(pts);
+    else if ((e = wide ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, u_field<128>, 128, 0)
+                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, u_field<32>, 32, 0)) != cudaSuccess)
       return e;
     occ = std::max(occ, 1);
   }
-  // As many chunks as fit the resident slots in one wave (equal chunks then
-  // finish together); many points alone fill the GPU with one chunk.
-  const int64_t bx = (a.numPoints + PT - 1) / PT;
+  // As many chunks as fit the resident CTAs in one wave (equal chunks then finish
+  // together; a chunk's first triangle cannot reuse its predecessor's node, so no
+  // more), of at least 8 triangles.  128-point CTAs in chunks of at least 256 made
+  // 650 points x 8,192 triangles 192 CTAs for 152 SMs (10.6 ms, now 6.2) and 90
+  // points x 64 triangles one (1.56 ms, now 0.30).
+  const int64_t bx = (a.numPoints + pts - 1) / pts;
   const int64_t want = std::max<int64_t>(1, (int64_t)S.sms * occ / std::max<int64_t>(bx, 1));
-  const int64_t K = std::max<int64_t>(1, std::min<int64_t>({want, (nTri + 255) / 256, 65535}));
+  const int64_t K = std::max<int64_t>(1, std::min<int64_t>({want, (nTri + 7) / 8, 65535}));
   const int64_t chunk = std::max<int64_t>(1, (nTri + K - 1) / K);
   S.lastChunks = K;
   if ((e = S.u_d.ensure((size_t)std::max<int64_t>(a.numPoints, 1) * 3 * 8)) != cudaSuccess) return e;
@@ -407,12 +417,17 @@ cudaError_t u_tilde_compute(const UTildeArgs& a, double* u, cudaEvent_t e0, cuda
   }
   if (a.numPoints > 0 && a.fast) {
     if ((e = launch_u_field_fast((const double*)S.tri_d.p, nTri, chunk, K, a.pointsDev, a.numPoints, a.omNuInv8pi,
-                                 a.om2NuOmNuInv8pi, a.C, (double*)S.part_d.p, st)) != cudaSuccess)
+                                 a.om2NuOmNuInv8pi, a.C, (double*)S.part_d.p, pts, st)) != cudaSuccess)
       return e;
   } else if (a.numPoints > 0) {
-    u_field<<<dim3((unsigned)bx, (unsigned)K), PT, 0, st>>>((const double*)S.tri_d.p, nTri, chunk, a.pointsDev,
-                                                            a.numPoints, a.omNuInv8pi, a.om2NuOmNuInv8pi,
-                                                            V{a.C[0], a.C[1], a.C[2]}, (double*)S.part_d.p);
+    const dim3 grid((unsigned)bx, (unsigned)K);
+    const V Cl{a.C[0], a.C[1], a.C[2]};
+    if (wide)
+      u_field<128><<<grid, 128, 0, st>>>((const double*)S.tri_d.p, nTri, chunk, a.pointsDev, a.numPoints, a.omNuInv8pi,
+                                         a.om2NuOmNuInv8pi, Cl, (double*)S.part_d.p);
+    else
+      u_field<32><<<grid, 32, 0, st>>>((const double*)S.tri_d.p, nTri, chunk, a.pointsDev, a.numPoints, a.omNuInv8pi,
+                                       a.om2NuOmNuInv8pi, Cl, (double*)S.part_d.p);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (a.numPoints > 0) {

@@ -24,12 +24,11 @@
 #include <cuda_runtime.h>
 
 #include "ddd_internal.h"
+#include "f64reg.cuh"
 #include "intmath_f64.cuh"
 
 namespace ddd {
 namespace {
-
-constexpr int PT = 128;
 
 // atan2(y, x) for y > 0 on the integer pipes: the quotient rounded once, then
 // im::atan (within ~1 ulp; CUDA documents 2 ulp for its atan2).
@@ -45,12 +44,14 @@ constexpr int TROW = kUTriRows;
 struct V {
   double x, y, z;
 };
-__device__ __forceinline__ V operator+(V a, V b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ V operator-(V a, V b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ V operator*(V a, double s) { return {a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ double dot(V a, V b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// Sums and products through rd (f64reg.cuh): the plain operations' bits.
+__device__ __forceinline__ V v3(rd x, rd y, rd z) { return {x, y, z}; }
+__device__ __forceinline__ V operator+(V a, V b) { return v3(rd(a.x) + b.x, rd(a.y) + b.y, rd(a.z) + b.z); }
+__device__ __forceinline__ V operator-(V a, V b) { return v3(rd(a.x) - b.x, rd(a.y) - b.y, rd(a.z) - b.z); }
+__device__ __forceinline__ V operator*(V a, rd s) { return v3(a.x * s, a.y * s, a.z * s); }
+__device__ __forceinline__ rd dot(V a, V b) { return rd(a.x) * b.x + rd(a.y) * b.y + rd(a.z) * b.z; }
 __device__ __forceinline__ V cross(V a, V b) {
-  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+  return v3(rd(a.y) * b.z - rd(a.z) * b.y, rd(a.z) * b.x - rd(a.x) * b.z, rd(a.x) * b.y - rd(a.y) * b.x);
 }
 
 // safeNorm (Misc.jl:289-300), as the reference-order kernel: |x| (eps when
@@ -58,8 +59,8 @@ __device__ __forceinline__ V cross(V a, V b) {
 __device__ __forceinline__ double unit(V& x) {
   const double n = sqrt(dot(x, x));
   if (n > DBL_EPSILON) {
-    const double inv = 1.0 / n;
-    x = {inv * x.x, inv * x.y, inv * x.z};
+    const rd inv = 1.0 / n;
+    x = v3(inv * x.x, inv * x.y, inv * x.z);
     return n;
   }
   x = {0.0, 0.0, 0.0};
@@ -70,6 +71,7 @@ __device__ __forceinline__ double jl_max0(double x) { return isnan(x) ? x : ((x 
 __device__ __forceinline__ double clamp11(double x) { return x > 1.0 ? 1.0 : (x < -1.0 ? -1.0 : x); }
 __device__ __forceinline__ double jl_sign(double x) { return x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : x); }
 
+template <int PT>
 __global__ void __launch_bounds__(PT) u_field_fast(const double* __restrict__ tri, int64_t nTri, int64_t chunk,
                                                    const double* __restrict__ points, int64_t M, double k1, double k2,
                                                    V Cl, double* __restrict__ part) {
@@ -117,12 +119,12 @@ __global__ void __launch_bounds__(PT) u_field_fast(const double* __restrict__ tr
       prevRBn = RBn;
       prevValid = true;
       const V AB = {s[12], s[13], s[14]}, BC = {s[15], s[16], s[17]}, CA = {s[18], s[19], s[20]};
-      const double ab = dot(RA, RB), bc = dot(RB, RC), ca = dot(RC, RA);
+      const rd ab = dot(RA, RB), bc = dot(RB, RC), ca = dot(RC, RA);
       const double num = dot(RA, cross(RB, RC));
       const double sgn = -jl_sign(dot(RA, cross(CA, AB)));
       double om;
       if (fabs(num) > 1e-10) {
-        om = sgn * (2.0 * atan2_pos(fabs(num), 1.0 + ab + bc + ca));
+        om = sgn * (2.0 * atan2_pos(fabs(num), rd_one() + ab + bc + ca));
       } else {  // (nearly) in the triangle's plane: the reference's expression
         const double ta = acos(clamp11(ab)), tb = acos(clamp11(bc)), tc = acos(clamp11(ca));
         const double th = (ta + tb + tc) / 2.0;
@@ -131,21 +133,21 @@ __global__ void __launch_bounds__(PT) u_field_fast(const double* __restrict__ tr
         om = sgn * (4.0 * im::atan(sqrt(f)));
       }
       const double fourPi = 4.0 * 3.141592653589793;
-      acc = acc + V{-s[9] * om / fourPi, -s[10] * om / fourPi, -s[11] * om / fourPi};
+      acc = acc + v3(-s[9] * rd(om) / fourPi, -s[10] * rd(om) / fourPi, -s[11] * rd(om) / fourPi);
       if (s[21] == 0.0) continue;
       const V b = {s[9], s[10], s[11]};
-      const double lAB = im::log((RBn * (1.0 + dot(RB, AB))) / (RAn * (1.0 + dot(RA, AB))));
+      const double lAB = im::log((RBn * (rd_one() + dot(RB, AB))) / (RAn * (rd_one() + dot(RA, AB))));
       V fs = V{s[23], s[24], s[25]} * lAB;
-      V gs = (RA + RB) * (dot(b, cross(RA, RB)) / (1.0 + clamp11(ab)));
+      V gs = (RA + RB) * (dot(b, cross(RA, RB)) / (rd_one() + clamp11(ab)));
       if (!(link & 4)) {
-        const double lBC = im::log((RCn * (1.0 + dot(RC, BC))) / (RBn * (1.0 + dot(RB, BC))));
+        const double lBC = im::log((RCn * (rd_one() + dot(RC, BC))) / (RBn * (rd_one() + dot(RB, BC))));
         fs = fs + V{s[26], s[27], s[28]} * lBC;
-        gs = gs + (RB + RC) * (dot(b, cross(RB, RC)) / (1.0 + clamp11(bc)));
+        gs = gs + (RB + RC) * (dot(b, cross(RB, RC)) / (rd_one() + clamp11(bc)));
       }
       if (!(link & 8)) {
-        const double lCA = im::log((RAn * (1.0 + dot(RA, CA))) / (RCn * (1.0 + dot(RC, CA))));
+        const double lCA = im::log((RAn * (rd_one() + dot(RA, CA))) / (RCn * (rd_one() + dot(RC, CA))));
         fs = fs + V{s[29], s[30], s[31]} * lCA;
-        gs = gs + (RC + RA) * (dot(b, cross(RC, RA)) / (1.0 + clamp11(ca)));
+        gs = gs + (RC + RA) * (dot(b, cross(RC, RA)) / (rd_one() + clamp11(ca)));
       }
       acc = acc - fs * k2 + gs * k1;
     }
@@ -160,18 +162,23 @@ __global__ void __launch_bounds__(PT) u_field_fast(const double* __restrict__ tr
 
 }  // namespace
 
-int u_field_fast_blocks_per_sm() {
+int u_field_fast_blocks_per_sm(int pts) {
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, u_field_fast, PT, 0) != cudaSuccess) return 1;
-  return occ;
+  const cudaError_t e = pts == 128 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, u_field_fast<128>, 128, 0)
+                                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, u_field_fast<32>, 32, 0);
+  return e == cudaSuccess ? occ : 1;
 }
 
 cudaError_t launch_u_field_fast(const double* tri, int64_t nTri, int64_t chunk, int64_t K, const double* points,
                                 int64_t M, double omNuInv8pi, double om2NuOmNuInv8pi, const double C[3], double* part,
-                                cudaStream_t st) {
+                                int pts, cudaStream_t st) {
   if (M <= 0) return cudaSuccess;
-  u_field_fast<<<dim3((unsigned)((M + PT - 1) / PT), (unsigned)K), PT, 0, st>>>(
-      tri, nTri, chunk, points, M, omNuInv8pi, om2NuOmNuInv8pi, V{C[0], C[1], C[2]}, part);
+  const dim3 grid((unsigned)((M + pts - 1) / pts), (unsigned)K);
+  const V Cl{C[0], C[1], C[2]};
+  if (pts == 128)
+    u_field_fast<128><<<grid, 128, 0, st>>>(tri, nTri, chunk, points, M, omNuInv8pi, om2NuOmNuInv8pi, Cl, part);
+  else
+    u_field_fast<32><<<grid, 32, 0, st>>>(tri, nTri, chunk, points, M, omNuInv8pi, om2NuOmNuInv8pi, Cl, part);
   return cudaGetLastError();
 }
 

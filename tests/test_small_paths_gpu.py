@@ -79,3 +79,26 @@ def test_sigma_few_points(pkg, synth, mode, rel, nseg):
             assert np.all(np.abs(part - whole[:, :m]) <= rel * np.abs(whole).max())
     finally:
         ctx.mode = "fp64"
+
+
+@pytest.mark.parametrize("mode,rel", [("fp64", 1e-12), ("fp64_fast", 1e-12)])
+@pytest.mark.parametrize("nseg", [1, 8, 9, 2000])
+def test_u_tilde_few_points(pkg, synth, mode, rel, nseg):
+    """calc_uTilde at 1, 33 and 1,023 points (one-warp CTAs, chunks from 8
+    triangles) against the same points inside a call of 1,024 (128-point CTAs,
+    other chunks): the same triangles in another grouping of at most 2,000 terms."""
+    from ddd_gb300 import fem
+    net = _synthetic(pkg, synth, 250, 11, cube=2000.0)
+    net.numSeg = nseg
+    mat = pkg.MaterialParameters(mu=1.0, nu=0.28)
+    mesh = fem.RegularCuboidMesh(2000.0, 2000.0, 2000.0, 4, 4, 4)
+    pts = np.asfortranarray(np.random.default_rng(nseg).uniform(-500.0, 2500.0, (3, 1024)))
+    ctx = pkg.get_context()
+    ctx.mode = mode
+    try:
+        whole = ctx.u_tilde(mat.omνInv8π, mat.om2νomνInv8π, mesh, pts, net)
+        for m in (1, 33, 1023):
+            part = ctx.u_tilde(mat.omνInv8π, mat.om2νomνInv8π, mesh, np.asfortranarray(pts[:, :m]), net)
+            assert np.all(np.abs(part - whole[:3 * m]) <= rel * np.abs(whole).max())
+    finally:
+        ctx.mode = "fp64"
