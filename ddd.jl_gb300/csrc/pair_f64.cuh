@@ -143,9 +143,20 @@ __device__ __forceinline__ D3 fsum11(const D3* V, const rd* F) {
   return s;
 }
 
+// The four corners' sum of an integral whose corner q lane 4 p + q holds, in the
+// corner loop's order and rounding.
+__device__ __forceinline__ rd quad_sum(rd v) {
+  rd s = rd(0.0) + rd(__shfl_sync(0xffffffffu, double(v), 0, 4));
+  s = s + -rd(__shfl_sync(0xffffffffu, double(v), 1, 4));
+  s = s + -rd(__shfl_sync(0xffffffffu, double(v), 2, 4));
+  return s + rd(__shfl_sync(0xffffffffu, double(v), 3, 4));
+}
+
 // General branch (1 - c^2 > sqrt(eps)) of calcSegSegForce.  NEED12 / NEED34 drop
 // the work of the forces on segment 1 / segment 2 when the caller discards them.
-template <bool NEED12, bool NEED34>
+// QUAD: the four lanes 4 p .. 4 p + 3 of a full warp hold the same pair and take
+// one corner each (all get the forces).
+template <bool NEED12, bool NEED34, bool QUAD = false>
 __device__ __forceinline__ void general_pair(const KConsts& K, D3 b1, D3 n11, D3 n12, D3 t1, rd t1N, D3 b2, D3 n21,
                                              D3 n22, D3 t2, rd t2N, rd c, D3& F1, D3& F2, D3& F3, D3& F4) {
   const rd mu4pi = K.mu4pi, mu4pinu = K.mu4pinu, mu8piaSq = K.mu8piaSq, mu4pinuaSq = K.mu4pinuaSq;
@@ -206,8 +217,14 @@ __device__ __forceinline__ void general_pair(const KConsts& K, D3 b1, D3 n11, D3
   const rd aSq_dSq = K.aSq + d * d * omcSq;
   const rd den = 1.0 / sqrt(omcSq * aSq_dSq);
   // ((I(x1,y1) - I(x1,y2)) - I(x2,y1)) + I(x2,y2), DislocationForces.jl:948-951.
+  if (QUAD) {
+    const int q = threadIdx.x & 3;
+    seg_seg_integ_acc(aSq_dSq, den, c, cSq, omcSqI, (q & 2) ? x2 : x1, (q & 1) ? y2 : y1, 0ull, integ);
+#pragma unroll
+    for (int k = 0; k < 19; ++k) integ[k] = quad_sum(integ[k]);
+  }
 #pragma unroll 1
-  for (int q = 0; q < 4; ++q) {
+  for (int q = QUAD ? 4 : 0; q < 4; ++q) {
     rd x = (q & 2) ? x2 : x1;
     rd y = (q & 1) ? y2 : y1;
     unsigned long long sm = (q == 1 || q == 2) ? 0x8000000000000000ull : 0ull;
@@ -513,6 +530,25 @@ __device__ __forceinline__ int parallel_pair(const KConsts& K, D3 b1, D3 n11, D3
     D3 tmp = F1;
     F1 = F2;
     F2 = tmp;
+  }
+  return cores;
+}
+
+// One side of calcParSegSegForce for the pair (a, b): SIDE 1 the forces on a's
+// nodes, SIDE 2 those on b's, with parallel_pair's operations.
+template <int SIDE>
+__device__ __forceinline__ int parallel_pair_side(const KConsts& K, const SegF64& a, const SegF64& b, D3& Fa, D3& Fb) {
+  const bool flip = dot(a.t, b.t) < 0.0;
+  const D3 n11 = flip ? a.n2 : a.n1, n12 = flip ? a.n1 : a.n2;
+  const D3 t1 = flip ? -a.t : a.t, b1 = flip ? -a.b : a.b;
+  int cores;
+  if (SIDE == 1) {
+    D3 F1, F2;
+    cores = par_side<1>(K, n11, n12, t1, a.tN, b1, b.n1, b.n2, b.t, b.tN, b.b, F1, F2);
+    Fa = flip ? F2 : F1;
+    Fb = flip ? F1 : F2;
+  } else {
+    cores = par_side<2>(K, b.n1, b.n2, b.t, b.tN, b.b, n11, n12, t1, a.tN, b1, Fa, Fb);
   }
   return cores;
 }

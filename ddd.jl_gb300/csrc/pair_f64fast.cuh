@@ -150,8 +150,29 @@ FM_HD void corner(const CornerK& P, rd x, rd y, long long sm, rd* integ) {
   }
 }
 
-// General branch of calcSegSegForce; NEED12 / NEED34 as in pair_f64.cuh.
-template <bool NEED12, bool NEED34, int FMATH>
+// The corners' sum over the lanes of a pair (pair_f64.cuh's QUAD form).
+FM_HD rd quad_total(rd v) {
+#if defined(__CUDA_ARCH__)
+  rd s = __shfl_sync(0xffffffffu, double(v), 0, 4);
+  s += -rd(__shfl_sync(0xffffffffu, double(v), 1, 4));
+  s += -rd(__shfl_sync(0xffffffffu, double(v), 2, 4));
+  s += rd(__shfl_sync(0xffffffffu, double(v), 3, 4));
+  return s;
+#else
+  return v;
+#endif
+}
+FM_HD int quad_lane() {
+#if defined(__CUDA_ARCH__)
+  return threadIdx.x & 3;
+#else
+  return 0;
+#endif
+}
+
+// General branch of calcSegSegForce; NEED12 / NEED34 / QUAD as in pair_f64.cuh
+// (QUAD on the GPU only).
+template <bool NEED12, bool NEED34, int FMATH, bool QUAD = false>
 FM_HD void general_pair(const KFast& K, X3 b1, X3 n11, X3 n12, X3 t1, rd t1N, X3 b2, X3 n21, X3 n22, X3 t2,
                         rd t2N, rd c, X3& F1, X3& F2, X3& F3, X3& F4) {
   const rd mu4pi = K.mu4pi, mu4pinu = K.mu4pinu, mu8piaSq = K.mu8piaSq, mu4pinuaSq = K.mu4pinuaSq;
@@ -212,9 +233,16 @@ FM_HD void general_pair(const KFast& K, X3 b1, X3 n11, X3 n12, X3 t1, rd t1N, X3
   const rd den = 1.0 / sqrt(omcSq * aSq_dSq);
   const CornerK P{aSq_dSq, c, cSq, omcSqI, twice(c), (rd_one() + c) * den, -twice(den)};
   // ((I(x1,y1) - I(x1,y2)) - I(x2,y1)) + I(x2,y2), DislocationForces.jl:948-951.
-  corner<FMATH, true>(P, x1, y1, 0LL, integ);
+  if (QUAD) {
+    const int q = quad_lane();
+    corner<FMATH, true>(P, (q & 2) ? x2 : x1, (q & 1) ? y2 : y1, 0LL, integ);
+#pragma unroll
+    for (int k = 0; k < 19; ++k) integ[k] = quad_total(integ[k]);
+  } else {
+    corner<FMATH, true>(P, x1, y1, 0LL, integ);
+  }
 #pragma unroll 1
-  for (int q = 1; q < 4; ++q) {
+  for (int q = QUAD ? 4 : 1; q < 4; ++q) {
     const rd x = (q & 2) ? x2 : x1;
     const rd y = (q & 1) ? y2 : y1;
     const long long sm = (q == 1 || q == 2) ? (long long)0x8000000000000000ULL : 0LL;

@@ -173,8 +173,8 @@ cudaError_t launch_segseg_small_df(const KConsts& K, const double* soa, const fl
   const KConstsDF kd = kconsts_df(K);
   const KConstsF kf = kconsts_f(K);
   cudaError_t e =
-      form ? launch_expanded<PolDF<1>>(A, PolDF<1>::Consts{kd, kf}, nb, scratch, partial, counters, st)
-           : launch_expanded<PolDF<0>>(A, PolDF<0>::Consts{kd, kf}, nb, scratch, partial, counters, st);
+      form ? launch_expanded<PolDF<1>>(A, PolDF<1>::Consts{kd, kf}, nb, numSeg, scratch, partial, counters, st)
+           : launch_expanded<PolDF<0>>(A, PolDF<0>::Consts{kd, kf}, nb, numSeg, scratch, partial, counters, st);
   return e != cudaSuccess ? e : strict::launch_reduce_all(partial, npad, numSeg, out, st);
 }
 

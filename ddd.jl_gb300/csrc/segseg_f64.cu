@@ -281,7 +281,8 @@ cudaError_t launch_segseg_small_f64(const KConsts& K, const double* soa, const u
                                     unsigned long long* counters, cudaStream_t st) {
   const int64_t nt = npad / TILE;
   const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
-  cudaError_t e = launch_expanded<PolF64>(A, PolF64::Consts{}, nt * (nt + 1) / 2, scratch, partial, counters, st);
+  cudaError_t e = launch_expanded<PolF64>(A, PolF64::Consts{}, nt * (nt + 1) / 2, numSeg, scratch, partial,
+                                          counters, st);
   return e != cudaSuccess ? e : launch_reduce_all(partial, npad, numSeg, out, st);
 }
 

@@ -79,7 +79,8 @@ cudaError_t launch_segseg_small_fx(const KConsts& K, const double* soa, const ui
   const int64_t nt = npad / TILE;
   const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
   cudaError_t e =
-      launch_expanded<PolF64Fast>(A, PolF64Fast::Consts{}, nt * (nt + 1) / 2, scratch, partial, counters, st);
+      launch_expanded<PolF64Fast>(A, PolF64Fast::Consts{}, nt * (nt + 1) / 2, numSeg, scratch, partial,
+                                          counters, st);
   return e != cudaSuccess ? e : strict::launch_reduce_all(partial, npad, numSeg, out, st);
 }
 

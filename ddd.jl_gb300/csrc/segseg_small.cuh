@@ -23,6 +23,7 @@ namespace {
 constexpr int XT = 128;               // tile of the all-pairs kernels
 constexpr int XPOS = XT * XT;         // pair positions (step k, row t) of one tile pair
 constexpr int kParCtas = 1216;        // near-parallel warps: 8 per SM
+constexpr int64_t kQuadSegs = 64;     // four lanes per pair up to here
 
 __device__ __forceinline__ void x_tile_index(int64_t b, int64_t& I, int64_t& J) {
   int64_t Jc = (int64_t)((sqrt(8.0 * (double)b + 1.0) - 1.0) * 0.5);
@@ -74,30 +75,43 @@ x_classify(const double* __restrict__ soa, const uint8_t* __restrict__ skip, int
 
 // One warp per CTA.  The first kParCtas warps share the near-parallel list,
 // every other one takes the 32 rows of a warp of one step: its general pairs.
-template <class P>
+// QUAD: 8 rows, four lanes per pair with a corner each.  A pair on its own is one
+// chain of ~1,600 FP64 instructions at 64 cycles, 76 us; four lanes shorten it and
+// repeat the rest of the pair's work, which pays while an SM has under two such
+// warps: up to 64 segments (2,016 pairs).  24 segments: 150 -> 132 us per call; at
+// 128 it costs 3 %.
+template <class P, bool QUAD>
 __global__ void __launch_bounds__(32)
 x_pairs(TileArgs A, typename P::Consts KP, const uint8_t* __restrict__ flags, const uint32_t* __restrict__ list,
         const unsigned* __restrict__ count, double* __restrict__ vals, unsigned long long* __restrict__ counters) {
   const int lane = threadIdx.x;
   if (blockIdx.x < kParCtas) {
-    const unsigned n = *count;
+    // Even CTAs take the forces on segment 1, odd ones those on segment 2: a short
+    // list is bound by one side's chain of dependent operations, not by both.
+    const unsigned n = *count, side = blockIdx.x & 1;
     unsigned long long nCore = 0;
-    for (unsigned e = blockIdx.x * 32u + lane; e < n; e += kParCtas * 32u) {
+    for (unsigned e = (blockIdx.x >> 1) * 32u + lane; e < n; e += kParCtas / 2 * 32u) {
       const uint32_t pos = list[e];
       const int t = pos & (XT - 1), k = (pos >> 7) & (XT - 1), jl = (t + k) & (XT - 1);
       int64_t I, J;
       x_tile_index(pos >> 14, I, J);
-      nCore += tb_parallel_pair(A, I * XT + t, J * XT + jl, vals + (int64_t)(pos >> 7) * 12 * XT + t, XT);
+      const SegF64 a = tb_load_seg64(A.soa, A.npad, I * XT + t), s = tb_load_seg64(A.soa, A.npad, J * XT + jl);
+      D3 F1, F2;
+      nCore += side ? parallel_pair_side<2>(A.K, a, s, F1, F2) : parallel_pair_side<1>(A.K, a, s, F1, F2);
+      double* v = vals + ((int64_t)(pos >> 7) * 12 + 6 * side) * XT + t;
+      v[0 * XT] = F1.x; v[1 * XT] = F1.y; v[2 * XT] = F1.z;
+      v[3 * XT] = F2.x; v[4 * XT] = F2.y; v[5 * XT] = F2.z;
     }
     if (counters && nCore) atomicAdd(&counters[2], nCore);
     return;
   }
   const unsigned u = blockIdx.x - kParCtas;
-  const int64_t bk = u >> 2;  // 128 b + k
-  const int t = (int)((u & 3) * 32 + lane);
+  constexpr int kWarps = QUAD ? 16 : 4;  // per step
+  const int64_t bk = u / kWarps;  // 128 b + k
+  const int t = QUAD ? (int)(u % kWarps) * 8 + (lane >> 2) : (int)(u % kWarps) * 32 + lane;
   const bool act = flags[bk * XT + t] == 1;
   if (!__any_sync(0xffffffffu, act)) return;
-  if (!act) return;
+  if (!QUAD && !act) return;  // a warp of quads stays whole: its lanes exchange corners
   int64_t I, J;
   x_tile_index(bk >> 7, I, J);
   const int64_t i = I * XT + t, j = J * XT + ((t + (int)(bk & (XT - 1))) & (XT - 1));
@@ -105,7 +119,11 @@ x_pairs(TileArgs A, typename P::Consts KP, const uint8_t* __restrict__ flags, co
   typename P::Scalar c;
   P::is_general(A, a, s, i, j, c);  // c; the class is the same FP64 decision
   typename P::Vec F1, F2, F3, F4;
-  P::template general<true>(KP, A, a, s, c, F1, F2, F3, F4);
+  if constexpr (QUAD)
+    P::template general<true, true>(KP, A, a, s, c, F1, F2, F3, F4);
+  else
+    P::template general<true>(KP, A, a, s, c, F1, F2, F3, F4);
+  if (QUAD && (!act || (lane & 3))) return;
   double* v = vals + bk * 12 * XT + t;
   v[0 * XT] = P::pack(F1.x); v[1 * XT] = P::pack(F1.y); v[2 * XT] = P::pack(F1.z);
   v[3 * XT] = P::pack(F2.x); v[4 * XT] = P::pack(F2.y); v[5 * XT] = P::pack(F2.z);
@@ -113,61 +131,83 @@ x_pairs(TileArgs A, typename P::Consts KP, const uint8_t* __restrict__ flags, co
   v[9 * XT] = P::pack(F4.x); v[10 * XT] = P::pack(F4.y); v[11 * XT] = P::pack(F4.z);
 }
 
+// All sixteen values are there (loaded) before anything after this point; without
+// it the compiler loads each next to its use, one memory latency after another.
+__device__ __forceinline__ void all_loaded(double* x) {
+  asm volatile(""
+               : "+d"(x[0]), "+d"(x[1]), "+d"(x[2]), "+d"(x[3]), "+d"(x[4]), "+d"(x[5]), "+d"(x[6]), "+d"(x[7]),
+                 "+d"(x[8]), "+d"(x[9]), "+d"(x[10]), "+d"(x[11]), "+d"(x[12]), "+d"(x[13]), "+d"(x[14]),
+                 "+d"(x[15]));
+}
+
 // The slot of tile pair blockIdx.x / 12, component blockIdx.x % 12, from the
 // stored pairs, in the tile kernel's order: a row segment's general pairs by
 // step, then its near-parallel ones by step; a column segment's general pairs
 // warp of rows by warp, by step within one, its near-parallel ones by row
-// within one.  Unconditional loads (a position without a pair holds anything
-// and is not added) keep the loop's loads in flight.
+// within one.  The loads of a batch of steps are in flight together and do not
+// wait for the classes (a position without a pair holds anything and is not
+// added): 30 us at one tile pair became 10.  Only the first `live` rows and
+// columns can hold pairs when there is one tile.
 template <class P>
 __global__ void __launch_bounds__(XT)
-x_fold(const double* __restrict__ vals, const uint8_t* __restrict__ flags, double* __restrict__ partial) {
+x_fold(const double* __restrict__ vals, const uint8_t* __restrict__ flags, int live, double* __restrict__ partial) {
   using Comp = typename P::Comp;
+  constexpr int NB = 16;
   const int64_t b = blockIdx.x / 12;
   const int c = blockIdx.x % 12, t = threadIdx.x;
   const double* v = vals + (b * XT * 12 + c) * XT;
   const uint8_t* f = flags + b * XPOS;
-  double r;
-  if (c < 6) {
+  double r = 0.0;
+  if (t >= live) {
+  } else if (c < 6) {
     Comp acc = P::comp_zero();
     double fp = 0.0;
-#pragma unroll 8
-    for (int k = 0; k < XT; ++k) {
-      const int cls = f[k * XT + t];
-      const double x = v[(int64_t)k * 12 * XT + t];
-      if (cls == 1) acc = acc + P::unpack(x);
-      if (cls == 2) fp = fp + x;
+    for (int k0 = 0; k0 < live; k0 += NB) {
+      double x[NB];
+      int cls[NB];
+#pragma unroll
+      for (int q = 0; q < NB; ++q) {
+        x[q] = v[(int64_t)(k0 + q) * 12 * XT + t];
+        cls[q] = f[(k0 + q) * XT + t];
+      }
+      all_loaded(x);
+#pragma unroll
+      for (int q = 0; q < NB; ++q) {
+        if (cls[q] == 1) acc = acc + P::unpack(x[q]);
+        if (cls[q] == 2) fp = fp + x[q];
+      }
     }
     r = P::comp_to_double(acc) + fp;
   } else {
-    Comp s[XT / 32];
-    double tot = 0.0;
-#pragma unroll
-    for (int w = 0; w < XT / 32; ++w) s[w] = P::comp_zero();
-#pragma unroll 4
-    for (int q = 0; q < 32; ++q) {
-#pragma unroll
-      for (int w = 0; w < XT / 32; ++w) {
-        // Rows of warp w in the order of the steps that pair them with column t.
-        const int row = 32 * w + (((t >> 5) == w ? (t & 31) + 32 - q : 31 - q) & 31);
-        const int k = (t - row) & (XT - 1);
-        const double x = v[(int64_t)k * 12 * XT + row];
-        if (f[k * XT + row] == 1) s[w] = s[w] + P::unpack(x);
-      }
-    }
-#pragma unroll
-    for (int w = 0; w < XT / 32; ++w) {
+    double col = 0.0, tot = 0.0;
+    for (int w = 0; 32 * w < live; ++w) {
+      Comp s = P::comp_zero();
       double fp = 0.0;
-#pragma unroll 8
-      for (int q = 0; q < 32; ++q) {
-        const int row = 32 * w + q, k = (t - row) & (XT - 1);
-        if (f[k * XT + row] == 2) fp = fp + v[(int64_t)k * 12 * XT + row];
+      for (int q0 = 0; q0 < 32; q0 += NB) {
+        double x[NB], y[NB];
+        int cx[NB], cy[NB];
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+          // Rows of warp w in the order of the steps that pair them with column t; by row.
+          const int rx = 32 * w + (((t >> 5) == w ? (t & 31) + 32 - q0 - q : 31 - q0 - q) & 31);
+          const int ry = 32 * w + q0 + q;
+          const int kx = (t - rx) & (XT - 1), ky = (t - ry) & (XT - 1);
+          x[q] = v[(int64_t)kx * 12 * XT + rx];
+          cx[q] = f[kx * XT + rx];
+          y[q] = v[(int64_t)ky * 12 * XT + ry];
+          cy[q] = f[ky * XT + ry];
+        }
+        all_loaded(x);
+        all_loaded(y);
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+          if (cx[q] == 1) s = s + P::unpack(x[q]);
+          if (cy[q] == 2) fp = fp + y[q];
+        }
       }
+      col = w == 0 ? P::comp_to_double(s) : col + P::comp_to_double(s);
       tot = tot + fp;
     }
-    double col = P::comp_to_double(s[0]);
-#pragma unroll
-    for (int w = 1; w < XT / 32; ++w) col += P::comp_to_double(s[w]);
     r = col + tot;
   }
   partial[(b * 12 + c) * XT + t] = r;
@@ -194,16 +234,23 @@ struct XScratch {
 
 // Classes, pairs and the slots of every tile pair (what the tile kernel writes).
 template <class P>
-cudaError_t launch_expanded(const TileArgs& A, const typename P::Consts& KP, int64_t nb, void* scratch,
-                            double* partial, unsigned long long* counters, cudaStream_t st) {
+cudaError_t launch_expanded(const TileArgs& A, const typename P::Consts& KP, int64_t nb, int64_t numSeg,
+                            void* scratch, double* partial, unsigned long long* counters, cudaStream_t st) {
+  const int live = nb == 1 ? (int)numSeg : XT;
   const XScratch x(scratch, nb);
   cudaError_t e = cudaMemsetAsync(x.count, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
   x_classify<<<(unsigned)(nb * XPOS / 256), 256, 0, st>>>(A.soa, A.skip, A.npad, x.flags, x.list, x.count, counters);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  x_pairs<P><<<(unsigned)(kParCtas + nb * XT * 4), 32, 0, st>>>(A, KP, x.flags, x.list, x.count, x.vals, counters);
+  if constexpr (P::kQuad) {
+    if (numSeg <= kQuadSegs)
+      x_pairs<P, true><<<kParCtas + XT * 16, 32, 0, st>>>(A, KP, x.flags, x.list, x.count, x.vals, counters);
+  }
+  if (!P::kQuad || numSeg > kQuadSegs)
+    x_pairs<P, false><<<(unsigned)(kParCtas + nb * XT * 4), 32, 0, st>>>(A, KP, x.flags, x.list, x.count, x.vals,
+                                                                         counters);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  x_fold<P><<<(unsigned)(nb * 12), XT, 0, st>>>(x.vals, x.flags, partial);
+  x_fold<P><<<(unsigned)(nb * 12), XT, 0, st>>>(x.vals, x.flags, live, partial);
   return cudaGetLastError();
 }
 
@@ -215,7 +262,8 @@ cudaError_t launch_expanded(const TileArgs& A, const typename P::Consts& KP, int
 // Near-parallel columns are listed in shared memory (column order) and evaluated
 // after the sweep: with ~5 % of the columns near-parallel, most CTAs have one
 // warp's worth of them, where a list per warp would make every warp run both
-// branches.  The threads' sums are added in a fixed tree; x_reduce_rows adds a
+// branches.  (37 rows x 6,001 segments: 570 us; one-warp CTAs of 128 columns, each
+// with its list, 654.)  The threads' sums are added in a fixed tree; x_reduce_rows adds a
 // row's blocks in a fixed order.
 constexpr int kRowThreads = 128;
 
@@ -268,9 +316,8 @@ x_rows(TileArgs A, typename P::Consts KP, const int64_t* __restrict__ rows, int6
       const SegF64 b = tb_load_seg64(A.soa, A.npad, gi);
       for (int e = tid; e < nPar; e += kRowThreads) {
         const SegF64 s = tb_load_seg64(A.soa, A.npad, j0 + list[e]);
-        D3 F1, F2, F3, F4;
-        nCore += parallel_pair<false>(A.K, b.b, b.n1, b.n2, b.t, b.tN, s.b, s.n1, s.n2, s.t, s.tN, dot(b.t, s.t), F1,
-                                      F2, F3, F4);
+        D3 F1, F2;
+        nCore += parallel_pair_side<1>(A.K, b, s, F1, F2);
         p1 = p1 + F1;
         p2 = p2 + F2;
       }

@@ -369,10 +369,12 @@ struct PolF64 {
     c = dot(a.t, b.t);
     return 1.0 - c * c > kSqrtEps;
   }
-  template <bool BOTH>
+  // QUAD: four lanes per pair (pair_f64.cuh), for the policies that have it.
+  static constexpr bool kQuad = true;
+  template <bool BOTH, bool QUAD = false>
   static __device__ __forceinline__ void general(const Consts&, const TileArgs& A, const Seg& a, const Seg& b, double c,
                                                  D3& F1, D3& F2, D3& F3, D3& F4) {
-    general_pair<true, BOTH>(A.K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, c, F1, F2, F3, F4);
+    general_pair<true, BOTH, QUAD>(A.K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, c, F1, F2, F3, F4);
   }
   // Dense pass of the classified modes: one general-branch pair, both sides.
   static __device__ __forceinline__ void dense_general(const Consts& KP, const TileArgs& A, int64_t gi, int64_t gj,

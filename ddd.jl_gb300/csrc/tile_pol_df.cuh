@@ -129,6 +129,7 @@ struct PolDF {
     add_df(s.fj[warp][4][j], F4.y);
     add_df(s.fj[warp][5][j], F4.z);
   }
+  static constexpr bool kQuad = false;
   // One component as segseg_small.cuh stores (hi, lo in 8 bytes) and adds it.
   using Comp = df64;
   static __device__ __forceinline__ double pack(df64 v) {

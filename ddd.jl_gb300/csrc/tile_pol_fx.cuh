@@ -16,12 +16,12 @@ __device__ __forceinline__ fx::X3 fx_x3(const D3& v) { return {v.x, v.y, v.z}; }
 __device__ __forceinline__ D3 fx_d3(const fx::X3& v) { return {v.x, v.y, v.z}; }
 
 struct PolF64Fast : PolF64 {
-  template <bool BOTH>
+  template <bool BOTH, bool QUAD = false>
   static __device__ __forceinline__ void general(const Consts&, const TileArgs& A, const Seg& a, const Seg& b,
                                                  double c, D3& F1, D3& F2, D3& F3, D3& F4) {
     const fx::KFast K{A.K.aSq, A.K.mu4pi, A.K.mu8pi, A.K.mu4pinu, A.K.mu8piaSq, A.K.mu4pinuaSq};
     fx::X3 G1, G2, G3, G4;
-    fx::general_pair<true, BOTH, fx::kMathInt>(K, fx_x3(a.b), fx_x3(a.n1), fx_x3(a.n2), fx_x3(a.t), a.tN, fx_x3(b.b),
+    fx::general_pair<true, BOTH, fx::kMathInt, QUAD>(K, fx_x3(a.b), fx_x3(a.n1), fx_x3(a.n2), fx_x3(a.t), a.tN, fx_x3(b.b),
                                        fx_x3(b.n1), fx_x3(b.n2), fx_x3(b.t), b.tN, c, G1, G2, G3, G4);
     F1 = fx_d3(G1);
     F2 = fx_d3(G2);
