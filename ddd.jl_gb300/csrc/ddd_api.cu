@@ -32,9 +32,15 @@ struct ddd_ctx {
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   std::mutex mu;
   std::string err;
-  DevBuf coord, bvec, segidx, ext, soa, soadf, skip, partial, expand, out, rows, x0, sigma, counters, probe, errflag;
-  DevBuf links, conn, segforce;  // mobility inputs
-  DevBuf vel, label, skippairs;  // collision inputs
+  DevBuf net, coord, bvec, soa, soadf, skip, partial, expand, out, rows, x0, sigma, counters, probe, errflag;
+  DevBuf links;                  // calc_uTilde inputs, with coord and bvec
+  DevBuf mobin, collin;          // packed mobility and collision inputs
+  // The packed network's parts (net).
+  const double *dCoord = nullptr, *dBvec = nullptr;
+  const int64_t* dSeg = nullptr;
+  const uint8_t* dExt = nullptr;
+  char* pin = nullptr;  // pinned staging of small copies (PinArena)
+  size_t pinUsed = 0;
   ddd::CollisionPlan* coll = nullptr;
   DevBuf upoints;  // calc_uTilde evaluation points
   ddd::UTildeScratch* ut = nullptr;
@@ -242,6 +248,72 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
+// Small copies of the host-array calls go through pinned memory, an input's arrays
+// packed into one copy: a 24-segment call made five pageable copies and one fill
+// of 2-5 us each around 100 us of kernels, and makes two copies.  The arena is
+// handed out front to back and starts again once the stream is idle (every call
+// ends that way; a call that failed half-way leaves its part until then).  Measured:
+// host call at 24 segments 132 -> 115 us, a 512-segment step (seg-seg, self and PK
+// force, mobility, collision) 985 -> 919 us; above 512 KB the arrays are large enough
+// for copies of their own.
+constexpr size_t kPinBytes = (size_t)2 << 20, kPinMost = (size_t)1 << 19;
+char* pin_take(ddd_ctx* ctx, size_t bytes) {
+  bytes = (bytes + 63) & ~(size_t)63;
+  if (bytes > kPinMost) return nullptr;
+  if (!ctx->pin && cudaHostAlloc((void**)&ctx->pin, kPinBytes, cudaHostAllocDefault) != cudaSuccess) {
+    ctx->pin = nullptr;
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (ctx->pinUsed + bytes > kPinBytes) {
+    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return nullptr;
+    ctx->pinUsed = 0;
+  }
+  char* p = ctx->pin + ctx->pinUsed;
+  ctx->pinUsed += bytes;
+  return p;
+}
+
+// Arrays bound for one device buffer, each at a multiple of 64 bytes.
+struct Upload {
+  static constexpr int kMost = 8;
+  const void* src[kMost];
+  size_t bytes[kMost], off[kMost], total = 0;
+  int n = 0;
+  size_t add(const void* p, size_t b) {
+    src[n] = p;
+    bytes[n] = b;
+    off[n] = total;
+    total += (b + 63) & ~(size_t)63;
+    return off[n++];
+  }
+};
+int send(ddd_ctx* ctx, DevBuf& dst, const Upload& u, const char* what) {
+  CK(dst.ensure(u.total), what);
+  char* d = dst.as<char>();
+  if (char* h = pin_take(ctx, u.total)) {
+    for (int k = 0; k < u.n; ++k)
+      if (u.bytes[k]) memcpy(h + u.off[k], u.src[k], u.bytes[k]);
+    CK(cudaMemcpyAsync(d, h, u.total, cudaMemcpyHostToDevice, ctx->stream), what);
+    return DDD_OK;
+  }
+  for (int k = 0; k < u.n; ++k)
+    if (u.bytes[k])
+      CK(cudaMemcpyAsync(d + u.off[k], u.src[k], u.bytes[k], cudaMemcpyHostToDevice, ctx->stream), what);
+  return DDD_OK;
+}
+// Reads `bytes` from the device into `host` and waits for the stream; `after`, if
+// given, is recorded behind the copy.
+int fetch(ddd_ctx* ctx, void* host, const void* dev, size_t bytes, cudaEvent_t after, const char* what) {
+  char* h = pin_take(ctx, bytes);
+  CK(cudaMemcpyAsync(h ? h : host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream), what);
+  if (after) CK(cudaEventRecord(after, ctx->stream), "event");
+  CK(cudaStreamSynchronize(ctx->stream), what);
+  ctx->pinUsed = 0;
+  if (h) memcpy(host, h, bytes);
+  return DDD_OK;
+}
+
 // Uploads the network and builds the packed SoA; returns npad.
 int upload_network(ddd_ctx* ctx, const double* coord, int64_t coordCols, const double* bVec, int64_t bVecCols,
                    const int64_t* segIdx, int64_t ld, const uint8_t* extSeg, int64_t numSeg, int64_t& npad,
@@ -249,20 +321,20 @@ int upload_network(ddd_ctx* ctx, const double* coord, int64_t coordCols, const d
   npad = ddd::strict::segseg_npad(numSeg);
   const size_t cB = (size_t)coordCols * 3 * sizeof(double), bB = (size_t)bVecCols * 3 * sizeof(double);
   const size_t sB = (size_t)ld * 3 * sizeof(int64_t), eB = extSeg ? (size_t)numSeg : 0;
-  CK(ctx->coord.ensure(cB), "alloc coord");
-  CK(ctx->bvec.ensure(bB), "alloc bVec");
-  CK(ctx->segidx.ensure(sB), "alloc segIdx");
-  if (eB) CK(ctx->ext.ensure(eB), "alloc extSeg");
   CK(ctx->soa.ensure(ddd::strict::segseg_soa_bytes(npad)), "alloc segment SoA");
   CK(ctx->skip.ensure((size_t)npad), "alloc skip flags");
-  CK(cudaMemcpyAsync(ctx->coord.p, coord, cB, cudaMemcpyHostToDevice, ctx->stream), "copy coord");
-  CK(cudaMemcpyAsync(ctx->bvec.p, bVec, bB, cudaMemcpyHostToDevice, ctx->stream), "copy bVec");
-  CK(cudaMemcpyAsync(ctx->segidx.p, segIdx, sB, cudaMemcpyHostToDevice, ctx->stream), "copy segIdx");
-  if (eB) CK(cudaMemcpyAsync(ctx->ext.p, extSeg, eB, cudaMemcpyHostToDevice, ctx->stream), "copy extSeg");
+  Upload u;
+  const size_t oC = u.add(coord, cB), oB = u.add(bVec, bB), oS = u.add(segIdx, sB), oE = u.add(extSeg, eB);
+  const int rc = send(ctx, ctx->net, u, "copy network");
+  if (rc) return rc;
+  const char* d = ctx->net.as<char>();
+  ctx->dCoord = (const double*)(d + oC);
+  ctx->dBvec = (const double*)(d + oB);
+  ctx->dSeg = (const int64_t*)(d + oS);
+  ctx->dExt = eB ? (const uint8_t*)(d + oE) : nullptr;
   h2d += (int64_t)(cB + bB + sB + eB);
-  CK(ddd::strict::launch_prep_segments(ctx->coord.as<double>(), ctx->bvec.as<double>(), ctx->segidx.as<int64_t>(), ld,
-                               eB ? ctx->ext.as<uint8_t>() : nullptr, numSeg, npad, ctx->soa.as<double>(),
-                               ctx->skip.as<uint8_t>(), ctx->stream),
+  CK(ddd::strict::launch_prep_segments(ctx->dCoord, ctx->dBvec, ctx->dSeg, ld, ctx->dExt, numSeg, npad,
+                                       ctx->soa.as<double>(), ctx->skip.as<uint8_t>(), ctx->stream),
      "prep_segments");
   return DDD_OK;
 }
@@ -289,7 +361,7 @@ int segseg_compute(ddd_ctx* ctx, const ddd_consts* k, const double* coord, int64
       }
   }
   const int64_t nOut = rowsMode ? nIdx : numSeg;
-  ctx->hostTmp.assign((size_t)nOut * 6, 0.0);
+  ctx->hostTmp.assign((size_t)nOut * 6 + 3, 0.0);  // the forces, then the kernels' three counters
   if (rep) memset(rep, 0, sizeof *rep);
   if (nOut == 0 || numSeg == 0) return DDD_OK;
 
@@ -298,39 +370,35 @@ int segseg_compute(ddd_ctx* ctx, const ddd_consts* k, const double* coord, int64
   CK(cudaEventRecord(ctx->ev[0], ctx->stream), "event");
   rc = upload_network(ctx, coord, coordCols, bVec, bVecCols, segIdx, ld, extSeg, numSeg, npad, h2d);
   if (rc) return rc;
-  CK(ctx->counters.ensure(3 * sizeof(unsigned long long)), "alloc counters");
-  CK(cudaMemsetAsync(ctx->counters.p, 0, 3 * sizeof(unsigned long long), ctx->stream), "memset counters");
-  CK(ctx->out.ensure((size_t)nOut * 6 * sizeof(double)), "alloc output");
+  const size_t outBytes = (size_t)nOut * 6 * sizeof(double), cntBytes = 3 * sizeof(unsigned long long);
+  CK(ctx->out.ensure(outBytes + cntBytes), "alloc output");
+  unsigned long long* dCnt = (unsigned long long*)(ctx->out.as<char>() + outBytes);
+  CK(cudaMemsetAsync(dCnt, 0, cntBytes, ctx->stream), "memset counters");
   if (!rowsMode) {
     CK(ctx->partial.ensure(partial_bytes(ctx, npad)), "alloc partial sums");
     CK(cudaEventRecord(ctx->ev[1], ctx->stream), "event");
     CK(run_segseg_all(ctx, K, ctx->soa.as<double>(), ctx->skip.as<uint8_t>(), npad, ctx->partial.as<double>(),
-                                  ctx->out.as<double>(), numSeg, ctx->counters.as<unsigned long long>(), ctx->stream),
+                      ctx->out.as<double>(), numSeg, dCnt, ctx->stream),
        "segseg_all_f64");
   } else {
     std::vector<int64_t> rows0((size_t)nIdx);
     for (int64_t q = 0; q < nIdx; ++q) rows0[q] = idx[q] - 1;
-    CK(ctx->rows.ensure((size_t)nIdx * sizeof(int64_t)), "alloc rows");
-    CK(cudaMemcpyAsync(ctx->rows.p, rows0.data(), (size_t)nIdx * sizeof(int64_t), cudaMemcpyHostToDevice,
-                       ctx->stream),
-       "copy idx");
+    Upload u;
+    u.add(rows0.data(), (size_t)nIdx * sizeof(int64_t));
+    if ((rc = send(ctx, ctx->rows, u, "copy idx"))) return rc;
     h2d += nIdx * (int64_t)sizeof(int64_t);
     const ddd::RowPlan plan = ddd::row_plan(npad, nIdx);
     CK(ctx->partial.ensure(ddd::row_partial_bytes(plan, rows_per_chunk(ctx, plan, nIdx))), "alloc partial sums");
     CK(cudaEventRecord(ctx->ev[1], ctx->stream), "event");
     CK(run_segseg_rows(ctx, K, ctx->soa.as<double>(), ctx->skip.as<uint8_t>(), npad, ctx->rows.as<int64_t>(),
-                       nIdx, plan, ctx->partial.as<double>(), ctx->out.as<double>(),
-                       ctx->counters.as<unsigned long long>(), ctx->stream),
+                       nIdx, plan, ctx->partial.as<double>(), ctx->out.as<double>(), dCnt, ctx->stream),
        "segseg_rows_f64");
   }
   CK(cudaEventRecord(ctx->ev[2], ctx->stream), "event");
-  unsigned long long cnt[3] = {0, 0, 0};
-  CK(cudaMemcpyAsync(ctx->hostTmp.data(), ctx->out.p, (size_t)nOut * 6 * sizeof(double), cudaMemcpyDeviceToHost,
-                     ctx->stream),
-     "copy forces");
-  CK(cudaMemcpyAsync(cnt, ctx->counters.p, sizeof cnt, cudaMemcpyDeviceToHost, ctx->stream), "copy counters");
-  CK(cudaEventRecord(ctx->ev[3], ctx->stream), "event");
-  CK(cudaStreamSynchronize(ctx->stream), "segseg_force");
+  rc = fetch(ctx, ctx->hostTmp.data(), ctx->out.p, outBytes + cntBytes, ctx->ev[3], "segseg_force");
+  if (rc) return rc;
+  unsigned long long cnt[3];
+  memcpy(cnt, ctx->hostTmp.data() + 6 * nOut, sizeof cnt);
   if (rep) {
     rep->pairs_general = (int64_t)cnt[0];
     rep->pairs_parallel = (int64_t)cnt[1];
@@ -376,11 +444,12 @@ void ddd_destroy(ddd_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  for (DevBuf* b : {&c->links, &c->conn, &c->segforce, &c->vel, &c->label, &c->skippairs}) b->release();
+  for (DevBuf* b : {&c->links, &c->mobin, &c->collin}) b->release();
+  if (c->pin) cudaFreeHost(c->pin);
   if (c->coll) ddd::collision_plan_destroy(c->coll);
   delete c->ut;
   c->upoints.release();
-  for (DevBuf* b : {&c->coord, &c->bvec, &c->segidx, &c->ext, &c->soa, &c->soadf, &c->skip, &c->partial, &c->expand, &c->out, &c->rows,
+  for (DevBuf* b : {&c->net, &c->coord, &c->bvec, &c->soa, &c->soadf, &c->skip, &c->partial, &c->expand, &c->out, &c->rows,
                     &c->x0, &c->sigma, &c->counters, &c->probe, &c->errflag})
     b->release();
   for (auto& ev : c->ev)
@@ -484,24 +553,24 @@ int self_pk_compute(ddd_ctx* ctx, const ddd_consts* k, const ddd_self_params* sp
        "copy idx");
   }
   if (sigmaHat) {
-    CK(ctx->sigma.ensure((size_t)n * 6 * sizeof(double)), "alloc sigmaHat");
-    CK(cudaMemcpyAsync(ctx->sigma.p, sigmaHat, (size_t)n * 6 * sizeof(double), cudaMemcpyHostToDevice, ctx->stream),
-       "copy sigmaHat");
+    Upload u;
+    u.add(sigmaHat, (size_t)n * 6 * sizeof(double));
+    if ((rc = send(ctx, ctx->sigma, u, "copy sigmaHat"))) return rc;
   }
   CK(ctx->out.ensure((size_t)n * 6 * sizeof(double)), "alloc output");
   double* dS = ctx->out.as<double>();
   CK(cudaEventRecord(ctx->ev[1], ctx->stream), "event");
-  CK(ddd::launch_self_pk(SK, ctx->coord.as<double>(), ctx->bvec.as<double>(), ctx->segidx.as<int64_t>(), ld,
-                         extSeg ? ctx->ext.as<uint8_t>() : nullptr, numSeg, idx ? ctx->rows.as<int64_t>() : nullptr,
-                         n, sigmaHat ? ctx->sigma.as<double>() : nullptr, dS, sigmaHat ? dS + 3 * n : nullptr,
+  CK(ddd::launch_self_pk(SK, ctx->dCoord, ctx->dBvec, ctx->dSeg, ld, ctx->dExt, numSeg,
+                         idx ? ctx->rows.as<int64_t>() : nullptr, n,
+                         sigmaHat ? ctx->sigma.as<double>() : nullptr, dS, sigmaHat ? dS + 3 * n : nullptr,
                          ctx->stream),
      "self_pk_f64");
   CK(cudaEventRecord(ctx->ev[2], ctx->stream), "event");
-  CK(cudaMemcpyAsync(S.data(), dS, (size_t)n * 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream), "copy S");
-  if (sigmaHat)
-    CK(cudaMemcpyAsync(PK.data(), dS + 3 * n, (size_t)n * 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream),
-       "copy PK");
-  CK(cudaStreamSynchronize(ctx->stream), "self force");
+  S.resize((size_t)n * (sigmaHat ? 6 : 3));  // S, then PK, as they lie on the device
+  rc = fetch(ctx, S.data(), dS, S.size() * sizeof(double), nullptr, "self force");
+  if (rc) return rc;
+  if (sigmaHat) std::copy(S.begin() + 3 * n, S.end(), PK.begin());
+  S.resize((size_t)n * 3);
   ctx->lastKernelMs = elapsed(ctx->ev[1], ctx->ev[2]);
   return DDD_OK;
 }
@@ -688,17 +757,12 @@ int mobility_compute(ddd_ctx* ctx, const ddd_mob_params* mp, const double* coord
   cudaStream_t st = ctx->stream;
   const size_t cB = (size_t)coordCols * 3 * 8, bB = (size_t)linkCols * 3 * 8, lB = (size_t)linkCols * 2 * 8;
   const size_t nB = (size_t)ldConn * numNode * 8, fB = (size_t)linkCols * 6 * 8;
-  CK(ctx->coord.ensure(cB), "alloc coord");
-  CK(ctx->bvec.ensure(bB), "alloc bVec");
-  CK(ctx->links.ensure(lB), "alloc links");
-  CK(ctx->conn.ensure(nB), "alloc connectivity");
-  CK(ctx->segforce.ensure(fB), "alloc segForce");
   CK(ctx->out.ensure((size_t)n * 6 * sizeof(double)), "alloc output");
-  CK(cudaMemcpyAsync(ctx->coord.p, coord, cB, cudaMemcpyHostToDevice, st), "copy coord");
-  CK(cudaMemcpyAsync(ctx->bvec.p, bVec, bB, cudaMemcpyHostToDevice, st), "copy bVec");
-  CK(cudaMemcpyAsync(ctx->links.p, links, lB, cudaMemcpyHostToDevice, st), "copy links");
-  CK(cudaMemcpyAsync(ctx->conn.p, connectivity, nB, cudaMemcpyHostToDevice, st), "copy connectivity");
-  CK(cudaMemcpyAsync(ctx->segforce.p, segForce, fB, cudaMemcpyHostToDevice, st), "copy segForce");
+  Upload u;
+  const size_t oC = u.add(coord, cB), oB = u.add(bVec, bB), oL = u.add(links, lB), oN = u.add(connectivity, nB),
+               oF = u.add(segForce, fB);
+  if (const int rc = send(ctx, ctx->mobin, u, "copy mobility inputs")) return rc;
+  const char* d = ctx->mobin.as<char>();
   if (idx) {
     std::vector<int64_t> rows0((size_t)n);
     for (int64_t q = 0; q < n; ++q) rows0[q] = idx[q] - 1;
@@ -708,14 +772,13 @@ int mobility_compute(ddd_ctx* ctx, const ddd_mob_params* mp, const double* coord
   }
   double* dOut = ctx->out.as<double>();
   CK(cudaEventRecord(ctx->ev[1], st), "event");
-  CK(ddd::launch_mobility_bcc(P, ctx->coord.as<double>(), ctx->bvec.as<double>(), ctx->links.as<int64_t>(),
-                              ctx->conn.as<int64_t>(), ldConn, ctx->segforce.as<double>(),
+  CK(ddd::launch_mobility_bcc(P, (const double*)(d + oC), (const double*)(d + oB), (const int64_t*)(d + oL),
+                              (const int64_t*)(d + oN), ldConn, (const double*)(d + oF),
                               idx ? ctx->rows.as<int64_t>() : nullptr, n, dOut, dOut + 3 * n, st),
      "mobility_bcc_f64");
   CK(cudaEventRecord(ctx->ev[2], st), "event");
-  CK(cudaMemcpyAsync(ctx->hostTmp.data(), dOut, (size_t)n * 6 * sizeof(double), cudaMemcpyDeviceToHost, st),
-     "copy node forces and velocities");
-  CK(cudaStreamSynchronize(st), "mobility");
+  if (const int rc = fetch(ctx, ctx->hostTmp.data(), dOut, (size_t)n * 6 * sizeof(double), nullptr, "mobility"))
+    return rc;
   ctx->lastKernelMs = elapsed(ctx->ev[1], ctx->ev[2]);
   return DDD_OK;
 }
@@ -832,18 +895,18 @@ int ddd_sigma_tilde(ddd_ctx* ctx, const ddd_consts* k, const double* x0, int64_t
   rc = upload_network(ctx, coord, coordCols, bVec, bVecCols, sel.data(), nSel, nullptr, nSel, npad, h2d);
   if (rc) return rc;
   const size_t xB = (size_t)numPoints * 3 * sizeof(double), sB = (size_t)numPoints * 6 * sizeof(double);
-  CK(ctx->x0.ensure(xB), "alloc points");
   CK(ctx->sigma.ensure(sB), "alloc sigma");
-  CK(cudaMemcpyAsync(ctx->x0.p, x0, xB, cudaMemcpyHostToDevice, ctx->stream), "copy points");
+  Upload u;
+  u.add(x0, xB);
+  if ((rc = send(ctx, ctx->x0, u, "copy points"))) return rc;
   h2d += (int64_t)xB;
   CK(cudaEventRecord(ctx->ev[1], ctx->stream), "event");
   CK(run_sigma(ctx, K, ctx->soa.as<double>(), npad, nSel, ctx->x0.as<double>(), numPoints,
                            ctx->sigma.as<double>(), ctx->stream),
      "sigma_tilde_f64");
   CK(cudaEventRecord(ctx->ev[2], ctx->stream), "event");
-  CK(cudaMemcpyAsync(sigma, ctx->sigma.p, sB, cudaMemcpyDeviceToHost, ctx->stream), "copy sigma");
-  CK(cudaEventRecord(ctx->ev[3], ctx->stream), "event");
-  CK(cudaStreamSynchronize(ctx->stream), "sigma_tilde");
+  rc = fetch(ctx, sigma, ctx->sigma.p, sB, ctx->ev[3], "sigma_tilde");
+  if (rc) return rc;
   if (rep) {
     rep->kernel_ms = elapsed(ctx->ev[1], ctx->ev[2]);
     rep->total_ms = elapsed(ctx->ev[0], ctx->ev[3]);
@@ -1134,26 +1197,19 @@ int ddd_detect_collision(ddd_ctx* ctx, double collisionDistSq, const double* coo
   cudaStream_t st = ctx->stream;
   const size_t cB = (size_t)numNode * 3 * 8, lB = (size_t)linkCols * 2 * 8, bB = (size_t)std::max<int64_t>(numSeg, 1) * 3 * 8;
   const size_t nB = (size_t)ldConn * numNode * 8, kB = skFlat.size() * 8;
-  CK(ctx->coord.ensure(cB), "alloc coord");
-  CK(ctx->vel.ensure(cB), "alloc nodeVel");
-  CK(ctx->label.ensure((size_t)numNode * 4), "alloc label");
-  CK(ctx->links.ensure(lB), "alloc links");
-  CK(ctx->bvec.ensure(bB), "alloc bVec");
-  CK(ctx->conn.ensure(nB), "alloc connectivity");
-  CK(ctx->skippairs.ensure(kB), "alloc skipSegs");
-  CK(cudaMemcpyAsync(ctx->coord.p, coord, cB, cudaMemcpyHostToDevice, st), "copy coord");
-  CK(cudaMemcpyAsync(ctx->vel.p, nodeVel, cB, cudaMemcpyHostToDevice, st), "copy nodeVel");
-  CK(cudaMemcpyAsync(ctx->label.p, label, (size_t)numNode * 4, cudaMemcpyHostToDevice, st), "copy label");
-  CK(cudaMemcpyAsync(ctx->links.p, links, lB, cudaMemcpyHostToDevice, st), "copy links");
-  if (numSeg > 0) CK(cudaMemcpyAsync(ctx->bvec.p, bVec, (size_t)numSeg * 3 * 8, cudaMemcpyHostToDevice, st), "copy bVec");
-  CK(cudaMemcpyAsync(ctx->conn.p, connectivity, nB, cudaMemcpyHostToDevice, st), "copy connectivity");
-  CK(cudaMemcpyAsync(ctx->skippairs.p, skFlat.data(), kB, cudaMemcpyHostToDevice, st), "copy skipSegs");
+  Upload u;
+  const size_t oC = u.add(coord, cB), oV = u.add(nodeVel, cB), oA = u.add(label, (size_t)numNode * 4),
+               oL = u.add(links, lB), oB = u.add(bVec, numSeg > 0 ? (size_t)numSeg * 3 * 8 : 0),
+               oN = u.add(connectivity, nB), oK = u.add(skFlat.data(), kB);
+  if (const int rc = send(ctx, ctx->collin, u, "copy collision inputs")) return rc;
+  const char* d = ctx->collin.as<char>();
   ddd::CollisionOut r{};
-  CK(ddd::collision_detect(ctx->coll, collisionDistSq, ctx->coord.as<double>(), ctx->vel.as<double>(),
-                           ctx->label.as<int32_t>(), ctx->links.as<int64_t>(), ctx->bvec.as<double>(),
-                           ctx->conn.as<int64_t>(), ldConn, numNode, numSeg, ctx->skippairs.as<int64_t>(),
+  CK(ddd::collision_detect(ctx->coll, collisionDistSq, (const double*)(d + oC), (const double*)(d + oV),
+                           (const int32_t*)(d + oA), (const int64_t*)(d + oL), (const double*)(d + oB),
+                           (const int64_t*)(d + oN), ldConn, numNode, numSeg, (const int64_t*)(d + oK),
                            (int64_t)sk.size(), box, maxAbs, &r, ctx->ev[1], ctx->ev[2], st),
      "detect_collision");
+  ctx->pinUsed = 0;  // collision_detect has waited for the stream
   ctx->lastKernelMs = elapsed(ctx->ev[1], ctx->ev[2]);
   out->collision = r.collision;
   out->type = r.type;
