@@ -112,31 +112,34 @@ cudaError_t run_segseg_all(ddd_ctx* c, const ddd::KConsts& K, const double* soa,
     cudaError_t e = prep_df_if_needed(c, npad, st);
     if (e != cudaSuccess) return e;
   }
-  // Small networks: one warp per 32 pairs, the pair values stored and folded.
-  // The store obeys the partial-sum limit too; without it (limit, no memory) the
-  // tile kernel gives the same bits.
+  // Small networks, and the tile pairs beyond the last full wave of the tile
+  // kernel: one warp per 32 pairs, the pair values stored and folded.  The store
+  // obeys the partial-sum limit too; without it (limit, no memory) the tile kernel
+  // takes all, with the same bits.
   const int64_t nt = npad / ddd::strict::segseg_npad(1), nb = nt * (nt + 1) / 2;
-  if (nb <= ddd::kExpandMaxPairs && cap >= nb && (int64_t)ddd::expand_bytes(nb) <= partial_limit(c)) {
-    const cudaError_t e = c->expand.ensure(ddd::expand_bytes(nb));
+  const ddd::ExpandRule& rule = use_df(c)    ? (df_form(c) ? ddd::kExpandMixed : ddd::kExpandDF)
+                                : use_fx(c)  ? ddd::kExpandFx
+                                : use_fma(c) ? ddd::kExpandFma
+                                             : ddd::kExpandF64;
+  int64_t from = ddd::expand_from(nb, rule);
+  void* x = nullptr;
+  if (cap >= nb && from < nb && (int64_t)ddd::expand_bytes(nb - from) <= partial_limit(c)) {
+    const cudaError_t e = c->expand.ensure(ddd::expand_bytes(nb - from));
     if (e == cudaSuccess) {
-      void* x = c->expand.p;
-      if (use_df(c))
-        return ddd::launch_segseg_small_df(K, soa, c->soadf.as<float>(), skip, npad, x, partial, out, numSeg, cnt, st,
-                                           df_form(c));
-      if (use_fx(c)) return ddd::launch_segseg_small_fx(K, soa, skip, npad, x, partial, out, numSeg, cnt, st);
-      return use_fma(c) ? ddd::fast::launch_segseg_small_f64(K, soa, skip, npad, x, partial, out, numSeg, cnt, st)
-                        : ddd::strict::launch_segseg_small_f64(K, soa, skip, npad, x, partial, out, numSeg, cnt, st);
+      x = c->expand.p;
+    } else {
+      if (e != cudaErrorMemoryAllocation) return e;
+      cudaGetLastError();
     }
-    if (e != cudaErrorMemoryAllocation) return e;
-    cudaGetLastError();
   }
-  if (use_df(c)) {
+  if (!x) from = nb;
+  if (use_df(c))
     return ddd::launch_segseg_all_df(K, soa, c->soadf.as<float>(), skip, npad, partial, out, numSeg, cnt, st,
-                                     df_form(c), cap);
-  }
-  if (use_fx(c)) return ddd::launch_segseg_all_fx(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap);
-  return use_fma(c) ? ddd::fast::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap)
-                    : ddd::strict::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap);
+                                     df_form(c), cap, from, x);
+  if (use_fx(c)) return ddd::launch_segseg_all_fx(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap, from, x);
+  return use_fma(c) ? ddd::fast::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap, from, x)
+                    : ddd::strict::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap, from,
+                                                         x);
 }
 
 // Index rows per launch: all of them when their partial sums (6 doubles per row

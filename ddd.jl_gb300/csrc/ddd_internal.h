@@ -57,12 +57,37 @@ inline RowPlan row_plan(int64_t npad, int64_t nRows) {
 }
 inline size_t row_partial_bytes(const RowPlan& p, int64_t nRows) { return (size_t)(nRows * p.nBlk) * 6 * sizeof(double); }
 
-// Expanded all-pairs of small networks (segseg_small.cuh): every pair's twelve
-// components, class and list entry stored, 128 x 128 positions per tile pair.
-// Up to 153 tile pairs (2,176 segments, 252 MB): beyond that the tile kernel has
-// two CTAs for most SMs and the store grows with the square of the size.
+// Expanded all-pairs (segseg_small.cuh): every pair's twelve components, class and
+// list entry stored, 128 x 128 positions per tile pair, at most 153 tile pairs at
+// a time (252 MB).  It takes networks of up to 153 tile pairs (2,176 segments)
+// whole, and of larger ones the tile pairs beyond the last full wave of the tile
+// kernel (304 CTAs), which that kernel would run on part of the GPU: `most`
+// less `perWave` for each full wave, while there are at most `waves`.  Beyond, the
+// CTAs' drift has filled the last wave, and the FP32-heavy forms pay for the
+// store.  Measured, with against without, tile pairs as waves * 304 + rest:
+//   strict   0+171 7.93 / 14.02 ms, 1+47 17.1 / 26.9, 2+212 39.6 / 42.6, 8+53 120.9 / 123.1
+//   fast     0+171 5.02 / 8.35, 1+47 10.3 / 15.9, 8+53 71.0 / 72.6; at 1+291 17.4 / 17.2
+//   df64     0+171 3.05 / 4.48, 1+224 8.93 / 9.40, 4+162 22.3 / 23.0; at 5+191 28.0 / 27.7
+//   FMA      none: the compiler contracts the two kernels differently (the others
+//            give the same bits), and at 300 tile pairs with a tenth of the pairs
+//            near-parallel that moved the forces by 2e-10
+//   f32c     0+171 1.72 / 2.34, 1+102 3.63 / 3.78; at 0+276 2.70 / 2.55, 1+224 4.89 / 4.64
 constexpr int64_t kExpandMaxPairs = 153;
-inline size_t expand_bytes(int64_t nb) { return (size_t)nb * 128 * 128 * (12 * sizeof(double) + 4 + 1) + 256; }
+constexpr int64_t kTileWave = 304;
+struct ExpandRule {
+  int waves, most, perWave;
+};
+constexpr ExpandRule kExpandF64 = {8, 304, 0}, kExpandFma = {-1, 0, 0}, kExpandFx = {8, 264, 0}, kExpandDF = {4, 240, 16},
+                     kExpandMixed = {1, 240, 128};
+// The first tile pair that goes to the expanded kernels.
+inline int64_t expand_from(int64_t nb, const ExpandRule& r) {
+  if (nb <= kExpandMaxPairs) return 0;
+  const int64_t w = nb / kTileWave, rest = nb % kTileWave;
+  return w <= r.waves && rest <= r.most - r.perWave * w ? nb - rest : nb;
+}
+inline size_t expand_bytes(int64_t nb) {
+  return (size_t)(nb < kExpandMaxPairs ? nb : kExpandMaxPairs) * 128 * 128 * (12 * sizeof(double) + 4 + 1) + 256;
+}
 
 // σ̃ with few points.  The literal FP64 kernels (strict, FMA) take sigma_split
 // (sigma_f64.cu) below kSigmaSplitPoints, where a thread per point leaves fewer
@@ -120,10 +145,8 @@ inline size_t sigma_part_bytes(const SigmaPlan& p, int64_t M) {
   int64_t segseg_band_end(int64_t J0, int64_t nt, int64_t capSlots); \
   cudaError_t launch_segseg_all_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad, \
                                     double* partial, double* out, int64_t numSeg, unsigned long long* counters, \
-                                    cudaStream_t st, int64_t capSlots); \
-  cudaError_t launch_segseg_small_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad, \
-                                      void* scratch, double* partial, double* out, int64_t numSeg, \
-                                      unsigned long long* counters, cudaStream_t st); \
+                                    cudaStream_t st, int64_t capSlots, int64_t expandFrom = INT64_MAX, \
+                                    void* expandScratch = nullptr); \
   cudaError_t launch_segseg_rows_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad, \
                                      const int64_t* rows, int64_t nRows, const RowPlan& plan, double* partial, \
                                      double* out, unsigned long long* counters, cudaStream_t st); \
@@ -148,10 +171,8 @@ size_t segseg_df_soa_bytes(int64_t npad);
 cudaError_t launch_prep_df(const double* soa, int64_t npad, float* soadf, cudaStream_t st);
 cudaError_t launch_segseg_all_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
                                  int64_t npad, double* partial, double* out, int64_t numSeg,
-                                 unsigned long long* counters, cudaStream_t st, int form, int64_t capSlots);
-cudaError_t launch_segseg_small_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
-                                   int64_t npad, void* scratch, double* partial, double* out, int64_t numSeg,
-                                   unsigned long long* counters, cudaStream_t st, int form);
+                                 unsigned long long* counters, cudaStream_t st, int form, int64_t capSlots,
+                                 int64_t expandFrom = INT64_MAX, void* expandScratch = nullptr);
 cudaError_t launch_segseg_rows_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
                                   int64_t npad, const int64_t* rows, int64_t nRows, const RowPlan& plan,
                                   double* partial, double* out, unsigned long long* counters, cudaStream_t st,
@@ -170,10 +191,8 @@ cudaError_t launch_sigma_fx(const KConsts& K, const double* soa, int64_t npad, i
 cudaError_t launch_sigma_slices(const double* part, int64_t M, int slices, double* sigma, cudaStream_t st);
 cudaError_t launch_segseg_all_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                                  double* partial, double* out, int64_t numSeg, unsigned long long* counters,
-                                 cudaStream_t st, int64_t capSlots);
-cudaError_t launch_segseg_small_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
-                                   void* scratch, double* partial, double* out, int64_t numSeg,
-                                   unsigned long long* counters, cudaStream_t st);
+                                 cudaStream_t st, int64_t capSlots, int64_t expandFrom = INT64_MAX,
+                                 void* expandScratch = nullptr);
 cudaError_t launch_segseg_rows_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                                   const int64_t* rows, int64_t nRows, const RowPlan& plan, double* partial,
                                   double* out, unsigned long long* counters, cudaStream_t st);

@@ -138,24 +138,35 @@ cudaError_t launch_prep_df(const double* soa, int64_t npad, float* soadf, cudaSt
 
 cudaError_t launch_segseg_all_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
                                  int64_t npad, double* partial, double* out, int64_t numSeg,
-                                 unsigned long long* counters, cudaStream_t st, int form, int64_t capSlots) {
+                                 unsigned long long* counters, cudaStream_t st, int form, int64_t capSlots,
+                                 int64_t expandFrom, void* expandScratch) {
   cudaError_t e = form ? set_attr_df<1>() : set_attr_df<0>();
   if (e != cudaSuccess) return e;
   const int64_t nt = npad / TILE;
   const int64_t nb = nt * (nt + 1) / 2;
   const TileArgs A{K, soa, skip, npad, soadf, nullptr};
+  const KConstsDF kd = kconsts_df(K);
+  const KConstsF kf = kconsts_f(K);
   // One launch over all slots, or (partial sums larger than capSlots slots)
   // bands of J columns in order, each reduced into the running output.
   for (int64_t J0 = 0; J0 < nt;) {
     const int64_t J1 = capSlots >= nb ? nt : strict::segseg_band_end(J0, nt, capSlots);
     const int64_t b0 = J0 * (J0 + 1) / 2, nbb = J1 * (J1 + 1) / 2 - b0;
-    if (form)
-      segseg_tile_df<1><<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolDF<1>>), st>>>(
-          A, PolDF<1>::Consts{kconsts_df(K), kconsts_f(K)}, b0, partial, counters);
-    else
-      segseg_tile_df<0><<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolDF<0>>), st>>>(
-          A, PolDF<0>::Consts{kconsts_df(K), kconsts_f(K)}, b0, partial, counters);
+    const int64_t nTile = capSlots >= nb && expandFrom < nb ? expandFrom : nbb;
+    if (nTile > 0) {
+      if (form)
+        segseg_tile_df<1><<<(unsigned)nTile, TILE, sizeof(TileSmemT<TILE, PolDF<1>>), st>>>(
+            A, PolDF<1>::Consts{kd, kf}, b0, partial, counters);
+      else
+        segseg_tile_df<0><<<(unsigned)nTile, TILE, sizeof(TileSmemT<TILE, PolDF<0>>), st>>>(
+            A, PolDF<0>::Consts{kd, kf}, b0, partial, counters);
+    }
     e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = form ? launch_expanded<PolDF<1>>(A, PolDF<1>::Consts{kd, kf}, nTile, nbb, numSeg, expandScratch, partial,
+                                           counters, st)
+               : launch_expanded<PolDF<0>>(A, PolDF<0>::Consts{kd, kf}, nTile, nbb, numSeg, expandScratch, partial,
+                                           counters, st);
     if (e != cudaSuccess) return e;
     e = capSlots >= nb ? strict::launch_reduce_all(partial, npad, numSeg, out, st)
                        : strict::launch_reduce_band(partial, J0, J1, numSeg, out, st);
@@ -163,19 +174,6 @@ cudaError_t launch_segseg_all_df(const KConsts& K, const double* soa, const floa
     J0 = J1;
   }
   return cudaSuccess;
-}
-
-cudaError_t launch_segseg_small_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,
-                                   int64_t npad, void* scratch, double* partial, double* out, int64_t numSeg,
-                                   unsigned long long* counters, cudaStream_t st, int form) {
-  const int64_t nt = npad / TILE, nb = nt * (nt + 1) / 2;
-  const TileArgs A{K, soa, skip, npad, soadf, nullptr};
-  const KConstsDF kd = kconsts_df(K);
-  const KConstsF kf = kconsts_f(K);
-  cudaError_t e =
-      form ? launch_expanded<PolDF<1>>(A, PolDF<1>::Consts{kd, kf}, nb, numSeg, scratch, partial, counters, st)
-           : launch_expanded<PolDF<0>>(A, PolDF<0>::Consts{kd, kf}, nb, numSeg, scratch, partial, counters, st);
-  return e != cudaSuccess ? e : strict::launch_reduce_all(partial, npad, numSeg, out, st);
 }
 
 cudaError_t launch_segseg_rows_df(const KConsts& K, const double* soa, const float* soadf, const uint8_t* skip,

@@ -249,15 +249,19 @@ cudaError_t launch_reduce_band(const double* partial, int64_t J0, int64_t J1, in
 
 cudaError_t launch_segseg_all_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                                   double* partial, double* out, int64_t numSeg, unsigned long long* counters,
-                                  cudaStream_t st, int64_t capSlots) {
+                                  cudaStream_t st, int64_t capSlots, int64_t expandFrom, void* expandScratch) {
   cudaError_t e = set_attr();
   if (e != cudaSuccess) return e;
   const int64_t nt = npad / TILE;
   const int64_t nb = nt * (nt + 1) / 2;
   const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
   if (capSlots >= nb) {
-    segseg_tile_f64<<<(unsigned)nb, TILE, sizeof(TileSmemT<TILE, PolF64>), st>>>(A, 0, partial, counters);
+    const int64_t nTile = expandFrom < nb ? expandFrom : nb;
+    if (nTile > 0)
+      segseg_tile_f64<<<(unsigned)nTile, TILE, sizeof(TileSmemT<TILE, PolF64>), st>>>(A, 0, partial, counters);
     e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = launch_expanded<PolF64>(A, PolF64::Consts{}, nTile, nb, numSeg, expandScratch, partial, counters, st);
     if (e != cudaSuccess) return e;
     segseg_reduce_all<<<(unsigned)((numSeg + 127) / 128), 128, 0, st>>>(partial, nt, numSeg, out);
     return cudaGetLastError();
@@ -274,16 +278,6 @@ cudaError_t launch_segseg_all_f64(const KConsts& K, const double* soa, const uin
     J0 = J1;
   }
   return cudaSuccess;
-}
-
-cudaError_t launch_segseg_small_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
-                                    void* scratch, double* partial, double* out, int64_t numSeg,
-                                    unsigned long long* counters, cudaStream_t st) {
-  const int64_t nt = npad / TILE;
-  const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
-  cudaError_t e = launch_expanded<PolF64>(A, PolF64::Consts{}, nt * (nt + 1) / 2, numSeg, scratch, partial,
-                                          counters, st);
-  return e != cudaSuccess ? e : launch_reduce_all(partial, npad, numSeg, out, st);
 }
 
 cudaError_t launch_segseg_rows_f64(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,

@@ -51,7 +51,7 @@ cudaError_t set_attr_fx() {
 
 cudaError_t launch_segseg_all_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                                  double* partial, double* out, int64_t numSeg, unsigned long long* counters,
-                                 cudaStream_t st, int64_t capSlots) {
+                                 cudaStream_t st, int64_t capSlots, int64_t expandFrom, void* expandScratch) {
   cudaError_t e = set_attr_fx();
   if (e != cudaSuccess) return e;
   const int64_t nt = npad / TILE;
@@ -62,8 +62,12 @@ cudaError_t launch_segseg_all_fx(const KConsts& K, const double* soa, const uint
   for (int64_t J0 = 0; J0 < nt;) {
     const int64_t J1 = capSlots >= nb ? nt : strict::segseg_band_end(J0, nt, capSlots);
     const int64_t b0 = J0 * (J0 + 1) / 2, nbb = J1 * (J1 + 1) / 2 - b0;
-    segseg_tile_fx<<<(unsigned)nbb, TILE, sizeof(TileSmemT<TILE, PolF64Fast>), st>>>(A, b0, partial, counters);
+    const int64_t nTile = capSlots >= nb && expandFrom < nb ? expandFrom : nbb;
+    if (nTile > 0)
+      segseg_tile_fx<<<(unsigned)nTile, TILE, sizeof(TileSmemT<TILE, PolF64Fast>), st>>>(A, b0, partial, counters);
     e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = launch_expanded<PolF64Fast>(A, PolF64Fast::Consts{}, nTile, nbb, numSeg, expandScratch, partial, counters, st);
     if (e != cudaSuccess) return e;
     e = capSlots >= nb ? strict::launch_reduce_all(partial, npad, numSeg, out, st)
                        : strict::launch_reduce_band(partial, J0, J1, numSeg, out, st);
@@ -71,17 +75,6 @@ cudaError_t launch_segseg_all_fx(const KConsts& K, const double* soa, const uint
     J0 = J1;
   }
   return cudaSuccess;
-}
-
-cudaError_t launch_segseg_small_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
-                                   void* scratch, double* partial, double* out, int64_t numSeg,
-                                   unsigned long long* counters, cudaStream_t st) {
-  const int64_t nt = npad / TILE;
-  const TileArgs A{K, soa, skip, npad, nullptr, nullptr};
-  cudaError_t e =
-      launch_expanded<PolF64Fast>(A, PolF64Fast::Consts{}, nt * (nt + 1) / 2, numSeg, scratch, partial,
-                                          counters, st);
-  return e != cudaSuccess ? e : strict::launch_reduce_all(partial, npad, numSeg, out, st);
 }
 
 cudaError_t launch_segseg_rows_fx(const KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,

@@ -44,12 +44,12 @@ __device__ __forceinline__ void x_tile_index(int64_t b, int64_t& I, int64_t& J) 
 // positions also go into a list.  Its order does not matter: each entry is
 // evaluated on its own and stored at its position.
 __global__ void __launch_bounds__(256)
-x_classify(const double* __restrict__ soa, const uint8_t* __restrict__ skip, int64_t npad, uint8_t* __restrict__ flags,
-           uint32_t* __restrict__ list, unsigned* __restrict__ count, unsigned long long* __restrict__ counters) {
+x_classify(const double* __restrict__ soa, const uint8_t* __restrict__ skip, int64_t npad, int64_t b0,
+           uint8_t* __restrict__ flags, uint32_t* __restrict__ list, unsigned* __restrict__ count, unsigned long long* __restrict__ counters) {
   const uint32_t pos = blockIdx.x * 256u + threadIdx.x;
   const int t = pos & (XT - 1), k = (pos >> 7) & (XT - 1), jl = (t + k) & (XT - 1);
   int64_t I, J;
-  x_tile_index(pos >> 14, I, J);
+  x_tile_index(b0 + (pos >> 14), I, J);
   const int64_t i = I * XT + t, j = J * XT + jl;
   int f = 0;
   if (skip[i] == 0 && skip[j] == 0 && (I != J || jl > t)) {
@@ -82,8 +82,9 @@ x_classify(const double* __restrict__ soa, const uint8_t* __restrict__ skip, int
 // 128 it costs 3 %.
 template <class P, bool QUAD>
 __global__ void __launch_bounds__(32)
-x_pairs(TileArgs A, typename P::Consts KP, const uint8_t* __restrict__ flags, const uint32_t* __restrict__ list,
-        const unsigned* __restrict__ count, double* __restrict__ vals, unsigned long long* __restrict__ counters) {
+x_pairs(TileArgs A, typename P::Consts KP, int64_t b0, const uint8_t* __restrict__ flags,
+        const uint32_t* __restrict__ list, const unsigned* __restrict__ count, double* __restrict__ vals,
+        unsigned long long* __restrict__ counters) {
   const int lane = threadIdx.x;
   if (blockIdx.x < kParCtas) {
     // Even CTAs take the forces on segment 1, odd ones those on segment 2: a short
@@ -94,7 +95,7 @@ x_pairs(TileArgs A, typename P::Consts KP, const uint8_t* __restrict__ flags, co
       const uint32_t pos = list[e];
       const int t = pos & (XT - 1), k = (pos >> 7) & (XT - 1), jl = (t + k) & (XT - 1);
       int64_t I, J;
-      x_tile_index(pos >> 14, I, J);
+      x_tile_index(b0 + (pos >> 14), I, J);
       const SegF64 a = tb_load_seg64(A.soa, A.npad, I * XT + t), s = tb_load_seg64(A.soa, A.npad, J * XT + jl);
       D3 F1, F2;
       nCore += side ? parallel_pair_side<2>(A.K, a, s, F1, F2) : parallel_pair_side<1>(A.K, a, s, F1, F2);
@@ -113,7 +114,7 @@ x_pairs(TileArgs A, typename P::Consts KP, const uint8_t* __restrict__ flags, co
   if (!__any_sync(0xffffffffu, act)) return;
   if (!QUAD && !act) return;  // a warp of quads stays whole: its lanes exchange corners
   int64_t I, J;
-  x_tile_index(bk >> 7, I, J);
+  x_tile_index(b0 + (bk >> 7), I, J);
   const int64_t i = I * XT + t, j = J * XT + ((t + (int)(bk & (XT - 1))) & (XT - 1));
   const typename P::Seg a = P::load_global(A, i), s = P::load_global(A, j);
   typename P::Scalar c;
@@ -232,26 +233,32 @@ struct XScratch {
   }
 };
 
-// Classes, pairs and the slots of every tile pair (what the tile kernel writes).
+// Classes, pairs and the slots (what the tile kernel writes) of tile pairs b0 to
+// nb - 1, at most kExpandMaxPairs at a time through one scratch.
 template <class P>
-cudaError_t launch_expanded(const TileArgs& A, const typename P::Consts& KP, int64_t nb, int64_t numSeg,
+cudaError_t launch_expanded(const TileArgs& A, const typename P::Consts& KP, int64_t b0, int64_t nb, int64_t numSeg,
                             void* scratch, double* partial, unsigned long long* counters, cudaStream_t st) {
   const int live = nb == 1 ? (int)numSeg : XT;
-  const XScratch x(scratch, nb);
-  cudaError_t e = cudaMemsetAsync(x.count, 0, sizeof(unsigned), st);
-  if (e != cudaSuccess) return e;
-  x_classify<<<(unsigned)(nb * XPOS / 256), 256, 0, st>>>(A.soa, A.skip, A.npad, x.flags, x.list, x.count, counters);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if constexpr (P::kQuad) {
-    if (numSeg <= kQuadSegs)
-      x_pairs<P, true><<<kParCtas + XT * 16, 32, 0, st>>>(A, KP, x.flags, x.list, x.count, x.vals, counters);
+  for (; b0 < nb; b0 += kExpandMaxPairs) {
+    const int64_t n = nb - b0 < kExpandMaxPairs ? nb - b0 : kExpandMaxPairs;
+    const XScratch x(scratch, n);
+    cudaError_t e = cudaMemsetAsync(x.count, 0, sizeof(unsigned), st);
+    if (e != cudaSuccess) return e;
+    x_classify<<<(unsigned)(n * XPOS / 256), 256, 0, st>>>(A.soa, A.skip, A.npad, b0, x.flags, x.list, x.count,
+                                                           counters);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if constexpr (P::kQuad) {
+      if (numSeg <= kQuadSegs)
+        x_pairs<P, true><<<kParCtas + XT * 16, 32, 0, st>>>(A, KP, b0, x.flags, x.list, x.count, x.vals, counters);
+    }
+    if (!P::kQuad || numSeg > kQuadSegs)
+      x_pairs<P, false><<<(unsigned)(kParCtas + n * XT * 4), 32, 0, st>>>(A, KP, b0, x.flags, x.list, x.count, x.vals,
+                                                                          counters);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    x_fold<P><<<(unsigned)(n * 12), XT, 0, st>>>(x.vals, x.flags, live, partial + b0 * 12 * XT);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  if (!P::kQuad || numSeg > kQuadSegs)
-    x_pairs<P, false><<<(unsigned)(kParCtas + nb * XT * 4), 32, 0, st>>>(A, KP, x.flags, x.list, x.count, x.vals,
-                                                                         counters);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  x_fold<P><<<(unsigned)(nb * 12), XT, 0, st>>>(x.vals, x.flags, live, partial);
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------

@@ -39,6 +39,35 @@ def test_expanded_equals_tile_kernel(pkg, synth, mode, n):
         assert rep[key] == rep_t[key]
 
 
+@pytest.mark.parametrize("mode", ["fp64", "fp64_fma", "fp64_fast", "df64", "f32c"])
+@pytest.mark.parametrize("nt", [18, 24, 25, 28, 40])
+def test_expanded_rest_equals_tile_kernel(pkg, synth, mode, nt):
+    """171 tile pairs (two chunks of the pair store), 300 (strict only), one wave of
+    304 and 21 or 102, two and 212; the tile kernel alone under a
+    limit that the store does not fit."""
+    n = 128 * nt - 37
+    net = _synthetic(pkg, synth, (n + 7) // 8, nt, parallel_fraction=0.1, cube=12000.0)
+    net.numSeg = n
+    net.extSeg[5::17] = 1
+    dln, mat = _params(pkg)
+    ctx = pkg.get_context()
+    ctx.mode = mode
+    try:
+        F = pkg.calcSegSegForce(dln, mat, net)
+        rep = dict(ctx.last_report)
+        ctx.partial_limit = nt * (nt + 1) // 2 * 12288
+        T = pkg.calcSegSegForce(dln, mat, net)
+        rep_t = dict(ctx.last_report)
+    finally:
+        ctx.mode, ctx.partial_limit = "fp64", 0
+    if mode == "fp64_fma":
+        assert np.linalg.norm(F - T) <= 1e-10 * np.linalg.norm(T)
+    else:
+        assert np.array_equal(F, T)
+    for key in ("pairs_general", "pairs_parallel", "core_sides"):
+        assert rep[key] == rep_t[key]
+
+
 @pytest.mark.parametrize("n,rows", [(2, 1), (33, 40), (2017, 1), (2017, 600)])
 def test_index_rows(pkg, synth, oracle, n, rows):
     """One step and seven steps per CTA (600 rows of 2,017 segments), columns
