@@ -1132,7 +1132,7 @@ def main():
                                  TILE_FX_DRAM_BYTES_PER_TILE_PAIR) * (n // 128) * (n // 128 + 1) // 2,
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch at 32,768 "
                                        "segments, scaled by tile pairs",
-                     "kernel": "segseg_tile_f64<0>" if args.mode == "fp64" else "segseg_tile_fx<0>",
+                     "kernel": "segseg_tile_f64" if args.mode == "fp64" else "segseg_tile_fx",
                      "peak_source": "measured FP64 FMA-chain probe on this GPU (ddd_probe_fma_peak, ~1 s per "
                                     "timing, best of 3); MEASURED_PEAKS.json holds no FP64 figure",
                      "probe_clock": probe_clock,

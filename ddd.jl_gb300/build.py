@@ -24,7 +24,8 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", 
 # registers left for the operators' two constants (2-4 % slower with them), and
 # for the strict calc_uTilde, mostly CUDA's acos and tan (2 % slower).
 VARIANTS = {
-    "segseg_f64.cu": [("strict", ["-DDDD_VARIANT=strict", "--fmad=false"]), ("fast", ["-DDDD_VARIANT=fast", "-DDDD_F64_CONTRACT"])],
+    "segseg_f64.cu": [("strict", ["-DDDD_VARIANT=strict", "--fmad=false"]),
+                      ("fast", ["-DDDD_VARIANT=fast", "-DDDD_F64_CONTRACT", "-DDDD_FMA"])],
     "sigma_f64.cu": [("strict", ["-DDDD_VARIANT=strict", "--fmad=false"]), ("fast", ["-DDDD_VARIANT=fast", "-DDDD_F64_CONTRACT"])],
     # df64 needs exact error-free transformations: no contraction.
     "segseg_df.cu": [("", ["--fmad=false", "-DDDD_F64_CONTRACT"])],

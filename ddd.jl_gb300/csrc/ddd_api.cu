@@ -117,11 +117,9 @@ cudaError_t run_segseg_all(ddd_ctx* c, const ddd::KConsts& K, const double* soa,
   // obeys the partial-sum limit too; without it (limit, no memory) the tile kernel
   // takes all, with the same bits.
   const int64_t nt = npad / ddd::strict::segseg_npad(1), nb = nt * (nt + 1) / 2;
-  const ddd::ExpandRule& rule = use_df(c)    ? (df_form(c) ? ddd::kExpandMixed : ddd::kExpandDF)
-                                : use_fx(c)  ? ddd::kExpandFx
-                                : use_fma(c) ? ddd::kExpandFma
-                                             : ddd::kExpandF64;
-  int64_t from = ddd::expand_from(nb, rule);
+  const ddd::ExpandRule& rule = use_df(c) ? (df_form(c) ? ddd::kExpandMixed : ddd::kExpandDF)
+                                : use_fx(c) ? ddd::kExpandFx : ddd::kExpandF64;
+  int64_t from = use_fma(c) ? nb : ddd::expand_from(nb, rule);
   void* x = nullptr;
   if (cap >= nb && from < nb && (int64_t)ddd::expand_bytes(nb - from) <= partial_limit(c)) {
     const cudaError_t e = c->expand.ensure(ddd::expand_bytes(nb - from));
@@ -137,7 +135,7 @@ cudaError_t run_segseg_all(ddd_ctx* c, const ddd::KConsts& K, const double* soa,
     return ddd::launch_segseg_all_df(K, soa, c->soadf.as<float>(), skip, npad, partial, out, numSeg, cnt, st,
                                      df_form(c), cap, from, x);
   if (use_fx(c)) return ddd::launch_segseg_all_fx(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap, from, x);
-  return use_fma(c) ? ddd::fast::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap, from, x)
+  return use_fma(c) ? ddd::fast::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap)
                     : ddd::strict::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap, from,
                                                          x);
 }

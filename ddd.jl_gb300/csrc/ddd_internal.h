@@ -68,18 +68,18 @@ inline size_t row_partial_bytes(const RowPlan& p, int64_t nRows) { return (size_
 //   strict   0+171 7.93 / 14.02 ms, 1+47 17.1 / 26.9, 2+212 39.6 / 42.6, 8+53 120.9 / 123.1
 //   fast     0+171 5.02 / 8.35, 1+47 10.3 / 15.9, 8+53 71.0 / 72.6; at 1+291 17.4 / 17.2
 //   df64     0+171 3.05 / 4.48, 1+224 8.93 / 9.40, 4+162 22.3 / 23.0; at 5+191 28.0 / 27.7
-//   FMA      none: the compiler contracts the two kernels differently (the others
-//            give the same bits), and at 300 tile pairs with a tenth of the pairs
-//            near-parallel that moved the forces by 2e-10
 //   f32c     0+171 1.72 / 2.34, 1+102 3.63 / 3.78; at 0+276 2.70 / 2.55, 1+224 4.89 / 4.64
 constexpr int64_t kExpandMaxPairs = 153;
 constexpr int64_t kTileWave = 304;
 struct ExpandRule {
   int waves, most, perWave;
 };
-constexpr ExpandRule kExpandF64 = {8, 304, 0}, kExpandFma = {-1, 0, 0}, kExpandFx = {8, 264, 0}, kExpandDF = {4, 240, 16},
+constexpr ExpandRule kExpandF64 = {8, 304, 0}, kExpandFx = {8, 264, 0}, kExpandDF = {4, 240, 16},
                      kExpandMixed = {1, 240, 128};
-// The first tile pair that goes to the expanded kernels.
+// The first tile pair that goes to the expanded kernels.  Not for the FMA form:
+// where the others give the tile kernel's bits, the compiler contracts its
+// near-parallel branch differently in each kernel, and through that branch's
+// cancellations the forces moved by up to 1e-8 of their norm.
 inline int64_t expand_from(int64_t nb, const ExpandRule& r) {
   if (nb <= kExpandMaxPairs) return 0;
   const int64_t w = nb / kTileWave, rest = nb % kTileWave;

@@ -509,10 +509,8 @@ __device__ __forceinline__ int par_side(const KConsts& K, D3 na1, D3 na2, D3 ta,
   return 0;
 }
 
-// calcParSegSegForce (DislocationForces.jl:1167-1442).  NEED34 = false skips
-// the second side (the index-list form discards it).  Returns the number of
+// calcParSegSegForce (DislocationForces.jl:1167-1442).  Returns the number of
 // sides (0-2) that needed the two core-correction evaluations.
-template <bool NEED34>
 __device__ __forceinline__ int parallel_pair(const KConsts& K, D3 b1, D3 n11, D3 n12, D3 t1, rd t1N, D3 b2,
                                               D3 n21, D3 n22, D3 t2, rd t2N, rd c, D3& F1, D3& F2, D3& F3,
                                               D3& F4) {
@@ -525,7 +523,7 @@ __device__ __forceinline__ int parallel_pair(const KConsts& K, D3 b1, D3 n11, D3
     b1 = -b1;
   }
   int cores = par_side<1>(K, n11, n12, t1, t1N, b1, n21, n22, t2, t2N, b2, F1, F2);
-  if (NEED34) cores += par_side<2>(K, n21, n22, t2, t2N, b2, n11, n12, t1, t1N, b1, F3, F4);
+  cores += par_side<2>(K, n21, n22, t2, t2N, b2, n11, n12, t1, t1N, b1, F3, F4);
   if (flip) {
     D3 tmp = F1;
     F1 = F2;

@@ -260,8 +260,10 @@ cudaError_t launch_segseg_all_f64(const KConsts& K, const double* soa, const uin
     if (nTile > 0)
       segseg_tile_f64<<<(unsigned)nTile, TILE, sizeof(TileSmemT<TILE, PolF64>), st>>>(A, 0, partial, counters);
     e = cudaGetLastError();
+#ifndef DDD_FMA
     if (e == cudaSuccess)
       e = launch_expanded<PolF64>(A, PolF64::Consts{}, nTile, nb, numSeg, expandScratch, partial, counters, st);
+#endif
     if (e != cudaSuccess) return e;
     segseg_reduce_all<<<(unsigned)((numSeg + 127) / 128), 128, 0, st>>>(partial, nt, numSeg, out);
     return cudaGetLastError();

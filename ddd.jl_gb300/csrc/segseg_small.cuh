@@ -1,7 +1,8 @@
 // Seg-seg kernels whose unit of work is a step of 32 or 128 pairs, for calls that
 // one CTA per 128 x 128 tile pair cannot spread over the GPU:
-//   * the all-pairs force of small networks ("expanded": every pair's forces are
-//     stored and folded afterwards),
+//   * the all-pairs force ("expanded": every pair's forces are stored and folded
+//     afterwards) of small networks, and of larger ones the tile pairs beyond the
+//     tile kernel's last full wave (not in the FMA build: ddd_internal.h),
 //   * the index-list force (any size): one row segment against all others.
 // Templated on the arithmetic policy of tile_body.cuh; the kernels have internal
 // linkage because the strict and the FMA build compile this header with
@@ -147,7 +148,7 @@ __device__ __forceinline__ void all_loaded(double* x) {
 // warp of rows by warp, by step within one, its near-parallel ones by row
 // within one.  The loads of a batch of steps are in flight together and do not
 // wait for the classes (a position without a pair holds anything and is not
-// added): 30 us at one tile pair became 10.  Only the first `live` rows and
+// added): 30 us at one tile pair became 12.  Only the first `live` rows and
 // columns can hold pairs when there is one tile.
 template <class P>
 __global__ void __launch_bounds__(XT)

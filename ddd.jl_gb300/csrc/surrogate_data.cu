@@ -39,7 +39,7 @@ __global__ void pair_data(KConsts K, const double* __restrict__ soa, int64_t npa
   if (1.0 - c * c > kSqrtEps)
     general_pair<true, true>(K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, c, F1, F2, F3, F4);
   else
-    parallel_pair<true>(K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, c, F1, F2, F3, F4);
+    parallel_pair(K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, c, F1, F2, F3, F4);
   const D3 ma = 0.5 * (a.n1 + a.n2), mb = 0.5 * (b.n1 + b.n2);
   const D3 rd = mb - ma;
   const float r[3] = {(float)rd.x, (float)rd.y, (float)rd.z};

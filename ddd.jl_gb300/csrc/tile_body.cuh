@@ -60,8 +60,8 @@ __device__ __forceinline__ SegF64 tb_load_seg64(const double* __restrict__ soa, 
 static __device__ __forceinline__ int tb_parallel_pair(const TileArgs& A, int64_t gi, int64_t gj, double* f, int stride) {
   const SegF64 a = tb_load_seg64(A.soa, A.npad, gi), b = tb_load_seg64(A.soa, A.npad, gj);
   D3 F1, F2, F3, F4;
-  const int cores = parallel_pair<true>(A.K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, dot(a.t, b.t), F1,
-                                        F2, F3, F4);
+  const int cores = parallel_pair(A.K, a.b, a.n1, a.n2, a.t, a.tN, b.b, b.n1, b.n2, b.t, b.tN, dot(a.t, b.t), F1, F2,
+                                  F3, F4);
   f[0 * stride] = F1.x; f[1 * stride] = F1.y; f[2 * stride] = F1.z;
   f[3 * stride] = F2.x; f[4 * stride] = F2.y; f[5 * stride] = F2.z;
   f[6 * stride] = F3.x; f[7 * stride] = F3.y; f[8 * stride] = F3.z;

@@ -3,9 +3,8 @@
 //   FORM 0: every general-pair operation in df64 (general_pair_df);
 //   FORM 1: corner antiderivatives and moments in df64, V-vector assembly and
 //           node sums in FP32 (general_pair_mixed), the "f32c" form.
-// Used by the precision-form kernels (segseg_df.cu), the batched persistent
-// kernel (segseg_batch.cu) and the surrogate's exact passes
-// (surrogate_force.cu).  Include from translation units compiled with
+// Used by the precision-form kernels (segseg_df.cu) and by the persistent
+// kernels of the batch and of the surrogate's exact passes (tile_launch.cu).  Include from translation units compiled with
 // --fmad=false (df64 needs exact TwoSum/TwoProd).
 #pragma once
 #include <cstdint>

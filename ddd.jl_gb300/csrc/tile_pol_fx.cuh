@@ -2,8 +2,8 @@
 // policy (segment data, branch decision, near-parallel branch, accumulation)
 // with the general branch of pair_f64fast.cuh, its logarithms and arctangents on
 // the integer pipes (intmath_f64.cuh).  Used by the all-pairs and
-// index-list kernels (segseg_f64fast.cu) and by the surrogate path's exact
-// passes (surrogate_force.cu); both translation units compile without
+// index-list kernels (segseg_f64fast.cu) and by the persistent kernels of the batch
+// and of the surrogate's exact passes (tile_launch.cu); both translation units compile without
 // contraction, so the fused operations are exactly pair_f64fast.cuh's.
 #pragma once
 #include "pair_f64.cuh"
