@@ -373,15 +373,20 @@ uint32_t slot_hash(uint32_t x) {
   return x;
 }
 
-// The exact tile pass in the arithmetic of `mode` (DDD_MODE_FP64 strict,
-// DDD_MODE_FP64_FAST, DDD_MODE_DF64 or DDD_MODE_F32C for the general branch).
+// The exact tile passes in the arithmetic of `mode` (DDD_MODE_FP64 strict,
+// DDD_MODE_FP64_FAST, DDD_MODE_DF64 or DDD_MODE_F32C for the general branch):
+// MODE 2 the near pass, MODE 0 whole tiles.
 template <int MODE>
 cudaError_t launch_exact(int mode, const TileArgs& A, const int4* items, const int32_t* nDev, int32_t nHost,
                          int32_t* next, double* partial, unsigned long long* counters, int grid, cudaStream_t st) {
-  if (mode == DDD_MODE_FP64 || mode == DDD_MODE_FP64_FAST)
-    return f64_tiles::exact_launch(mode == DDD_MODE_FP64_FAST, MODE, A, items, nDev, nHost, next, partial, counters,
-                                   grid, st);
-  return df_tiles::exact_launch(mode != DDD_MODE_DF64, MODE, A, items, nDev, nHost, next, partial, counters, grid, st);
+  const bool f64 = mode == DDD_MODE_FP64 || mode == DDD_MODE_FP64_FAST;
+  const int pol = f64 ? mode == DDD_MODE_FP64_FAST : mode != DDD_MODE_DF64;
+  if constexpr (MODE == 2)
+    return f64 ? near_tiles::near_launch(pol, A, items, nDev, nHost, next, partial, counters, grid, st)
+               : df_tiles::near_launch(pol, A, items, nDev, nHost, next, partial, counters, grid, st);
+  else
+    return f64 ? f64_tiles::exact_launch(pol, A, items, nDev, nHost, next, partial, counters, grid, st)
+               : df_tiles::exact_launch(pol, A, items, nDev, nHost, next, partial, counters, grid, st);
 }
 
 cudaError_t ensure_plan(ddd_surrogate* s, int64_t numSeg, double auditFraction) {
@@ -397,7 +402,7 @@ cudaError_t ensure_plan(ddd_surrogate* s, int64_t numSeg, double auditFraction) 
     P.auditFraction = -1.0;
     if ((e = cudaDeviceGetAttribute(&P.sms, cudaDevAttrMultiProcessorCount, s->device)) != cudaSuccess) return e;
     int per = 0;  // the df64 policies use the same shared memory and register budget
-    if ((e = f64_tiles::exact_occupancy(&per)) != cudaSuccess) return e;
+    if ((e = near_tiles::near_occupancy(&per)) != cudaSuccess) return e;
     P.gridExact = P.sms * std::max(1, per);
     P.gridQuad = P.sms * quad_far_blocks_per_sm(3);
     const size_t n = (size_t)numSeg, np = (size_t)P.npad;

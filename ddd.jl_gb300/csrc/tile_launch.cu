@@ -1,8 +1,12 @@
 // Persistent kernels over tile pairs: CTAs take work items from a global counter
 // (one atomicAdd per item, no waiting) and run the shared tile body on each.
-// Compiled twice, with --fmad=false: the FP64 policies with f64reg.cuh's
-// operators, the df64 ones (DDD_DF_POLICIES) with plain ones, whose two constants
-// their FP32 main loop has no registers for.
+// Compiled three times, with --fmad=false: the FP64 policies with f64reg.cuh's
+// operators; the df64 ones (DDD_DF_POLICIES) with plain ones, whose two constants
+// their FP32 main loop has no registers for; and the near pass of the FP64 ones
+// (DDD_NEAR_PASS) with plain ones too: its dense chunks hold few pairs, and a
+// pair that starts with those constants' loads and spills took the whole call of
+// 32,768 segments with the 2-point far field from 53.2 to 59.3 ms (fast FP64 near
+// pairs; 75.0 to 78.2 strict).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -13,6 +17,9 @@
 #ifdef DDD_DF_POLICIES
 #include "tile_pol_df.cuh"
 #define DDD_TILE_NS df_tiles
+#elif defined(DDD_NEAR_PASS)
+#include "tile_pol_fx.cuh"
+#define DDD_TILE_NS near_tiles
 #else
 #include "tile_pol_fx.cuh"
 #define DDD_TILE_NS f64_tiles
@@ -75,6 +82,22 @@ static cudaError_t launch(const TileArgs& A, const int4* items, const int32_t* n
   return cudaGetLastError();
 }
 
+#if defined(DDD_NEAR_PASS) || defined(DDD_DF_POLICIES)
+cudaError_t near_launch(int pol, const TileArgs& A, const int4* items, const int32_t* nDev, int32_t nHost,
+                        int32_t* next, double* partial, unsigned long long* counters, int grid, cudaStream_t st) {
+  return pol ? launch<128, 2, Pol1>(A, items, nDev, nHost, next, partial, counters, grid, st)
+             : launch<128, 2, Pol0>(A, items, nDev, nHost, next, partial, counters, grid, st);
+}
+
+cudaError_t near_occupancy(int* per) {
+  const cudaError_t e = set_attr<128, 2, Pol0>();
+  return e != cudaSuccess ? e
+                          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, persistent_tiles<128, 2, Pol0>, 128,
+                                                                          sizeof(TileSmemT<128, Pol0>));
+}
+#endif
+
+#ifndef DDD_NEAR_PASS
 template <int T, class P>
 static cudaError_t prepare(int device, int64_t nItems, unsigned* grid) {
   cudaError_t e = set_attr<T, 0, P>();
@@ -88,20 +111,10 @@ static cudaError_t prepare(int device, int64_t nItems, unsigned* grid) {
   return cudaSuccess;
 }
 
-cudaError_t exact_launch(int pol, int mode, const TileArgs& A, const int4* items, const int32_t* nDev, int32_t nHost,
+cudaError_t exact_launch(int pol, const TileArgs& A, const int4* items, const int32_t* nDev, int32_t nHost,
                          int32_t* next, double* partial, unsigned long long* counters, int grid, cudaStream_t st) {
-  if (mode == 2)
-    return pol ? launch<128, 2, Pol1>(A, items, nDev, nHost, next, partial, counters, grid, st)
-               : launch<128, 2, Pol0>(A, items, nDev, nHost, next, partial, counters, grid, st);
   return pol ? launch<128, 0, Pol1>(A, items, nDev, nHost, next, partial, counters, grid, st)
              : launch<128, 0, Pol0>(A, items, nDev, nHost, next, partial, counters, grid, st);
-}
-
-cudaError_t exact_occupancy(int* per) {
-  const cudaError_t e = set_attr<128, 2, Pol0>();
-  return e != cudaSuccess ? e
-                          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, persistent_tiles<128, 2, Pol0>, 128,
-                                                                          sizeof(TileSmemT<128, Pol0>));
 }
 
 cudaError_t batch_prepare(int pol, int T, int device, int64_t nItems, unsigned* grid) {
@@ -117,6 +130,7 @@ cudaError_t batch_launch(int pol, int T, const TileArgs& A, unsigned grid, const
   return pol ? launch<128, 0, Pol1>(A, items, nullptr, nItems, next, partial, counters, grid, st)
              : launch<128, 0, Pol0>(A, items, nullptr, nItems, next, partial, counters, grid, st);
 }
+#endif
 
 }  // namespace DDD_TILE_NS
 }  // namespace ddd
