@@ -216,7 +216,15 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
   __syncthreads();
   const int nPar = sm.total;
   D3 fp1 = {0, 0, 0}, fp2 = {0, 0, 0}, fjp3 = {0, 0, 0}, fjp4 = {0, 0, 0};
-  D3 fjt3 = {0, 0, 0}, fjt4 = {0, 0, 0};  // MODE 0: column sums of the warps before jw
+  // MODE 0: column sums of the warps before jw, apart so that segseg_small.cuh can
+  // add in the same order.  The FMA build has no such path and keeps one sum: the
+  // second made it 1 % slower (16,384 segments 293 -> 291 ms without).
+#ifdef DDD_FMA
+  constexpr bool byWarp = false;
+#else
+  constexpr bool byWarp = !CLS;
+#endif
+  D3 fjt3 = {0, 0, 0}, fjt4 = {0, 0, 0};
   int jw = 0;
   unsigned long long nCore = 0;
   // Chunks of CH never straddle the two runs, so a warp runs one branch.
@@ -261,7 +269,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
     for (int q = 0; q < lim; ++q) {
       const int pe = sm.plist[base + q];
       if ((pe & 0xff) == t) {
-        if (!CLS && (pe >> 13) != jw) {  // the rows of the next warp
+        if (byWarp && (pe >> 13) != jw) {  // the rows of the next warp
           fjt3 = fjt3 + fjp3;
           fjt4 = fjt4 + fjp4;
           fjp3 = fjp4 = {0, 0, 0};
@@ -304,8 +312,8 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
   p[3 * T + t] = r2.x + fp2.x;
   p[4 * T + t] = r2.y + fp2.y;
   p[5 * T + t] = r2.z + fp2.z;
-  fjt3 = fjt3 + fjp3;
-  fjt4 = fjt4 + fjp4;
+  fjt3 = byWarp ? fjt3 + fjp3 : fjp3;
+  fjt4 = byWarp ? fjt4 + fjp4 : fjp4;
   const double add[6] = {fjt3.x, fjt3.y, fjt3.z, fjt4.x, fjt4.y, fjt4.z};
 #pragma unroll
   for (int c = 0; c < 6; ++c) p[(6 + c) * T + t] = P::template col_sum<T>(sm.pol, c, t) + add[c];
