@@ -41,6 +41,10 @@ struct ddd_ctx {
   const uint8_t* dExt = nullptr;
   char* pin = nullptr;  // pinned staging of small copies (PinArena)
   size_t pinUsed = 0;
+  // Last use of `expand` (Expand): its stream, and the event behind it when that
+  // stream is the caller's.
+  cudaStream_t expandStream = nullptr;
+  cudaEvent_t expandEv = nullptr;
   ddd::CollisionPlan* coll = nullptr;
   DevBuf upoints;  // calc_uTilde evaluation points
   ddd::UTildeScratch* ut = nullptr;
@@ -105,6 +109,47 @@ size_t partial_bytes(const ddd_ctx* c, int64_t npad) {
   return (size_t)partial_slots(c, npad) * ddd::strict::segseg_partial_bytes_all(ddd::strict::segseg_npad(1));
 }
 
+// Scratch of one call on stream `st` in ctx->expand: the pair store or the partial
+// stresses.  Calls of one context on several streams share it (one may be in flight
+// while the next is queued), so each use waits for the one before.  A stream under
+// capture gets none: a graph must neither allocate nor keep a buffer that a later
+// call replaces, and no event orders its replays.  Without it (p null: no memory
+// either) the caller takes the form that needs none.
+struct Expand {
+  ddd_ctx* c;
+  cudaStream_t st;
+  void* p = nullptr;
+  Expand(ddd_ctx* ctx, cudaStream_t stream) : c(ctx), st(stream) {}
+  Expand(const Expand&) = delete;
+  Expand& operator=(const Expand&) = delete;
+  cudaError_t take(size_t bytes) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(st, &cap);
+    if (e != cudaSuccess || cap != cudaStreamCaptureStatusNone) return e;
+    e = c->expand.ensure(bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return cudaSuccess;
+    }
+    // The context's own stream outlives this call; a caller's stream may be gone (and
+    // its handle reused), so its event was recorded behind the use.
+    if (e == cudaSuccess && c->expandStream && (c->expandStream != c->stream || st != c->stream)) {
+      if (!c->expandEv) e = cudaEventCreateWithFlags(&c->expandEv, cudaEventDisableTiming);
+      if (e == cudaSuccess && c->expandStream == c->stream) e = cudaEventRecord(c->expandEv, c->stream);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, c->expandEv, 0);
+    }
+    if (e == cudaSuccess && st != c->stream && !c->expandEv)
+      e = cudaEventCreateWithFlags(&c->expandEv, cudaEventDisableTiming);
+    if (e == cudaSuccess) p = c->expand.p;
+    return e;
+  }
+  ~Expand() {
+    if (!p) return;
+    c->expandStream = st;
+    if (st != c->stream) cudaEventRecord(c->expandEv, st);
+  }
+};
+
 cudaError_t run_segseg_all(ddd_ctx* c, const ddd::KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                            double* partial, double* out, int64_t numSeg, unsigned long long* cnt, cudaStream_t st) {
   const int64_t cap = partial_slots(c, npad);
@@ -120,24 +165,19 @@ cudaError_t run_segseg_all(ddd_ctx* c, const ddd::KConsts& K, const double* soa,
   const ddd::ExpandRule& rule = use_df(c) ? (df_form(c) ? ddd::kExpandMixed : ddd::kExpandDF)
                                 : use_fx(c) ? ddd::kExpandFx : ddd::kExpandF64;
   int64_t from = use_fma(c) ? nb : ddd::expand_from(nb, rule);
-  void* x = nullptr;
+  Expand x(c, st);
   if (cap >= nb && from < nb && (int64_t)ddd::expand_bytes(nb - from) <= partial_limit(c)) {
-    const cudaError_t e = c->expand.ensure(ddd::expand_bytes(nb - from));
-    if (e == cudaSuccess) {
-      x = c->expand.p;
-    } else {
-      if (e != cudaErrorMemoryAllocation) return e;
-      cudaGetLastError();
-    }
+    const cudaError_t e = x.take(ddd::expand_bytes(nb - from));
+    if (e != cudaSuccess) return e;
   }
-  if (!x) from = nb;
+  if (!x.p) from = nb;
   if (use_df(c))
     return ddd::launch_segseg_all_df(K, soa, c->soadf.as<float>(), skip, npad, partial, out, numSeg, cnt, st,
-                                     df_form(c), cap, from, x);
-  if (use_fx(c)) return ddd::launch_segseg_all_fx(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap, from, x);
+                                     df_form(c), cap, from, x.p);
+  if (use_fx(c)) return ddd::launch_segseg_all_fx(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap, from, x.p);
   return use_fma(c) ? ddd::fast::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap)
                     : ddd::strict::launch_segseg_all_f64(K, soa, skip, npad, partial, out, numSeg, cnt, st, cap, from,
-                                                         x);
+                                                         x.p);
 }
 
 // Index rows per launch: all of them when their partial sums (6 doubles per row
@@ -173,35 +213,26 @@ cudaError_t run_segseg_rows(ddd_ctx* c, const ddd::KConsts& K, const double* soa
   return cudaSuccess;
 }
 
-// Scratch of a σ̃ call in ctx->expand, which no other call in flight uses: null
-// when none is wanted, or when there is no memory for it (the caller then takes
-// the form without).
-cudaError_t sigma_scratch(ddd_ctx* c, size_t bytes, double** out) {
-  *out = nullptr;
-  if (!bytes) return cudaSuccess;
-  const cudaError_t e = c->expand.ensure(bytes);
-  if (e == cudaSuccess) *out = c->expand.as<double>();
-  if (e != cudaErrorMemoryAllocation) return e;
-  cudaGetLastError();
-  return cudaSuccess;
-}
-
 cudaError_t run_sigma(ddd_ctx* c, const ddd::KConsts& K, const double* soa, int64_t npad, int64_t nSeg,
                       const double* x0, int64_t M, double* sigma, cudaStream_t st) {
-  double* scratch = nullptr;
+  Expand x(c, st);
   if (use_df(c) || use_fx(c)) {
     // Resident CTAs: 152 SMs x 8 CTAs of 128 (mixed) or 24 warps (fast).
     ddd::SigmaPlan plan = use_df(c) ? ddd::sigma_plan(nSeg, M, 128, 1216) : ddd::sigma_plan(nSeg, M, 32, 3648);
     const size_t bytes = ddd::sigma_part_bytes(plan, M);
-    cudaError_t e = sigma_scratch(c, bytes, &scratch);
+    cudaError_t e = prep_df_if_needed(c, npad, st);  // both precision modes: the mixed σ̃ form
+    if (e == cudaSuccess && bytes) e = x.take(bytes);
     if (e != cudaSuccess) return e;
+    double* scratch = static_cast<double*>(x.p);
     if (!scratch) plan = ddd::SigmaPlan{1, 1, npad};
     if (use_fx(c)) return ddd::launch_sigma_fx(K, soa, npad, nSeg, x0, M, sigma, plan, scratch, st);
-    if ((e = prep_df_if_needed(c, npad, st)) != cudaSuccess) return e;  // both precision modes: the mixed σ̃ form
     return ddd::launch_sigma_mixed(K, c->soadf.as<float>(), npad, nSeg, x0, M, sigma, plan, scratch, st);
   }
-  const cudaError_t e = sigma_scratch(c, M < ddd::kSigmaSplitPoints ? ddd::sigma_split_bytes(npad) : 0, &scratch);
-  if (e != cudaSuccess) return e;
+  if (M < ddd::kSigmaSplitPoints) {
+    const cudaError_t e = x.take(ddd::sigma_split_bytes(npad));
+    if (e != cudaSuccess) return e;
+  }
+  double* scratch = static_cast<double*>(x.p);
   return use_fma(c) ? ddd::fast::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, scratch, st)
                     : ddd::strict::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, scratch, st);
 }
@@ -455,6 +486,7 @@ void ddd_destroy(ddd_ctx* c) {
     b->release();
   for (auto& ev : c->ev)
     if (ev) cudaEventDestroy(ev);
+  if (c->expandEv) cudaEventDestroy(c->expandEv);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }

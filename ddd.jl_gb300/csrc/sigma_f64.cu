@@ -9,6 +9,8 @@
 // too few points for that take sigma_split.
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "ddd_internal.h"
 #include "pair_f64.cuh"
 
@@ -126,6 +128,10 @@ cudaError_t launch_sigma_f64(const KConsts& K, const double* soa, int64_t npad, 
     sigma_tilde_f64<<<(unsigned)((M + SIG_TILE - 1) / SIG_TILE), SIG_TILE, 0, st>>>(K, soa, npad, nSeg, x0, M, sigma);
     return cudaGetLastError();
   }
+  // Loaded here too: a later call under stream capture has no scratch.
+  static std::atomic<uint64_t> loaded{0};
+  const cudaError_t le = set_smem_once(sigma_tilde_f64, 0, loaded);
+  if (le != cudaSuccess) return le;
   double* store[2] = {scratch, scratch + 6 * kSigmaChunk};
   double* txb = scratch + 12 * kSigmaChunk;
   sigma_txb<<<(unsigned)((npad + 255) / 256), 256, 0, st>>>(soa, npad, txb);

@@ -294,7 +294,11 @@ int ddd_sigma_tilde(ddd_ctx* ctx, const ddd_consts* k, const double* x0, int64_t
  * pointers in the layouts above.  The work is enqueued on `stream`
  * (a cudaStream_t, NULL = the context's stream) and the call returns without
  * waiting unless rep != NULL.  Same semantics as ddd_segseg_force (idx == NULL)
- * and ddd_sigma_tilde (idx == NULL). */
+ * and ddd_sigma_tilde (idx == NULL).  A call (with rep == NULL) can be captured
+ * on `stream` when an earlier one of its kind, in its mode and with at least as
+ * many segments, has sized the context's buffers: it then allocates nothing.
+ * Under capture a call takes the kernels that need no scratch beyond those
+ * buffers, slower at small sizes; forces and strict stresses keep their bits. */
 int ddd_segseg_force_device(ddd_ctx* ctx, const ddd_consts* k, const double* segs, int64_t ldSegs,
                             const uint8_t* ext, int64_t numSeg, double* force, void* stream, ddd_report* rep);
 int ddd_sigma_tilde_device(ddd_ctx* ctx, const ddd_consts* k, const double* x0, int64_t numPoints,
