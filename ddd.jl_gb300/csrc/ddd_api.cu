@@ -180,16 +180,6 @@ cudaError_t run_segseg_all(ddd_ctx* c, const ddd::KConsts& K, const double* soa,
                                                          x.p);
 }
 
-// Index rows per launch: all of them when their partial sums (6 doubles per row
-// and column block) fit in the context's limit, else as many as do, at least one
-// tile's worth.  Rows are independent, so chunking changes no bit of the result.
-int64_t rows_per_chunk(const ddd_ctx* c, const ddd::RowPlan& plan, int64_t nRows) {
-  const int64_t tile = ddd::strict::segseg_npad(1);
-  const int64_t fit = partial_limit(c) / (int64_t)ddd::row_partial_bytes(plan, 1);
-  const int64_t chunk = fit < tile ? tile : fit;
-  return chunk < nRows ? chunk : nRows;
-}
-
 cudaError_t run_segseg_rows(ddd_ctx* c, const ddd::KConsts& K, const double* soa, const uint8_t* skip, int64_t npad,
                             const int64_t* rows, int64_t nRows, const ddd::RowPlan& plan, double* partial, double* out,
                             unsigned long long* cnt, cudaStream_t st) {
@@ -197,7 +187,7 @@ cudaError_t run_segseg_rows(ddd_ctx* c, const ddd::KConsts& K, const double* soa
     cudaError_t e = prep_df_if_needed(c, npad, st);
     if (e != cudaSuccess) return e;
   }
-  const int64_t chunk = rows_per_chunk(c, plan, nRows);
+  const int64_t chunk = ddd::rows_per_chunk(plan, nRows, partial_limit(c));
   for (int64_t r0 = 0; r0 < nRows; r0 += chunk) {
     const int64_t n = nRows - r0 < chunk ? nRows - r0 : chunk;
     const int64_t* r = rows + r0;
@@ -420,7 +410,7 @@ int segseg_compute(ddd_ctx* ctx, const ddd_consts* k, const double* coord, int64
     if ((rc = send(ctx, ctx->rows, u, "copy idx"))) return rc;
     h2d += nIdx * (int64_t)sizeof(int64_t);
     const ddd::RowPlan plan = ddd::row_plan(npad, nIdx);
-    CK(ctx->partial.ensure(ddd::row_partial_bytes(plan, rows_per_chunk(ctx, plan, nIdx))), "alloc partial sums");
+    CK(ctx->partial.ensure(ddd::row_partial_bytes(plan, ddd::rows_per_chunk(plan, nIdx, partial_limit(ctx)))), "alloc partial sums");
     CK(cudaEventRecord(ctx->ev[1], ctx->stream), "event");
     CK(run_segseg_rows(ctx, K, ctx->soa.as<double>(), ctx->skip.as<uint8_t>(), npad, ctx->rows.as<int64_t>(),
                        nIdx, plan, ctx->partial.as<double>(), ctx->out.as<double>(), dCnt, ctx->stream),

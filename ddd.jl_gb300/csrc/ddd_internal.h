@@ -56,6 +56,17 @@ inline RowPlan row_plan(int64_t npad, int64_t nRows) {
   return RowPlan{(npad + 128 * m - 1) / (128 * m), m};
 }
 inline size_t row_partial_bytes(const RowPlan& p, int64_t nRows) { return (size_t)(nRows * p.nBlk) * 6 * sizeof(double); }
+// Rows per launch: all of them when their partial sums fit in `limit` bytes, else as
+// many as do, at least 128; never more CTAs than a grid has (2^31 - 1: 2,000,000
+// rows of as many segments would be 3.9e9).  Rows are independent, so chunking
+// changes no bit of the result.
+inline int64_t rows_per_chunk(const RowPlan& p, int64_t nRows, int64_t limit) {
+  int64_t n = limit / (int64_t)row_partial_bytes(p, 1);
+  if (n < 128) n = 128;
+  const int64_t grid = INT32_MAX / p.nBlk;
+  if (n > grid) n = grid;
+  return n < nRows ? n : nRows;
+}
 
 // Expanded all-pairs (segseg_small.cuh): every pair's twelve components, class and
 // list entry stored, 128 x 128 positions per tile pair, at most 153 tile pairs at

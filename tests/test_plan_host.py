@@ -1,0 +1,45 @@
+"""The launch plans' arithmetic on a CPU (ddd_internal.h): what a kernel gets to index stays inside
+a grid, a buffer and a limit, also at sizes that no test can run."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    out = str(tmp_path_factory.mktemp("plan") / "libplan.so")
+    r = subprocess.run([cxx, "-O1", "-std=c++17", "-fPIC", "-shared", "-I", os.path.join(CUDA, "include"), "-I",
+                        os.path.join(ROOT, "ddd.jl_gb300", "csrc"), os.path.join(ROOT, "tests", "plan_host", "plan_host.cpp"),
+                        "-o", out], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    lib = ctypes.CDLL(out)
+
+    def call(name, n, *args):
+        o = np.zeros(n, np.int64)
+        getattr(lib, name)(*[ctypes.c_int64(int(a)) for a in args], o.ctypes.data_as(ctypes.c_void_p))
+        return [int(v) for v in o]
+
+    return call
+
+
+@pytest.mark.parametrize("n,rows,limit", [(1, 1, 0), (6001, 37, 0), (6001, 6001, 16 << 30), (2_000_000, 2_000_000, 200 << 30),
+                                          (16_000_000, 16_000_000, 1 << 40), (100_000, 3_000_000_000, 1 << 42)])
+def test_row_chunks(plan, n, rows, limit):
+    """A chunk's CTAs fit a grid, its partial sums the limit (or 128 rows), and every column has a block."""
+    npad = -(-n // 128) * 128
+    blocks, m, chunk = plan("plan_rows", 3, npad, rows, limit)
+    assert 1 <= m <= 8 and blocks * m * 128 >= npad > (blocks - 1) * m * 128
+    assert 1 <= chunk <= rows and chunk * blocks < 2 ** 31
+    assert chunk * blocks * 48 <= max(limit, 128 * blocks * 48)
+    assert chunk == rows or chunk >= 128 or (chunk + 1) * blocks >= 2 ** 31
