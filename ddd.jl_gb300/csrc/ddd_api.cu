@@ -218,13 +218,14 @@ cudaError_t run_sigma(ddd_ctx* c, const ddd::KConsts& K, const double* soa, int6
     if (use_fx(c)) return ddd::launch_sigma_fx(K, soa, npad, nSeg, x0, M, sigma, plan, scratch, st);
     return ddd::launch_sigma_mixed(K, c->soadf.as<float>(), npad, nSeg, x0, M, sigma, plan, scratch, st);
   }
-  if (M < ddd::kSigmaSplitPoints) {
-    const cudaError_t e = x.take(ddd::sigma_split_bytes(npad));
+  const int64_t chunk = ddd::sigma_split_chunk(nSeg, M);
+  if (chunk) {
+    const cudaError_t e = x.take(ddd::sigma_split_bytes(chunk, npad));
     if (e != cudaSuccess) return e;
   }
   double* scratch = static_cast<double*>(x.p);
-  return use_fma(c) ? ddd::fast::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, scratch, st)
-                    : ddd::strict::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, scratch, st);
+  return use_fma(c) ? ddd::fast::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, chunk, scratch, st)
+                    : ddd::strict::launch_sigma_f64(K, soa, npad, nSeg, x0, M, sigma, chunk, scratch, st);
 }
 
 

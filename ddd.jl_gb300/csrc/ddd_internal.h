@@ -102,11 +102,22 @@ inline size_t expand_bytes(int64_t nb) {
 
 // σ̃ with few points.  The literal FP64 kernels (strict, FMA) take sigma_split
 // (sigma_f64.cu) below kSigmaSplitPoints, where a thread per point leaves fewer
-// than ~5 warps per SM; its scratch is two stores of kSigmaChunk evaluations and
-// t x b.
+// than ~5 warps per SM; its scratch is two stores of one chunk's evaluations and
+// t x b.  A chunk is one launch: 2^19 evaluations (25 MB per store, 270 us), and as
+// many more as keep a call at kSigmaMostLaunches, since a caller waits once ~1,000
+// launches are queued and the device form promises not to.  Up to 2^23 (2^32
+// evaluations in all, 2 s); beyond, 0: the point kernel.
 constexpr int64_t kSigmaSplitPoints = 24576;
-constexpr int64_t kSigmaChunk = 1 << 19;
-inline size_t sigma_split_bytes(int64_t npad) { return (size_t)(12 * kSigmaChunk + 3 * npad) * sizeof(double); }
+constexpr int64_t kSigmaMostLaunches = 512;
+inline int64_t sigma_split_chunk(int64_t nSeg, int64_t M) {
+  if (M >= kSigmaSplitPoints) return 0;
+  for (int64_t chunk = 1 << 19; chunk <= 1 << 23; chunk *= 2) {
+    const int64_t step = chunk / M;  // segments
+    if ((nSeg + step - 1) / step < kSigmaMostLaunches) return chunk;
+  }
+  return 0;
+}
+inline size_t sigma_split_bytes(int64_t chunk, int64_t npad) { return (size_t)(12 * chunk + 3 * npad) * sizeof(double); }
 
 // The fast and the mixed form cut the segments into slices of whole tiles
 // (blockIdx.y) until the call has ~4 times the CTAs that are resident, and a warp
@@ -162,7 +173,7 @@ inline size_t sigma_part_bytes(const SigmaPlan& p, int64_t M) {
                                      const int64_t* rows, int64_t nRows, const RowPlan& plan, double* partial, \
                                      double* out, unsigned long long* counters, cudaStream_t st); \
   cudaError_t launch_sigma_f64(const KConsts& K, const double* soa, int64_t npad, int64_t nSeg, const double* x0, \
-                               int64_t M, double* sigma, double* scratch, cudaStream_t st); \
+                               int64_t M, double* sigma, int64_t chunk, double* scratch, cudaStream_t st); \
   cudaError_t launch_reduce_all(const double* partial, int64_t npad, int64_t numSeg, double* out, cudaStream_t st); \
   cudaError_t launch_reduce_band(const double* partial, int64_t J0, int64_t J1, int64_t numSeg, double* out, \
                                  cudaStream_t st); \

@@ -69,7 +69,7 @@ sigma_tilde_f64(KConsts K, const double* __restrict__ soa, int64_t npad, int64_t
 }
 
 // Fewer points than kSigmaSplitPoints: a thread per (segment, point) instead of
-// per point, segments in chunks of kSigmaChunk evaluations.  The contributions go
+// per point, segments in chunks of `chunk` evaluations (sigma_split_chunk).  The contributions go
 // to a store and are added to sigma in segment order by the first blocks of the
 // next chunk's launch, beside its evaluations (one DADD of a point's chain takes
 // 64 cycles, so a chunk's chain is ~1/10 of its evaluations' time), so every
@@ -83,13 +83,13 @@ sigma_tilde_f64(KConsts K, const double* __restrict__ soa, int64_t npad, int64_t
 __global__ void __launch_bounds__(SIG_TILE, 24)
 sigma_split(KConsts K, const double* __restrict__ soa, int64_t npad, const double* __restrict__ txb,
             const double* __restrict__ x0, unsigned M, unsigned addBlocks, const double* __restrict__ prev,
-            unsigned prevSegs, bool first, double* __restrict__ sigma, double* __restrict__ store, int64_t s0,
-            unsigned segs) {
+            unsigned prevSegs, bool first, double* __restrict__ sigma, double* __restrict__ store, int64_t chunk,
+            int64_t s0, unsigned segs) {
   if (blockIdx.x < addBlocks) {
     const unsigned q = blockIdx.x * SIG_TILE + threadIdx.x;
     if (q >= 6 * M) return;
     const unsigned c = q / M, j = q % M;
-    const double* p = prev + (int64_t)c * kSigmaChunk + j;
+    const double* p = prev + c * chunk + j;
     double acc = first ? 0.0 : sigma[6 * (int64_t)j + c];
 #pragma unroll 16
     for (unsigned s = 0; s < prevSegs; ++s) acc += p[s * M];
@@ -107,7 +107,7 @@ sigma_split(KConsts K, const double* __restrict__ soa, int64_t npad, const doubl
               D3{g[3 * npad], g[4 * npad], g[5 * npad]}, D3{g[9 * npad], g[10 * npad], g[11 * npad]},
               D3{tx[0], tx[npad], tx[2 * npad]}, D3{x[0], x[1], x[2]}, sig);
 #pragma unroll
-  for (int c = 0; c < 6; ++c) store[(int64_t)c * kSigmaChunk + e] = sig[c];
+  for (int c = 0; c < 6; ++c) store[c * chunk + e] = sig[c];
 }
 
 // t x b of every segment (3 x npad), as the point kernel forms it per tile.
@@ -122,7 +122,7 @@ __global__ void sigma_txb(const double* __restrict__ soa, int64_t npad, double* 
 }
 
 cudaError_t launch_sigma_f64(const KConsts& K, const double* soa, int64_t npad, int64_t nSeg, const double* x0,
-                             int64_t M, double* sigma, double* scratch, cudaStream_t st) {
+                             int64_t M, double* sigma, int64_t chunk, double* scratch, cudaStream_t st) {
   if (M == 0) return cudaSuccess;
   if (!scratch) {
     sigma_tilde_f64<<<(unsigned)((M + SIG_TILE - 1) / SIG_TILE), SIG_TILE, 0, st>>>(K, soa, npad, nSeg, x0, M, sigma);
@@ -132,19 +132,19 @@ cudaError_t launch_sigma_f64(const KConsts& K, const double* soa, int64_t npad, 
   static std::atomic<uint64_t> loaded{0};
   const cudaError_t le = set_smem_once(sigma_tilde_f64, 0, loaded);
   if (le != cudaSuccess) return le;
-  double* store[2] = {scratch, scratch + 6 * kSigmaChunk};
-  double* txb = scratch + 12 * kSigmaChunk;
+  double* store[2] = {scratch, scratch + 6 * chunk};
+  double* txb = scratch + 12 * chunk;
   sigma_txb<<<(unsigned)((npad + 255) / 256), 256, 0, st>>>(soa, npad, txb);
-  const int64_t step = kSigmaChunk / M;  // M < kSigmaSplitPoints <= kSigmaChunk
+  const int64_t step = chunk / M;
   const unsigned addBlocks = (unsigned)((6 * M + SIG_TILE - 1) / SIG_TILE);
   unsigned prevSegs = 0;
-  int chunk = 0;
-  for (int64_t s0 = 0; s0 < nSeg || prevSegs; s0 += step, ++chunk) {
+  int turn = 0;
+  for (int64_t s0 = 0; s0 < nSeg || prevSegs; s0 += step, ++turn) {
     const unsigned segs = s0 < nSeg ? (unsigned)(nSeg - s0 < step ? nSeg - s0 : step) : 0;
     const unsigned add = prevSegs ? addBlocks : 0;
     const unsigned eval = (unsigned)((segs * M + SIG_TILE - 1) / SIG_TILE);
-    sigma_split<<<add + eval, SIG_TILE, 0, st>>>(K, soa, npad, txb, x0, (unsigned)M, add, store[(chunk + 1) & 1],
-                                                 prevSegs, chunk == 1, sigma, store[chunk & 1], s0, segs);
+    sigma_split<<<add + eval, SIG_TILE, 0, st>>>(K, soa, npad, txb, x0, (unsigned)M, add, store[(turn + 1) & 1],
+                                                 prevSegs, turn == 1, sigma, store[turn & 1], chunk, s0, segs);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     prevSegs = segs;

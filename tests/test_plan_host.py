@@ -43,3 +43,20 @@ def test_row_chunks(plan, n, rows, limit):
     assert 1 <= chunk <= rows and chunk * blocks < 2 ** 31
     assert chunk * blocks * 48 <= max(limit, 128 * blocks * 48)
     assert chunk == rows or chunk >= 128 or (chunk + 1) * blocks >= 2 ** 31
+
+
+@pytest.mark.parametrize("nseg,points", [(1, 1), (4096, 613), (16384, 24575), (65536, 24575), (1_000_000, 1000),
+                                         (174_000, 24575), (1_000_000, 24575), (100_000_000, 1), (10 ** 10, 1)])
+def test_sigma_chunks(plan, nseg, points):
+    """At most 512 launches, each of at least one segment and indexed in 32 bits; 2^19 evaluations
+    where that many launches do, none (the point kernel) where 2^23 would not."""
+    chunk, scratch, most = plan("plan_sigma", 3, nseg, points)
+    assert points < most
+    if chunk:
+        step = chunk // points
+        assert step >= 1 and -(-nseg // step) + 1 <= 512 and 6 * chunk < 2 ** 31
+        assert chunk == 2 ** 19 or -(-nseg // (chunk // 2 // points)) + 1 > 512
+        assert scratch == 96 * chunk + 24 * (-(-nseg // 128) * 128)
+    else:
+        assert -(-nseg // (2 ** 23 // points)) + 1 > 512
+    assert plan("plan_sigma", 3, nseg, most)[0] == 0

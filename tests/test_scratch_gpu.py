@@ -110,3 +110,29 @@ def test_capture_after_a_larger_call(torch_, pkg, synth, mode, rel):
     torch.cuda.synchronize()
     for (out, _), cap in zip(calls, captured):
         assert torch.equal(out, cap)
+
+
+@pytest.mark.parametrize("nseg", [16384, 65536])
+def test_many_segments_few_points(torch_, pkg, synth, nseg):
+    """σ̃ just below the points that a thread each takes (24,575; chunks of 2^20 and 2^22 evaluations):
+    the bits of the kernel above that line, and the call returns while most of it is still to run."""
+    import time
+    torch = torch_
+    c = Calls(torch, pkg, synth, "fp64")
+    st = torch.cuda.Stream()
+    S, go = c.sigma(nseg, 24576)
+    x = torch.from_numpy(np.random.default_rng(1).uniform(0.0, CUBE, (24576, 3))).cuda()
+    segs = _segs(torch, synth, nseg, 1)
+    T = torch.zeros((24575, 6), dtype=torch.float64, device="cuda")
+    few = lambda: c.ctx.sigma_tilde_device(c.k, x.data_ptr(), 24575, segs.data_ptr(), nseg, nseg, T.data_ptr(),
+                                           stream=st.cuda_stream)
+    go(st)
+    few()
+    torch.cuda.synchronize()
+    assert torch.equal(S[:24575], T)
+    t0 = time.perf_counter()
+    few()
+    t1 = time.perf_counter()
+    torch.cuda.synchronize()
+    t2 = time.perf_counter()
+    assert t1 - t0 < 0.25 * (t2 - t0)
