@@ -158,15 +158,16 @@ cudaError_t run_segseg_all(ddd_ctx* c, const ddd::KConsts& K, const double* soa,
     if (e != cudaSuccess) return e;
   }
   // Small networks, and the tile pairs beyond the last full wave of the tile
-  // kernel: one warp per 32 pairs, the pair values stored and folded.  The store
-  // obeys the partial-sum limit too; without it (limit, no memory) the tile kernel
-  // takes all, with the same bits.
+  // kernel: one warp per 32 pairs, the pair values stored and folded.  The store and
+  // the slots together obey the partial-sum limit; without it (limit, no memory,
+  // capture) the tile kernel takes all, with the same bits.
   const int64_t nt = npad / ddd::strict::segseg_npad(1), nb = nt * (nt + 1) / 2;
   const ddd::ExpandRule& rule = use_df(c) ? (df_form(c) ? ddd::kExpandMixed : ddd::kExpandDF)
                                 : use_fx(c) ? ddd::kExpandFx : ddd::kExpandF64;
   int64_t from = use_fma(c) ? nb : ddd::expand_from(nb, rule);
   Expand x(c, st);
-  if (cap >= nb && from < nb && (int64_t)ddd::expand_bytes(nb - from) <= partial_limit(c)) {
+  if (cap >= nb && from < nb &&
+      ddd::scratch_fits(ddd::expand_bytes(nb - from), partial_bytes(c, npad), partial_limit(c))) {
     const cudaError_t e = x.take(ddd::expand_bytes(nb - from));
     if (e != cudaSuccess) return e;
   }
@@ -211,7 +212,7 @@ cudaError_t run_sigma(ddd_ctx* c, const ddd::KConsts& K, const double* soa, int6
     ddd::SigmaPlan plan = use_df(c) ? ddd::sigma_plan(nSeg, M, 128, 1216) : ddd::sigma_plan(nSeg, M, 32, 3648);
     const size_t bytes = ddd::sigma_part_bytes(plan, M);
     cudaError_t e = prep_df_if_needed(c, npad, st);  // both precision modes: the mixed σ̃ form
-    if (e == cudaSuccess && bytes) e = x.take(bytes);
+    if (e == cudaSuccess && bytes && ddd::scratch_fits(bytes, 0, partial_limit(c))) e = x.take(bytes);
     if (e != cudaSuccess) return e;
     double* scratch = static_cast<double*>(x.p);
     if (!scratch) plan = ddd::SigmaPlan{1, 1, npad};
@@ -219,7 +220,7 @@ cudaError_t run_sigma(ddd_ctx* c, const ddd::KConsts& K, const double* soa, int6
     return ddd::launch_sigma_mixed(K, c->soadf.as<float>(), npad, nSeg, x0, M, sigma, plan, scratch, st);
   }
   const int64_t chunk = ddd::sigma_split_chunk(nSeg, M);
-  if (chunk) {
+  if (chunk && ddd::scratch_fits(ddd::sigma_split_bytes(chunk, npad), 0, partial_limit(c))) {
     const cudaError_t e = x.take(ddd::sigma_split_bytes(chunk, npad));
     if (e != cudaSuccess) return e;
   }

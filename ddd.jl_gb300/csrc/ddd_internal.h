@@ -70,7 +70,7 @@ inline int64_t rows_per_chunk(const RowPlan& p, int64_t nRows, int64_t limit) {
 
 // Expanded all-pairs (segseg_small.cuh): every pair's twelve components, class and
 // list entry stored, 128 x 128 positions per tile pair, at most 153 tile pairs at
-// a time (252 MB).  It takes networks of up to 153 tile pairs (2,176 segments)
+// a time (253 MB; 285 MB as GrowBuf allocates).  It takes networks of up to 153 tile pairs (2,176 segments)
 // whole, and of larger ones the tile pairs beyond the last full wave of the tile
 // kernel (304 CTAs), which that kernel would run on part of the GPU: `most`
 // less `perWave` for each full wave, while there are at most `waves`.  Beyond, the
@@ -276,10 +276,12 @@ cudaError_t launch_minimum_distance(const double* pts, int64_t n, double* out, c
 struct GrowBuf {
   void* p = nullptr;
   size_t cap = 0;
+  // What a request for `bytes` allocates.
+  static size_t grown(size_t bytes) { return bytes + bytes / 8 + 256; }
   cudaError_t ensure(size_t bytes) {
     if (bytes <= cap) return cudaSuccess;
     release();
-    const size_t want = bytes + bytes / 8 + 256;
+    const size_t want = grown(bytes);
     cudaError_t e = cudaMalloc(&p, want);
     if (e != cudaSuccess) {
       p = nullptr;
@@ -299,6 +301,12 @@ struct GrowBuf {
   GrowBuf& operator=(const GrowBuf&) = delete;
   ~GrowBuf() { release(); }
 };
+
+// Whether a call whose partial sums take `partial` bytes may have `bytes` of scratch
+// beside them under the context's partial-sum limit, both as allocated.
+inline bool scratch_fits(size_t bytes, size_t partial, int64_t limit) {
+  return GrowBuf::grown(bytes) + (partial ? GrowBuf::grown(partial) : 0) <= (size_t)limit;
+}
 
 // u_tilde.cu: calc_uTilde's displacements at numPoints points (u: host, 3 x
 // numPoints).  The host arrays drive the segment pass; the *Dev copies feed the

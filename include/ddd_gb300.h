@@ -379,9 +379,13 @@ int ddd_get_mode(const ddd_ctx* ctx);
  * rounding.  The idx forms keep 6 doubles per row of idx and block of 128 to
  * 1,024 columns; past the limit their rows run in chunks (of at least 128), with
  * results unchanged bit for bit.  Networks of up to ~9,300 segments also store the
- * pair forces of some tile pairs (at most 252 MB); when that store is past the
- * limit, or does not fit the device, it is left out, with the same bits.  No
- * reference counterpart (the reference allocates per call).
+ * pair forces of some tile pairs (up to 285 MB of device memory): only when the
+ * store and the partial sums fit the limit together, and the device, else it is
+ * left out, with the same bits.  The field stress at few points keeps partial
+ * stresses in the same buffer (57 MB, and up to 0.9 GB past 268 million
+ * point-segment pairs), only within the limit as well.  The context keeps its
+ * buffers, at the largest size so far, until ddd_destroy.  No reference counterpart (the
+ * reference allocates per call).
  * ddd_get_partial_limit returns the limit in force. */
 int ddd_set_partial_limit(ddd_ctx* ctx, int64_t bytes);
 int64_t ddd_get_partial_limit(const ddd_ctx* ctx);

@@ -19,9 +19,11 @@ def plan(tmp_path_factory):
     if cxx is None:
         pytest.skip("no C++ compiler")
     out = str(tmp_path_factory.mktemp("plan") / "libplan.so")
-    r = subprocess.run([cxx, "-O1", "-std=c++17", "-fPIC", "-shared", "-I", os.path.join(CUDA, "include"), "-I",
-                        os.path.join(ROOT, "ddd.jl_gb300", "csrc"), os.path.join(ROOT, "tests", "plan_host", "plan_host.cpp"),
-                        "-o", out], capture_output=True, text=True)
+    # -Bsymbolic: the counting cudaMalloc stays its own beside a loaded CUDA runtime.
+    cmd = [cxx, "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", os.path.join(CUDA, "include"),
+           "-I", os.path.join(ROOT, "ddd.jl_gb300", "csrc"),
+           os.path.join(ROOT, "tests", "plan_host", "plan_host.cpp"), "-o", out]
+    r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     lib = ctypes.CDLL(out)
 
@@ -33,8 +35,8 @@ def plan(tmp_path_factory):
     return call
 
 
-@pytest.mark.parametrize("n,rows,limit", [(1, 1, 0), (6001, 37, 0), (6001, 6001, 16 << 30), (2_000_000, 2_000_000, 200 << 30),
-                                          (16_000_000, 16_000_000, 1 << 40), (100_000, 3_000_000_000, 1 << 42)])
+@pytest.mark.parametrize("n,rows,limit", [(1, 1, 0), (6001, 37, 0), (6001, 6001, 16 << 30),
+                                          (2_000_000, 2_000_000, 200 << 30), (16_000_000, 16_000_000, 1 << 40), (100_000, 3_000_000_000, 1 << 42)])
 def test_row_chunks(plan, n, rows, limit):
     """A chunk's CTAs fit a grid, its partial sums the limit (or 128 rows), and every column has a block."""
     npad = -(-n // 128) * 128
@@ -60,3 +62,13 @@ def test_sigma_chunks(plan, nseg, points):
     else:
         assert -(-nseg // (2 ** 23 // points)) + 1 > 512
     assert plan("plan_sigma", 3, nseg, most)[0] == 0
+
+
+@pytest.mark.parametrize("nb", [1, 10, 153, 253])
+def test_store_and_limit(plan, nb):
+    """The pair store is taken only when all that the call allocates for it and for the partial sums
+    is within the limit; the largest is 285 MB."""
+    held = plan("plan_store", 2, nb, nb, 0)[0]
+    assert plan("plan_store", 2, nb, nb, held)[1] == 1
+    assert plan("plan_store", 2, nb, nb, held - 1)[1] == 0
+    assert plan("plan_store", 2, nb, 0, 2 ** 40)[0] <= 285_000_000

@@ -136,3 +136,19 @@ def test_many_segments_few_points(torch_, pkg, synth, nseg):
     torch.cuda.synchronize()
     t2 = time.perf_counter()
     assert t1 - t0 < 0.25 * (t2 - t0)
+
+
+@pytest.mark.parametrize("mode", ["fp64", "fp64_fast", "f32c"])
+def test_stress_without_scratch(torch_, pkg, synth, mode):
+    """Under a limit that no scratch fits, σ̃ of few points is what the same points give in a call
+    with a thread each: the bits of the kernel without slices."""
+    torch = torch_
+    c = Calls(torch, pkg, synth, mode)
+    c.ctx.partial_limit = 1
+    st = torch.cuda.Stream()
+    S, go = c.sigma(1000, 700000)
+    T, few = c.sigma(1000, 700)
+    go(st)
+    few(st)
+    torch.cuda.synchronize()
+    assert torch.equal(S[:700], T)
