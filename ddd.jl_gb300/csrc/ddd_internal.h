@@ -41,21 +41,24 @@ cudaError_t set_smem_once(Kernel* kernel, int bytes, std::atomic<uint64_t>& done
   return e;
 }
 
-// Index rows (segseg_small.cuh): a row's columns in nBlk blocks of 128 m, one
-// CTA each.  m grows from 1 to 8 with the work so that a call has ~1,216 CTAs
-// (four rounds of the 304 that are resident) before a CTA takes more steps; it
-// depends on the call's whole row count, so that chunks of rows change no sum.
-constexpr int kRowMaxSteps = 8;
+// Index rows (segseg_small.cuh): a row's columns in nBlk blocks of `threads` m, one
+// CTA each (segseg_small.cuh says why df64's is larger).  m grows from 1 to 8 with the work so
+// that a call has ~four rounds of resident CTAs (1,216 of 128 threads) before a CTA
+// takes more steps; it depends on the call's whole row count, so that chunks of rows
+// change no sum.
+constexpr int kRowMaxSteps = 8, kRowThreads = 128, kRowThreadsDF64 = 256;
 struct RowPlan {
   int64_t nBlk;
   int m;
 };
-inline RowPlan row_plan(int64_t npad, int64_t nRows) {
+inline RowPlan row_plan(int64_t npad, int64_t nRows, int threads) {
   const int64_t q = nRows * (npad / 128) / 1216;
   const int m = q < 1 ? 1 : q > kRowMaxSteps ? kRowMaxSteps : (int)q;
-  return RowPlan{(npad + 128 * m - 1) / (128 * m), m};
+  return RowPlan{(npad + threads * m - 1) / (threads * m), m};
 }
-inline size_t row_partial_bytes(const RowPlan& p, int64_t nRows) { return (size_t)(nRows * p.nBlk) * 6 * sizeof(double); }
+inline size_t row_partial_bytes(const RowPlan& p, int64_t nRows) {
+  return (size_t)(nRows * p.nBlk) * 6 * sizeof(double);
+}
 // Rows per launch: all of them when their partial sums fit in `limit` bytes, else as
 // many as do, at least 128; never more CTAs than a grid has (2^31 - 1: 2,000,000
 // rows of as many segments would be 3.9e9).  Rows are independent, so chunking

@@ -264,27 +264,32 @@ cudaError_t launch_expanded(const TileArgs& A, const typename P::Consts& KP, int
 
 // ---------------------------------------------------------------------------
 // Index rows (calcSegSegForce(..., idx), DislocationForces.jl:831-877): one CTA
-// takes one row segment against 128 m columns, one column per thread and step,
-// so no lane idles however few rows there are (the earlier tile form held one
+// takes one row segment against m columns per thread, one column per thread and
+// step, so no lane idles however few rows there are (the earlier tile form held one
 // row per thread: 37 rows kept 37 of 128 lanes busy for 128 steps).
 // Near-parallel columns are listed in shared memory (column order) and evaluated
 // after the sweep: with ~5 % of the columns near-parallel, most CTAs have one
 // warp's worth of them, where a list per warp would make every warp run both
 // branches.  (37 rows x 6,001 segments: 570 us; one-warp CTAs of 128 columns, each
-// with its list, 654.)  The threads' sums are added in a fixed tree; x_reduce_rows adds a
-// row's blocks in a fixed order.
-constexpr int kRowThreads = 128;
-
+// with its list, 654.)  The threads' sums are added in a fixed tree; x_reduce_rows
+// adds a row's blocks in a fixed order.
+//
+// df64 takes one CTA of 256 threads per SM: its pair is ~10,000 instructions, several
+// times what an SM holds, and two CTAs at different places of it fetched them twice
+// (ncu: 1.3 instructions per cycle, half the warps' cycles without one).  The step's
+// barriers keep the eight warps together.  6,001 segments: 1,500 rows 7.18 -> 4.97
+// ms, 6,001 rows 28.5 -> 19.6, where a row per thread had taken 6.4 and 20.2.  The
+// other forms lose 2 to 8 % so.
 template <class P>
-__global__ void __launch_bounds__(kRowThreads, 2)
+__global__ void __launch_bounds__(P::kRowCta, 256 / P::kRowCta)
 x_rows(TileArgs A, typename P::Consts KP, const int64_t* __restrict__ rows, int64_t nBlk, int m,
        double* __restrict__ partial, unsigned long long* __restrict__ counters) {
-  constexpr int NW = kRowThreads / 32;
-  __shared__ uint16_t list[kRowThreads * kRowMaxSteps];
+  constexpr int CT = P::kRowCta, NW = CT / 32;
+  __shared__ uint16_t list[CT * kRowMaxSteps];
   __shared__ int cnt[NW];
   __shared__ double red[NW][6];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t r = blockIdx.x / nBlk, j0 = (blockIdx.x % nBlk) * kRowThreads * m;
+  const int64_t r = blockIdx.x / nBlk, j0 = (blockIdx.x % nBlk) * CT * m;
   const int64_t gi = rows[r];
   typename P::Acc f1 = P::acc_zero(), f2 = P::acc_zero();
   D3 p1 = {0, 0, 0}, p2 = {0, 0, 0};
@@ -293,7 +298,7 @@ x_rows(TileArgs A, typename P::Consts KP, const int64_t* __restrict__ rows, int6
   if (A.skip[gi] == 0) {
     const typename P::Seg a = P::load_global(A, gi);
     for (int q = 0; q < m; ++q) {
-      const int64_t j = j0 + q * kRowThreads + tid;
+      const int64_t j = j0 + q * CT + tid;
       bool par = false;
       if (j < A.npad && A.skip[j] == 0 && j != gi) {
         const typename P::Seg s = P::load_global(A, j);
@@ -317,12 +322,12 @@ x_rows(TileArgs A, typename P::Consts KP, const int64_t* __restrict__ rows, int6
         if (w < warp) at += cnt[w];
         nPar += cnt[w];
       }
-      if (par) list[at + __popc(mask & ((1u << lane) - 1))] = (uint16_t)(q * kRowThreads + tid);
+      if (par) list[at + __popc(mask & ((1u << lane) - 1))] = (uint16_t)(q * CT + tid);
       __syncthreads();
     }
     if (tid < nPar) {
       const SegF64 b = tb_load_seg64(A.soa, A.npad, gi);
-      for (int e = tid; e < nPar; e += kRowThreads) {
+      for (int e = tid; e < nPar; e += CT) {
         const SegF64 s = tb_load_seg64(A.soa, A.npad, j0 + list[e]);
         D3 F1, F2;
         nCore += parallel_pair_side<1>(A.K, b, s, F1, F2);
@@ -387,7 +392,7 @@ template <class P>
 cudaError_t launch_rows(const TileArgs& A, const typename P::Consts& KP, const int64_t* rows, int64_t nRows,
                         const RowPlan& plan, double* partial, double* out, unsigned long long* counters,
                         cudaStream_t st) {
-  x_rows<P><<<(unsigned)(nRows * plan.nBlk), kRowThreads, 0, st>>>(A, KP, rows, plan.nBlk, plan.m, partial, counters);
+  x_rows<P><<<(unsigned)(nRows * plan.nBlk), P::kRowCta, 0, st>>>(A, KP, rows, plan.nBlk, plan.m, partial, counters);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   x_reduce_rows<<<(unsigned)((nRows + 3) / 4), 128, 0, st>>>(partial, plan.nBlk, nRows, out);

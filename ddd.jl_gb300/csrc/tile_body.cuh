@@ -377,6 +377,7 @@ struct PolF64 {
     c = dot(a.t, b.t);
     return 1.0 - c * c > kSqrtEps;
   }
+  static constexpr int kRowCta = 128;  // threads per CTA of x_rows (ddd_internal.h's kRowThreads)
   // QUAD: four lanes per pair (pair_f64.cuh), for the policies that have it.
   static constexpr bool kQuad = true;
   template <bool BOTH, bool QUAD = false>

@@ -377,7 +377,7 @@ int ddd_get_mode(const ddd_ctx* ctx);
  * column, nt slots), each band's sums added to the output in band order: the
  * same deterministic result on every call, equal to the unbanded one to
  * rounding.  The idx forms keep 6 doubles per row of idx and block of 128 to
- * 1,024 columns; past the limit their rows run in chunks (of at least 128), with
+ * 2,048 columns; past the limit their rows run in chunks (of at least 128), with
  * results unchanged bit for bit.  Networks of up to ~9,300 segments also store the
  * pair forces of some tile pairs (up to 285 MB of device memory): only when the
  * store and the partial sums fit the limit together, and the device, else it is

@@ -14,8 +14,8 @@ using namespace ddd;
 
 extern "C" {
 // The row plan of a call: column blocks, steps per CTA, rows per launch.
-void plan_rows(int64_t npad, int64_t nRows, int64_t limit, int64_t* out) {
-  const RowPlan p = row_plan(npad, nRows);
+void plan_rows(int64_t npad, int64_t nRows, int64_t limit, int64_t threads, int64_t* out) {
+  const RowPlan p = row_plan(npad, nRows, (int)threads);
   out[0] = p.nBlk;
   out[1] = p.m;
   out[2] = rows_per_chunk(p, nRows, limit);
