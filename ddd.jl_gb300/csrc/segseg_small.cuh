@@ -145,11 +145,11 @@ __device__ __forceinline__ void all_loaded(double* x) {
 // The slot of tile pair blockIdx.x / 12, component blockIdx.x % 12, from the
 // stored pairs, in the tile kernel's order: a row segment's general pairs by
 // step, then its near-parallel ones by step; a column segment's general pairs
-// warp of rows by warp, by step within one, its near-parallel ones by row
-// within one.  The loads of a batch of steps are in flight together and do not
-// wait for the classes (a position without a pair holds anything and is not
-// added): 30 us at one tile pair became 12.  Only the first `live` rows and
-// columns can hold pairs when there is one tile.
+// warp of rows by warp, by step within one, its near-parallel ones by row.  The
+// loads of a batch of steps are in flight together and do not wait for the classes
+// (a position without a pair holds anything and is not added): 30 us at one tile
+// pair became 12.  Only the first `live` rows and columns can hold pairs when there
+// is one tile.
 template <class P>
 __global__ void __launch_bounds__(XT)
 x_fold(const double* __restrict__ vals, const uint8_t* __restrict__ flags, int live, double* __restrict__ partial) {
@@ -181,10 +181,9 @@ x_fold(const double* __restrict__ vals, const uint8_t* __restrict__ flags, int l
     }
     r = P::comp_to_double(acc) + fp;
   } else {
-    double col = 0.0, tot = 0.0;
+    double col = 0.0, fp = 0.0;
     for (int w = 0; 32 * w < live; ++w) {
       Comp s = P::comp_zero();
-      double fp = 0.0;
       for (int q0 = 0; q0 < 32; q0 += NB) {
         double x[NB], y[NB];
         int cx[NB], cy[NB];
@@ -208,9 +207,8 @@ x_fold(const double* __restrict__ vals, const uint8_t* __restrict__ flags, int l
         }
       }
       col = w == 0 ? P::comp_to_double(s) : col + P::comp_to_double(s);
-      tot = tot + fp;
     }
-    r = col + tot;
+    r = col + fp;
   }
   partial[(b * 12 + c) * XT + t] = r;
 }

@@ -13,9 +13,8 @@
 // step) and evaluated densely, T at a time, with the FP64 calcParSegSegForce.
 // The block's partial forces — 6 per row segment, 6 per column segment — are
 // written to `p` as [side][component][T] doubles.  A column segment's
-// near-parallel forces are summed warp of rows by warp of rows, then over the
-// warps (segseg_small.cuh adds in the same order).  No floating-point atomics:
-// the result is deterministic.
+// near-parallel forces are summed by row (segseg_small.cuh adds in the same order).
+// No floating-point atomics: the result is deterministic.
 //
 // In MODE 2 every selected pair goes through the compacted dense pass.  The
 // sweep takes the reference's FP64 branch decision for each selected pair and
@@ -216,16 +215,6 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
   __syncthreads();
   const int nPar = sm.total;
   D3 fp1 = {0, 0, 0}, fp2 = {0, 0, 0}, fjp3 = {0, 0, 0}, fjp4 = {0, 0, 0};
-  // MODE 0: column sums of the warps before jw, apart so that segseg_small.cuh can
-  // add in the same order.  The FMA build has no such path and keeps one sum: the
-  // second cost it 1 % (65,536 segments 4,602 -> 4,636 ms).
-#ifdef DDD_FMA
-  constexpr bool byWarp = false;
-#else
-  constexpr bool byWarp = !CLS;
-#endif
-  D3 fjt3 = {0, 0, 0}, fjt4 = {0, 0, 0};
-  int jw = 0;
   unsigned long long nCore = 0;
   // Chunks of CH never straddle the two runs, so a warp runs one branch.
   for (int base = 0; base < nPar;) {
@@ -267,14 +256,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
       }
     }
     for (int q = 0; q < lim; ++q) {
-      const int pe = sm.plist[base + q];
-      if ((pe & 0xff) == t) {
-        if (byWarp && (pe >> 13) != jw) {  // the rows of the next warp
-          fjt3 = fjt3 + fjp3;
-          fjt4 = fjt4 + fjp4;
-          fjp3 = fjp4 = {0, 0, 0};
-          jw = pe >> 13;
-        }
+      if ((sm.plist[base + q] & 0xff) == t) {
         const double* f = sm.cf[q];
         fjp3 = fjp3 + D3{f[6], f[7], f[8]};
         fjp4 = fjp4 + D3{f[9], f[10], f[11]};
@@ -312,9 +294,7 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
   p[3 * T + t] = r2.x + fp2.x;
   p[4 * T + t] = r2.y + fp2.y;
   p[5 * T + t] = r2.z + fp2.z;
-  fjt3 = byWarp ? fjt3 + fjp3 : fjp3;
-  fjt4 = byWarp ? fjt4 + fjp4 : fjp4;
-  const double add[6] = {fjt3.x, fjt3.y, fjt3.z, fjt4.x, fjt4.y, fjt4.z};
+  const double add[6] = {fjp3.x, fjp3.y, fjp3.z, fjp4.x, fjp4.y, fjp4.z};
 #pragma unroll
   for (int c = 0; c < 6; ++c) p[(6 + c) * T + t] = P::template col_sum<T>(sm.pol, c, t) + add[c];
 
