@@ -255,9 +255,16 @@ __device__ __forceinline__ void tile_body(const TileArgs& A, const typename P::C
         fp2 = fp2 + D3{f[3], f[4], f[5]};
       }
     }
-    for (int q = 0; q < lim; ++q) {
-      if ((sm.plist[base + q] & 0xff) == t) {
-        const double* f = sm.cf[q];
+    // The chunk's entries on this thread's column, in order.  Found first, 32 at a time:
+    // as a condition on each sum, the compiler predicates the six additions and the warp
+    // issues them for every entry (2,900 segments on one slip system, fast FP64: 14.1 ms
+    // against 12.8).
+    for (int q0 = 0; q0 < lim; q0 += 32) {
+      uint32_t hit = 0;
+      for (int q = 0; q < 32 && q0 + q < lim; ++q)
+        hit |= (uint32_t)((sm.plist[base + q0 + q] & 0xff) == t) << q;
+      for (; hit; hit &= hit - 1) {
+        const double* f = sm.cf[q0 + __ffs(hit) - 1];
         fjp3 = fjp3 + D3{f[6], f[7], f[8]};
         fjp4 = fjp4 + D3{f[9], f[10], f[11]};
       }
