@@ -78,18 +78,22 @@ inline int64_t rows_per_chunk(const RowPlan& p, int64_t nRows, int64_t limit) {
 // kernel (304 CTAs), which that kernel would run on part of the GPU: `most`
 // less `perWave` for each full wave, while there are at most `waves`.  Beyond, the
 // CTAs' drift has filled the last wave, and the FP32-heavy forms pay for the
-// store.  Measured, with against without, tile pairs as waves * 304 + rest:
-//   strict   0+171 7.93 / 14.02 ms, 1+47 17.1 / 26.9, 2+212 39.6 / 42.6, 8+53 120.9 / 123.1
-//   fast     0+171 5.02 / 8.35, 1+47 10.3 / 15.9, 8+53 71.0 / 72.6; at 1+291 17.4 / 17.2
-//   df64     0+171 3.05 / 4.48, 1+224 8.93 / 9.40, 4+162 22.3 / 23.0; at 5+191 28.0 / 27.7
-//   f32c     0+171 1.72 / 2.34, 1+102 3.63 / 3.78; at 0+276 2.70 / 2.55, 1+224 4.89 / 4.64
+// store.  Measured in ms, with against without, tile pairs as waves * 304 +
+// rest, on 12 slip systems (5 % near-parallel pairs) and on one (37 %):
+//   strict   0+171 7.97 / 13.8 and 9.32 / 16.3, 1+47 16.8 / 26.5 and 20.4 / 31.2,
+//            2+212 39.2 / 42.4, 4+269 71.0 / 72.1, 8+53 118.5 / 121.2
+//   fast     0+171 5.05 / 8.13, 1+47 9.93 / 15.5, 1+224 15.2 / 16.5, 8+53 69.0 / 70.7
+//   df64     0+171 3.05 / 4.33, 0+231 4.08 / 4.39, 1+47 5.46 / 8.36, 1+224 8.59 / 9.10
+//   f32c     0+171 1.72 / 2.18 and 3.31 / 5.17, 0+231 2.27 / 2.29, 1+47 2.98 / 3.40 and
+//            6.83 / 9.44; left out: 1+102 3.43 / 3.47, and 6.60 / 5.62 where nine loops
+//            in ten have a near-parallel neighbour
 constexpr int64_t kExpandMaxPairs = 153;
 constexpr int64_t kTileWave = 304;
 struct ExpandRule {
   int waves, most, perWave;
 };
 constexpr ExpandRule kExpandF64 = {8, 304, 0}, kExpandFx = {8, 264, 0}, kExpandDF = {4, 240, 16},
-                     kExpandMixed = {1, 240, 128};
+                     kExpandMixed = {1, 240, 192};
 // The first tile pair that goes to the expanded kernels.  Not for the FMA form:
 // where the others give the tile kernel's bits, the compiler contracts its
 // near-parallel branch differently in each kernel, and through that branch's
