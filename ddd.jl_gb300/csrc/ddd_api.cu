@@ -411,8 +411,7 @@ int segseg_compute(ddd_ctx* ctx, const ddd_consts* k, const double* coord, int64
     u.add(rows0.data(), (size_t)nIdx * sizeof(int64_t));
     if ((rc = send(ctx, ctx->rows, u, "copy idx"))) return rc;
     h2d += nIdx * (int64_t)sizeof(int64_t);
-    const ddd::RowPlan plan =
-        ddd::row_plan(npad, nIdx, ctx->mode == DDD_MODE_DF64 ? ddd::kRowThreadsDF64 : ddd::kRowThreads);
+    const ddd::RowPlan plan = ddd::row_plan(npad, nIdx, ctx->mode == DDD_MODE_DF64);
     const int64_t rowChunk = ddd::rows_per_chunk(plan, nIdx, partial_limit(ctx));
     CK(ctx->partial.ensure(ddd::row_partial_bytes(plan, rowChunk)), "alloc partial sums");
     CK(cudaEventRecord(ctx->ev[1], ctx->stream), "event");

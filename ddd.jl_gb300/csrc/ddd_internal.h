@@ -42,19 +42,21 @@ cudaError_t set_smem_once(Kernel* kernel, int bytes, std::atomic<uint64_t>& done
 }
 
 // Index rows (segseg_small.cuh): a row's columns in nBlk blocks of `threads` m, one
-// CTA each (segseg_small.cuh says why df64's is larger).  m grows from 1 to 8 with the work so
-// that a call has ~four rounds of resident CTAs (1,216 of 128 threads) before a CTA
-// takes more steps; it depends on the call's whole row count, so that chunks of rows
-// change no sum.
-constexpr int kRowMaxSteps = 8, kRowThreads = 128, kRowThreadsDF64 = 256;
+// CTA each.  m grows from 1 to 8 with the work so that a call has ~four rounds of
+// resident CTAs (1,216 of 128 threads) before a CTA takes more steps; it depends on
+// the call's whole row count, so that chunks of rows change no sum.  df64 takes CTAs
+// of 256 threads from m = 4 on (segseg_small.cuh says why; below, the finer cut wins:
+// 64 rows of 2,900 segments on one slip system 330 against 378 us).
+constexpr int kRowMaxSteps = 8;
 struct RowPlan {
   int64_t nBlk;
-  int m;
+  int m, threads;
 };
-inline RowPlan row_plan(int64_t npad, int64_t nRows, int threads) {
+inline RowPlan row_plan(int64_t npad, int64_t nRows, bool df64) {
   const int64_t q = nRows * (npad / 128) / 1216;
   const int m = q < 1 ? 1 : q > kRowMaxSteps ? kRowMaxSteps : (int)q;
-  return RowPlan{(npad + threads * m - 1) / (threads * m), m};
+  const int threads = df64 && m >= 4 ? 256 : 128;
+  return RowPlan{(npad + threads * m - 1) / (threads * m), m, threads};
 }
 inline size_t row_partial_bytes(const RowPlan& p, int64_t nRows) {
   return (size_t)(nRows * p.nBlk) * 6 * sizeof(double);

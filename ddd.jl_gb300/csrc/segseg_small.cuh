@@ -272,17 +272,18 @@ cudaError_t launch_expanded(const TileArgs& A, const typename P::Consts& KP, int
 // with its list, 654.)  The threads' sums are added in a fixed tree; x_reduce_rows
 // adds a row's blocks in a fixed order.
 //
-// df64 takes one CTA of 256 threads per SM: its pair is ~10,000 instructions, several
-// times what an SM holds, and two CTAs at different places of it fetched them twice
-// (ncu: 1.3 instructions per cycle, half the warps' cycles without one).  The step's
-// barriers keep the eight warps together.  6,001 segments: 1,500 rows 7.18 -> 4.97
-// ms, 6,001 rows 28.5 -> 19.6, where a row per thread had taken 6.4 and 20.2.  The
-// other forms lose 2 to 8 % so.
-template <class P>
-__global__ void __launch_bounds__(P::kRowCta, 256 / P::kRowCta)
+// df64 takes one CTA of 256 threads per SM when a call has many rows: its pair is
+// ~10,000 instructions, several times what an SM holds, and two CTAs at different
+// places of it fetched them twice (ncu: 1.3 instructions per cycle, half the warps'
+// cycles without one).  The step's barriers keep the eight warps together.  6,001
+// segments: 150 rows 0.838 -> 0.687 ms, 1,500 rows 7.18 -> 4.97, 6,001 rows 28.7 ->
+// 19.5, where a row per thread had taken 2.5, 6.4 and 20.8.  The other forms lose 2 to
+// 8 % so.
+template <class P, int CT>
+__global__ void __launch_bounds__(CT, 256 / CT)
 x_rows(TileArgs A, typename P::Consts KP, const int64_t* __restrict__ rows, int64_t nBlk, int m,
        double* __restrict__ partial, unsigned long long* __restrict__ counters) {
-  constexpr int CT = P::kRowCta, NW = CT / 32;
+  constexpr int NW = CT / 32;
   __shared__ uint16_t list[CT * kRowMaxSteps];
   __shared__ int cnt[NW];
   __shared__ double red[NW][6];
@@ -390,7 +391,12 @@ template <class P>
 cudaError_t launch_rows(const TileArgs& A, const typename P::Consts& KP, const int64_t* rows, int64_t nRows,
                         const RowPlan& plan, double* partial, double* out, unsigned long long* counters,
                         cudaStream_t st) {
-  x_rows<P><<<(unsigned)(nRows * plan.nBlk), P::kRowCta, 0, st>>>(A, KP, rows, plan.nBlk, plan.m, partial, counters);
+  const unsigned grid = (unsigned)(nRows * plan.nBlk);
+  if constexpr (P::kRowWide) {
+    if (plan.threads == 256)
+      x_rows<P, 256><<<grid, 256, 0, st>>>(A, KP, rows, plan.nBlk, plan.m, partial, counters);
+  }
+  if (plan.threads == 128) x_rows<P, 128><<<grid, 128, 0, st>>>(A, KP, rows, plan.nBlk, plan.m, partial, counters);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   x_reduce_rows<<<(unsigned)((nRows + 3) / 4), 128, 0, st>>>(partial, plan.nBlk, nRows, out);

@@ -364,7 +364,7 @@ struct PolF64 {
     c = dot(a.t, b.t);
     return 1.0 - c * c > kSqrtEps;
   }
-  static constexpr int kRowCta = 128;  // threads per CTA of x_rows (ddd_internal.h's kRowThreads)
+  static constexpr bool kRowWide = false;  // x_rows with 256-thread CTAs too (segseg_small.cuh)
   // QUAD: four lanes per pair (pair_f64.cuh), for the policies that have it.
   static constexpr bool kQuad = true;
   template <bool BOTH, bool QUAD = false>

@@ -128,7 +128,7 @@ struct PolDF {
     add_df(s.fj[warp][4][j], F4.y);
     add_df(s.fj[warp][5][j], F4.z);
   }
-  static constexpr int kRowCta = FORM == 0 ? 256 : 128;  // threads per CTA of x_rows (ddd_internal.h's kRowThreads*)
+  static constexpr bool kRowWide = FORM == 0;  // x_rows with 256-thread CTAs too (segseg_small.cuh)
   static constexpr bool kQuad = false;
   // One component as segseg_small.cuh stores (hi, lo in 8 bytes) and adds it.
   using Comp = df64;

@@ -13,12 +13,13 @@ extern "C" cudaError_t cudaFree(void*) { return cudaSuccess; }
 using namespace ddd;
 
 extern "C" {
-// The row plan of a call: column blocks, steps per CTA, rows per launch.
-void plan_rows(int64_t npad, int64_t nRows, int64_t limit, int64_t threads, int64_t* out) {
-  const RowPlan p = row_plan(npad, nRows, (int)threads);
+// The row plan of a call: column blocks, steps per CTA, rows per launch, threads.
+void plan_rows(int64_t npad, int64_t nRows, int64_t limit, int64_t df64, int64_t* out) {
+  const RowPlan p = row_plan(npad, nRows, df64);
   out[0] = p.nBlk;
   out[1] = p.m;
   out[2] = rows_per_chunk(p, nRows, limit);
+  out[3] = p.threads;
 }
 // The chunk of a few-point stress call (evaluations), its scratch, its point limit.
 void plan_sigma(int64_t nSeg, int64_t M, int64_t* out) {

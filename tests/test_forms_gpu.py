@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("mode", ["fp64_fma", "fp64_fast", "df64", "f32c"])
 @pytest.mark.parametrize("n,rows", [(2, 1), (33, 40), (129, 3), (2017, 600)])
 def test_index_rows_forms(pkg, synth, oracle, mode, n, rows):
-    """One step and seven steps per CTA (600 rows of 2,017 segments; 256 threads in df64, else 128),
+    """One step and seven steps per CTA (600 rows of 2,017 segments; there 256 threads in df64),
     columns that end inside a block, repeated and external rows, under each form's bounds of
     test_segseg_gpu.py."""
     net = _synthetic(pkg, synth, (n + 7) // 8, 7 + n, parallel_fraction=0.2, cube=3000.0)

@@ -37,11 +37,12 @@ def plan(tmp_path_factory):
 
 @pytest.mark.parametrize("n,rows,limit", [(1, 1, 0), (6001, 37, 0), (6001, 6001, 16 << 30),
                                           (2_000_000, 2_000_000, 200 << 30), (16_000_000, 16_000_000, 1 << 40), (100_000, 3_000_000_000, 1 << 42)])
-@pytest.mark.parametrize("threads", [128, 256])
-def test_row_chunks(plan, threads, n, rows, limit):
+@pytest.mark.parametrize("df64", [0, 1])
+def test_row_chunks(plan, df64, n, rows, limit):
     """A chunk's CTAs fit a grid, its partial sums the limit (or 128 rows), and every column has a block."""
     npad = -(-n // 128) * 128
-    blocks, m, chunk = plan("plan_rows", 3, npad, rows, limit, threads)
+    blocks, m, chunk, threads = plan("plan_rows", 4, npad, rows, limit, df64)
+    assert threads == (256 if df64 and m >= 4 else 128)
     assert 1 <= m <= 8 and blocks * m * threads >= npad > (blocks - 1) * m * threads
     assert 1 <= chunk <= rows and chunk * blocks < 2 ** 31
     assert chunk * blocks * 48 <= max(limit, 128 * blocks * 48)
