@@ -279,8 +279,12 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
 // ends that way; a call that failed half-way leaves its part until then).  Measured:
 // host call at 24 segments 132 -> 115 us, a 512-segment step (seg-seg, self and PK
 // force, mobility, collision) 985 -> 919 us; above 512 KB the arrays are large enough
-// for copies of their own.
+// for copies of their own, a lone array above 256 KB (20,000 points of a stress call,
+// 480 KB: 150 us, 139 without).  Results are copied out of it once more by the host,
+// which pays up to 128 KB: dlnMobility of 4,500 nodes (216 KB) 160 us, 154 without,
+// stress at 9,000 points (432 KB) 123 and 109.
 constexpr size_t kPinBytes = (size_t)2 << 20, kPinMost = (size_t)1 << 19;
+constexpr size_t kPinMostAlone = (size_t)1 << 18, kPinMostRead = (size_t)1 << 17;
 char* pin_take(ddd_ctx* ctx, size_t bytes) {
   bytes = (bytes + 63) & ~(size_t)63;
   if (bytes > kPinMost) return nullptr;
@@ -315,7 +319,7 @@ struct Upload {
 int send(ddd_ctx* ctx, DevBuf& dst, const Upload& u, const char* what) {
   CK(dst.ensure(u.total), what);
   char* d = dst.as<char>();
-  if (char* h = pin_take(ctx, u.total)) {
+  if (char* h = u.n == 1 && u.total > kPinMostAlone ? nullptr : pin_take(ctx, u.total)) {
     for (int k = 0; k < u.n; ++k)
       if (u.bytes[k]) memcpy(h + u.off[k], u.src[k], u.bytes[k]);
     CK(cudaMemcpyAsync(d, h, u.total, cudaMemcpyHostToDevice, ctx->stream), what);
@@ -329,7 +333,7 @@ int send(ddd_ctx* ctx, DevBuf& dst, const Upload& u, const char* what) {
 // Reads `bytes` from the device into `host` and waits for the stream; `after`, if
 // given, is recorded behind the copy.
 int fetch(ddd_ctx* ctx, void* host, const void* dev, size_t bytes, cudaEvent_t after, const char* what) {
-  char* h = pin_take(ctx, bytes);
+  char* h = bytes <= kPinMostRead ? pin_take(ctx, bytes) : nullptr;
   CK(cudaMemcpyAsync(h ? h : host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream), what);
   if (after) CK(cudaEventRecord(after, ctx->stream), "event");
   CK(cudaStreamSynchronize(ctx->stream), what);
