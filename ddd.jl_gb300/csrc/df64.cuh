@@ -228,7 +228,9 @@ DF_HD df64 df_atan(df64 x) {
 // issue slot and one 4-cycle latency (measured).  The pair kernels hold 8 warps
 // per SM (255 registers), and their df64 code is chains of dependent additions:
 // the FMA pipe was 46 % busy.
-#if defined(__CUDACC__)
+//
+// DDD_F2_PLAIN: the same source on scalar instructions (tests compare the two).
+#if defined(__CUDACC__) && !defined(DDD_F2_PLAIN)
 struct f2 {
   unsigned long long v;
 };
@@ -363,7 +365,9 @@ DF_HD df2 df_log(df2 a) {
   const df2 u = (m - c) / (m + c);
   const df2 u2 = u * u;
   const f2 t = u2.hi;
-  // Lane by lane: a packed product used once would be fused into its sum.
+  // Lane by lane: the compiler fuses a packed product that is used once into its sum,
+  // also under --fmad=false.  Every other product here has two uses or more, or a power
+  // of two as a factor (tests/test_df2_gpu.py compares all lanes on the device).
   auto poly = [](float w) { return w * (0.2f + w * 0.14285714285714285f); };
   const f2 tail = f2_make(poly(f2_x(t)), poly(f2_y(t)));
   const df2 P = df2{f2_dup(kDfThird_HI), f2_dup(kDfThird_LO)} + tail;
