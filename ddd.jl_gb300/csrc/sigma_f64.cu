@@ -69,11 +69,13 @@ sigma_tilde_f64(KConsts K, const double* __restrict__ soa, int64_t npad, int64_t
 }
 
 // Fewer points than kSigmaSplitPoints: a thread per (segment, point) instead of
-// per point, segments in chunks of `chunk` evaluations (sigma_split_chunk).  The contributions go
-// to a store and are added to sigma in segment order by the first blocks of the
-// next chunk's launch, beside its evaluations (one DADD of a point's chain takes
-// 64 cycles, so a chunk's chain is ~1/10 of its evaluations' time), so every
-// point's sum keeps the reference's order and bits.  Two stores alternate.
+// per point, segments in chunks of `chunk` evaluations (sigma_split_chunk).  The
+// contributions go to a store and are added to sigma in segment order by the first
+// blocks of the next chunk's launch, beside its evaluations (one DADD of a point's
+// chain takes 64 cycles, so a chunk's chain is ~1/10 of its evaluations' time), so
+// every point's sum keeps the reference's order, and in the strict build its bits
+// (the FMA build contracts an evaluation differently in the two kernels: 4e-16 of
+// the largest stress).  Two stores alternate.
 //
 // Why: a point per thread is 20 one-warp CTAs for 613 points, one warp per SM at
 // 64 cycles per FP64 instruction (its latency) instead of 16-19 (the pipe's
