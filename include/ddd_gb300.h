@@ -125,7 +125,10 @@ int ddd_version(void);
  *   3 × 2 × numSeg and is overwritten.
  * idx != NULL: for each k, i = idx[k] (1-based, duplicates allowed), the sum over
  *   all j != i (non-external) of the forces on segment i's two nodes; force is
- *   3 × 2 × nIdx and is overwritten; column k stays 0 when segment i is external. */
+ *   3 × 2 × nIdx and is overwritten; column k stays 0 when segment i is external.
+ *   A row's sum is grouped by blocks of columns whose size depends on nIdx: the
+ *   same call gives the same bits, a row in a longer or shorter list the same
+ *   value to rounding. */
 int ddd_segseg_force(ddd_ctx* ctx, const ddd_consts* k, const double* coord, int64_t coordCols, const double* bVec,
                      int64_t bVecCols, const int64_t* segIdx, int64_t ldSegIdx, const uint8_t* extSeg,
                      int64_t numSeg, const int64_t* idx, int64_t nIdx, double* force, ddd_report* rep);
@@ -261,7 +264,11 @@ int ddd_minimum_distance(ddd_ctx* ctx, const double* pts, int64_t n, double* out
  * component c: uTilde[uDofs[3p + c] - 1] += u_c(p), or uTilde[3p + c] when
  * uDofs is NULL (calc_uTilde's 1:3numPoints); calc_uTilde! passes
  * boundaries.uDofsDln after zeroing uTilde, exactly the reference's indexing.
- * Each point's sum runs over the triangles in the reference's order. */
+ * Each point's sum runs over the triangles in the reference's order, cut into
+ * chunks of consecutive triangles (8 or more, as many chunks as one wave of the
+ * GPU holds) whose sums are added in that order.  The cut depends on the numbers
+ * of points and triangles and on the mode: the same call gives the same bits, a
+ * point in a call of another size the same value to rounding. */
 typedef struct ddd_u_mesh {
   double C[3];
   double lo[3], hi[3];
@@ -281,7 +288,14 @@ int ddd_u_tilde(ddd_ctx* ctx, double omNuInv8pi, double om2NuOmNuInv8pi, const d
  * calc_σTilde!(σ, x0, ...) — src/Processing/DislocationFEM.jl:24-84, kernel
  * _calc_σTilde! :86-303.  Both write sigma (6 × numPoints) fresh.  Segments are
  * rows 1:numSeg of segIdx, or the rows listed in idx (1-based, <= ldSegIdx);
- * extSeg is ignored, as in the reference. */
+ * extSeg is ignored, as in the reference.  In DDD_MODE_FP64 a point's sum runs
+ * over the segments in list order and does not depend on the other points.  In
+ * DDD_MODE_FP64_FAST, DDD_MODE_DF64 and DDD_MODE_F32C a call with few points sums
+ * slices of the segments, and their number depends on the numbers of points and
+ * segments (and on the partial-sum limit): the same call gives the same bits, a
+ * point in a call of another size the same value to rounding.  In
+ * DDD_MODE_FP64_FMA the order is the list's too, but calls under 24,576 points
+ * take another kernel, whose terms round differently. */
 int ddd_sigma_tilde(ddd_ctx* ctx, const ddd_consts* k, const double* x0, int64_t numPoints, const double* coord,
                     int64_t coordCols, const double* bVec, int64_t bVecCols, const int64_t* segIdx,
                     int64_t ldSegIdx, int64_t numSeg, const int64_t* idx, int64_t nIdx, double* sigma,
