@@ -19,29 +19,28 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", 
 
 
 # Translation units compiled more than once: (object suffix, extra flags).
-# DDD_F64_CONTRACT (f64reg.cuh): plain FP64 operators, for the FMA build, which
-# the compiler contracts, and for the df64 kernels, whose FP32 main loop has no
-# registers left for the operators' two constants (2-4 % slower with them), for
-# the strict calc_uTilde, mostly CUDA's acos and tan (2 % slower), and for the
-# FP64 near pass (tile_launch.cu).
+# DDD_F64_PLAIN (f64reg.cuh): plain FP64 operators, for the FMA build, which the
+# compiler contracts, for the df64 kernels, whose FP32 main loop has no registers
+# left for the operators' two constants (2-4 % slower with them), and for the FP64
+# near pass (tile_launch.cu).
 VARIANTS = {
     "segseg_f64.cu": [("strict", ["-DDDD_VARIANT=strict", "--fmad=false"]),
-                      ("fast", ["-DDDD_VARIANT=fast", "-DDDD_F64_CONTRACT", "-DDDD_FMA"])],
-    "sigma_f64.cu": [("strict", ["-DDDD_VARIANT=strict", "--fmad=false"]), ("fast", ["-DDDD_VARIANT=fast", "-DDDD_F64_CONTRACT"])],
+                      ("fast", ["-DDDD_VARIANT=fast", "-DDDD_F64_PLAIN", "-DDDD_FMA"])],
+    "sigma_f64.cu": [("strict", ["-DDDD_VARIANT=strict", "--fmad=false"]), ("fast", ["-DDDD_VARIANT=fast", "-DDDD_F64_PLAIN"])],
     # df64 needs exact error-free transformations: no contraction.
-    "segseg_df.cu": [("", ["--fmad=false", "-DDDD_F64_CONTRACT"])],
+    "segseg_df.cu": [("", ["--fmad=false", "-DDDD_F64_PLAIN"])],
     # explicit fused multiply-adds only (host builds of its header give the same bits)
     "segseg_f64fast.cu": [("", ["--fmad=false"])],
     "sigma_fx.cu": [("", ["--fmad=false"])],
     "segseg_batch.cu": [("", ["--fmad=false"])],
-    "tile_launch.cu": [("f64", ["--fmad=false"]), ("near", ["--fmad=false", "-DDDD_NEAR_PASS", "-DDDD_F64_CONTRACT"]),
-                       ("df", ["--fmad=false", "-DDDD_DF_POLICIES", "-DDDD_F64_CONTRACT"])],
+    "tile_launch.cu": [("f64", ["--fmad=false"]), ("near", ["--fmad=false", "-DDDD_NEAR_PASS", "-DDDD_F64_PLAIN"]),
+                       ("df", ["--fmad=false", "-DDDD_DF_POLICIES", "-DDDD_F64_PLAIN"])],
     "surrogate_data.cu": [("", ["--fmad=false"])],
     "surrogate_force.cu": [("", ["--fmad=false"])],
     "self_force.cu": [("", ["--fmad=false"])],
     "mobility.cu": [("", ["--fmad=false"])],
     "collision.cu": [("", ["--fmad=false"])],
-    "u_tilde.cu": [("", ["--fmad=false", "-DDDD_F64_CONTRACT", "-Xcompiler", "-ffp-contract=off"])],
+    "u_tilde.cu": [("", ["--fmad=false", "-Xcompiler", "-ffp-contract=off"])],
     "u_tilde_fast.cu": [("", ["--fmad=false"])],
 }
 

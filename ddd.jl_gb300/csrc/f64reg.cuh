@@ -17,15 +17,15 @@
 // too, and the compiler moves a value that it knows to be the same in every lane
 // there (a constant, a load from one address).  So each lane loads its own copy.
 //
-// Translation units that want the compiler's own contraction (the FMA build)
-// define DDD_F64_CONTRACT, as do those with df64 kernels; a host compiler gets
-// plain double.
+// Translation units that want the compiler's own operators (to be contracted in the
+// FMA build, or for the registers: build.py) define DDD_F64_PLAIN; a host compiler
+// gets plain double.
 #pragma once
 #include <cstdint>
 
 namespace ddd {
 
-#if defined(__CUDACC__) && !defined(DDD_F64_CONTRACT)
+#if defined(__CUDACC__) && !defined(DDD_F64_PLAIN)
 
 #define DDD_X8(v) v, v, v, v, v, v, v, v
 static __device__ double kF64Ones[32] = {DDD_X8(1.0), DDD_X8(1.0), DDD_X8(1.0), DDD_X8(1.0)};

@@ -25,7 +25,6 @@
 #include <vector>
 
 #include "ddd_internal.h"
-#include "f64reg.cuh"
 #include "intmath_f64.cuh"
 
 namespace ddd {
@@ -37,14 +36,12 @@ constexpr int TROW = kUTriRows;  // doubles per triangle (layout below)
 struct V {
   double x, y, z;
 };
-// Sums and products through rd (f64reg.cuh): the plain operations' bits.
-__device__ __forceinline__ V v3(rd x, rd y, rd z) { return {x, y, z}; }
-__device__ __forceinline__ V operator+(V a, V b) { return v3(rd(a.x) + b.x, rd(a.y) + b.y, rd(a.z) + b.z); }
-__device__ __forceinline__ V operator-(V a, V b) { return v3(rd(a.x) - b.x, rd(a.y) - b.y, rd(a.z) - b.z); }
-__device__ __forceinline__ V operator*(V a, rd s) { return v3(a.x * s, a.y * s, a.z * s); }
-__device__ __forceinline__ rd dot(V a, V b) { return rd(a.x) * b.x + rd(a.y) * b.y + rd(a.z) * b.z; }
-__device__ __forceinline__ V cross(V a, V b) {
-  return v3(rd(a.y) * b.z - rd(a.z) * b.y, rd(a.z) * b.x - rd(a.x) * b.z, rd(a.x) * b.y - rd(a.y) * b.x);
+__host__ __device__ __forceinline__ V operator+(V a, V b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
+__host__ __device__ __forceinline__ V operator-(V a, V b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+__host__ __device__ __forceinline__ V operator*(V a, double s) { return {a.x * s, a.y * s, a.z * s}; }
+__host__ __device__ __forceinline__ double dot(V a, V b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__host__ __device__ __forceinline__ V cross(V a, V b) {
+  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
 __device__ __forceinline__ V ld3(const double* a, int64_t n) { return {a[3 * n], a[3 * n + 1], a[3 * n + 2]}; }
 
@@ -53,8 +50,8 @@ __device__ __forceinline__ V ld3(const double* a, int64_t n) { return {a[3 * n],
 __device__ __forceinline__ double safe_norm(V& x) {
   const double n = sqrt(dot(x, x));
   if (n > DBL_EPSILON) {
-    const rd inv = 1.0 / n;
-    x = v3(inv * x.x, inv * x.y, inv * x.z);
+    const double inv = 1.0 / n;
+    x = {inv * x.x, inv * x.y, inv * x.z};
     return n;
   }
   x = {0.0, 0.0, 0.0};
@@ -183,26 +180,27 @@ __device__ __forceinline__ V tri_u(const double* s, double omNuInv8pi, double om
   // RC . RA here equals the previous triangle's RB . RC term by term.
   const double ta = acos(RAdRB), tb = acos(RBdRC), tc = (chained && closure && ch.closure) ? ch.tb : acos(RCdRA);
   ch = {RB, RBn, tb, closure, true};
-  const rd th = (rd(ta) + tb + tc) * 0.5;  // halving is exact
-  const rd factor = jl_max0(rd(tan(th * 0.5)) * rd(tan((th - ta) * 0.5)) * rd(tan((th - tb) * 0.5)) *
-                            rd(tan((th - tc) * 0.5)));
-  rd omega = 4.0 * im::atan(sqrt(double(factor)));
+  const double th = (ta + tb + tc) / 2.0;
+  const double factor =
+      jl_max0(tan(th / 2.0) * tan((th - ta) / 2.0) * tan((th - tb) / 2.0) * tan((th - tc) / 2.0));
+  double omega = 4.0 * im::atan(sqrt(factor));
   omega = -jl_sign(dot(RA, cross(CA, AB))) * omega;
-  const rd fourPi = 4.0 * 3.141592653589793;
-  V u = v3(-b.x * omega / fourPi, -b.y * omega / fourPi, -b.z * omega / fourPi);
+  const double fourPi = 4.0 * 3.141592653589793;
+  V u = {-b.x * omega / fourPi, -b.y * omega / fourPi, -b.z * omega / fourPi};
   if (s[21] == 0.0) return u;
   const V bAB = {s[23], s[24], s[25]}, bBC = {s[26], s[27], s[28]}, bCA = {s[29], s[30], s[31]};
-  const V fAB = bAB * rd(im::log((rd(RBn) / RAn) * (rd_one() + dot(RB, AB)) / (rd_one() + dot(RA, AB))));
-  const V fBC = bBC * rd(im::log((rd(RCn) / RBn) * (rd_one() + dot(RC, BC)) / (rd_one() + dot(RB, BC))));
-  const V fCA = bCA * rd(im::log((rd(RAn) / RCn) * (rd_one() + dot(RA, CA)) / (rd_one() + dot(RC, CA))));
-  const rd sAB = dot(b, cross(RA, RB)), sBC = dot(b, cross(RB, RC)), sCA = dot(b, cross(RC, RA));
+  const V fAB = bAB * im::log((RBn / RAn) * (1.0 + dot(RB, AB)) / (1.0 + dot(RA, AB)));
+  const V fBC = bBC * im::log((RCn / RBn) * (1.0 + dot(RC, BC)) / (1.0 + dot(RB, BC)));
+  const V fCA = bCA * im::log((RAn / RCn) * (1.0 + dot(RA, CA)) / (1.0 + dot(RC, CA)));
+  const double sAB = dot(b, cross(RA, RB)), sBC = dot(b, cross(RB, RC)), sCA = dot(b, cross(RC, RA));
   const V vAB = RA + RB, vBC = RB + RC, vCA = RC + RA;
-  const rd dAB = rd_one() + RAdRB, dBC = rd_one() + RBdRC, dCA = rd_one() + RCdRA;
-  const V gAB = v3(sAB * vAB.x / dAB, sAB * vAB.y / dAB, sAB * vAB.z / dAB);
-  const V gBC = v3(sBC * vBC.x / dBC, sBC * vBC.y / dBC, sBC * vBC.z / dBC);
-  const V gCA = v3(sCA * vCA.x / dCA, sCA * vCA.y / dCA, sCA * vCA.z / dCA);
+  const double dAB = 1.0 + RAdRB, dBC = 1.0 + RBdRC, dCA = 1.0 + RCdRA;
+  const V gAB = {sAB * vAB.x / dAB, sAB * vAB.y / dAB, sAB * vAB.z / dAB};
+  const V gBC = {sBC * vBC.x / dBC, sBC * vBC.y / dBC, sBC * vBC.z / dBC};
+  const V gCA = {sCA * vCA.x / dCA, sCA * vCA.y / dCA, sCA * vCA.z / dCA};
   const V fs = fAB + fBC + fCA, gs = gAB + gBC + gCA;
-  return u - fs * om2NuOmNuInv8pi + gs * omNuInv8pi;
+  return u - V{om2NuOmNuInv8pi * fs.x, om2NuOmNuInv8pi * fs.y, om2NuOmNuInv8pi * fs.z} +
+         V{omNuInv8pi * gs.x, omNuInv8pi * gs.y, omNuInv8pi * gs.z};
 }
 
 // Block (x, y): points x * PT.., triangles [y * chunk, (y + 1) * chunk), in
